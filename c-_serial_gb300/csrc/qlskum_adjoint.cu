@@ -85,8 +85,7 @@ template <int MODE>
 __global__ void __launch_bounds__(128) k_flux(AdjView a, const double4_32a *__restrict__ q,
                                                const double4_32a *__restrict__ dq, const double4_32a *__restrict__ qm,
                                                const double *__restrict__ delta, const double4_32a *__restrict__ flux,
-                                               const double *__restrict__ sums, const double *__restrict__ ends,
-                                               long long ns, const double4_32a *__restrict__ bF,
+                                               const double *__restrict__ ends, long long ns, const double4_32a *__restrict__ bF,
                                                double4_32a *__restrict__ bq, double4_32a *__restrict__ bdq,
                                                double4_32a *__restrict__ bqm, double *__restrict__ bdelta)
 {
@@ -114,37 +113,30 @@ __global__ void __launch_bounds__(128) k_flux(AdjView a, const double4_32a *__re
     const bool used[4] = {true, true, f != kWall, f != kOuter};
     const bool geo = GEO;
 
-    // forward: the directional sums, for the bars of the moments (GEO only:
-    // the forward kernel's stored sums, or recomputed; without them the bar of
-    // delta comes from the stage's flux residual, F = delta * scale * sum_d G_d,
-    // so dF/ddelta = F / delta)
+    // forward: the directional sums, for the bars of the moments (GEO only;
+    // without them the bar of delta comes from the stage's flux residual,
+    // F = delta * scale * sum_d G_d, so dF/ddelta = F / delta)
     double sx[4][4], sy[4][4];
     for (int d = 0; d < 4; d++)
         for (int r = 0; r < 4; r++) sx[d][r] = sy[d][r] = 0.0;
-    if (geo && sums) {
-        const double *o = sums + 32 * (size_t)i;
-        for (int d = 0; d < 4; d++)
-            for (int r = 0; r < 4; r++) {
-                sx[d][r] = o[8 * d + r];
-                sy[d][r] = o[8 * d + 4 + r];
-            }
-    }
-    for (int j = 0; geo && !sums && j < nb; j++) {
+    for (int j = 0; geo && j < nb; j++) {
         const long long e = base + 32LL * j;
         const int k = c.e_nbr[e];
         const double4_32a g = c.e_geo[e];
         const double2 sw = c.e_sn[e];
         const unsigned dir = c.e_dir[e];
-        double qk[4], dxk[4], dyk[4], mxk[4], mnk[4], Pi[4], Pk[4];
+        double qk[4], dxk[4], dyk[4], mxk[4], mnk[4], kept[12];
         ld4(q[k], qk);
         ld4(dq[2 * k], dxk);
         ld4(dq[2 * k + 1], dyk);
         ld4(qm[2 * k], mxk);
         ld4(qm[2 * k + 1], mnk);
-        edge_states<double>(g.x, g.y, qi, dxi, dyi, mxi, mni, e2i, qk, dxk, dyk, mxk, mnk, c.eps2[k], Pi, Pk);
-        Kin<double> ki, kk;
-        kin_prep<double>(nx, ny, Pi[1], Pi[2], Pi[0], Pi[3], ki);
-        kin_prep<double>(nx, ny, Pk[1], Pk[2], Pk[0], Pk[3], kk);
+        for (int w = 0; ends && w < 12; w++) kept[w] = ends[w * ns + e];
+        adj::End64 s;
+        adj::end64(nx, ny, g.x, g.y, qi, dxi, dyi, mxi, mni, e2i, s, ends ? kept : nullptr);
+        const Kin<double> ki = s.k;
+        adj::end64(nx, ny, g.x, g.y, qk, dxk, dyk, mxk, mnk, c.eps2[k], s, ends ? kept + 6 : nullptr);
+        const Kin<double> kk = s.k;
 #define QLSKUM_FWD(D)                                                                \
         if (dir & (1u << D)) {                                                       \
             double Gi[4], Gk[4];                                                     \
@@ -1161,13 +1153,13 @@ void update(const Launch &L, const AdjView &a, const CaseConst &K, const double4
 }
 
 void flux(const Launch &L, const AdjView &a, const double4_32a *q, const double4_32a *dq, const double4_32a *qm,
-          const double *delta, const double4_32a *flux, const double *sums, const double *ends, long long ns,
-          const double4_32a *bF, double4_32a *bq, double4_32a *bdq, double4_32a *bqm, double *bdelta)
+          const double *delta, const double4_32a *flux, const double *ends, long long ns, const double4_32a *bF,
+          double4_32a *bq, double4_32a *bdq, double4_32a *bqm, double *bdelta)
 {
-    adjk::k_flux<0><<<adjk::grid_for(a.c.n, 128), 128, 0, L.stream>>>(a, q, dq, qm, delta, flux, nullptr, ends, ns,
-                                                                       bF, bq, bdq, bqm, bdelta);
+    adjk::k_flux<0><<<adjk::grid_for(a.c.n, 128), 128, 0, L.stream>>>(a, q, dq, qm, delta, flux, ends, ns, bF,
+                                                                       bq, bdq, bqm, bdelta);
     if (a.bedge && a.n_geo > 0)
-        adjk::k_flux<2><<<adjk::grid_for(a.n_geo, 128), 128, 0, L.stream>>>(a, q, dq, qm, delta, flux, sums, ends, ns,
+        adjk::k_flux<2><<<adjk::grid_for(a.n_geo, 128), 128, 0, L.stream>>>(a, q, dq, qm, delta, flux, ends, ns,
                                                                             bF, bq, bdq, bqm, bdelta);
 }
 

@@ -1,0 +1,206 @@
+// FP64 elementary functions and edge ends with few FP64 instructions, for the
+// drop-in form's flux kernels and their reverse.
+//
+// GB300 executes one FP64 instruction per warp and SM in 16 cycles, against
+// four FP32 or integer ones per cycle, so the flux kernels are bound by the
+// number of FP64 instructions alone.  What can be done beside the FP64 pipe
+// without touching the FP64 result is done there: comparisons on the bit
+// patterns, argument reductions and seeds in FP32, and the high-order terms
+// of an expansion, whose contribution is below 2^-28 of the result, so that
+// an FP32 evaluation (relative error 2^-24) stays below 2^-52 of it.
+//
+// Each function's error is at most about an ulp of its result (of 1 for erf),
+// as the CUDA functions it replaces; arguments outside the ranges below
+// (which a physical state does not reach, and every Inf / NaN) take those.
+//
+// FP64 instructions per call: gauss_erf 10 (exp and erf: about 50), exp32 6
+// (about 16), rsqrt64 5, ratio64 4.
+#pragma once
+#include "qlskum_math.cuh"
+
+namespace qlskum {
+namespace fast64 {
+
+__device__ __forceinline__ unsigned abs_hi(double x) { return (unsigned)__double2hiint(x) & 0x7fffffffu; }
+
+__device__ __forceinline__ double flip(double x, unsigned sign)
+{
+    return __hiloint2double((int)((unsigned)__double2hiint(x) ^ sign), __double2loint(x));
+}
+
+// |x| <= 1e-5 (the limiter's cut, limiters_mod.h:70) on the bit pattern; false for NaN.
+__device__ __forceinline__ bool within_cut(double x)
+{
+    return (__double_as_longlong(x) & 0x7fffffffffffffffLL) <= __double_as_longlong(10e-6);
+}
+
+// A finite seed that FP32 holds as a normal number.
+__device__ __forceinline__ bool seed_ok(float s) { return fabsf(s) > 1e-37f && fabsf(s) < 1e37f; }
+
+__device__ __noinline__ double div_slow(double a, double b) { return a / b; }
+__device__ __noinline__ double rsqrt_slow(double x) { return rsqrt(x); }
+__device__ __noinline__ double exp32_slow(double x) { return 32.0 * exp(x); }
+__device__ __noinline__ double2 gauss_erf_slow(double s) { return make_double2(0.5641895835477563 * exp(-s * s), erf(s)); }
+
+// num / den: the FP32 quotient corrected twice by its FP64 remainder.
+__device__ __forceinline__ double ratio64(double num, double den)
+{
+    const float r = __fdividef(1.0f, d2f(den));
+    const float q = d2f(num) * r;
+    if (!seed_ok(r) || !(fabsf(q) < 1e37f)) return div_slow(num, den);
+    const double rd = f2d(r);
+    double v = f2d(q);
+    v = fma(fma(-den, v, num), rd, v);
+    return fma(fma(-den, v, num), rd, v);
+}
+
+// 1 / sqrt(x): FP32 seed y, then y (1 + e/2 + 3 e^2 / 8), e = 1 - x y^2 (the next term is 2^-64).
+__device__ __forceinline__ double rsqrt64(double x)
+{
+    const float s = rsqrtf(d2f(x));
+    if (!seed_ok(s)) return rsqrt_slow(x);
+    const double y = f2d(s);
+    const double e = fma(-(x * y), y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// 32 exp(x) from tab[i] = 32 2^(i/512): x = k ln2/512 + r, |r| <= 2^-10.5,
+// exp(r) - 1 = r (1 + r (1/2 + r/6 + r^2/24)), the last two terms in FP32.
+__device__ __forceinline__ double exp32(double x, const double *__restrict__ tab)
+{
+    if (abs_hi(x) >= 0x40800000u) return exp32_slow(x);  // |x| >= 512 or NaN
+    const float kf = rintf(d2f(x) * 738.65986f);
+    const double kd = f2d(kf);
+    const int k = (int)kf;
+    double r = fma(-kd, 0.0013538030870311431, x);
+    r = fma(-kd, 4.529388308293554e-20, r);
+    const float rf = d2f(r);
+    const double h = 0.5 + f2d(rf * fmaf(rf, 0.041666667f, 0.16666667f));
+    const double p = r * fma(r, h, 1.0);
+    const double t = __ldg(tab + (k & 511));
+    const double ts = __hiloint2double(__double2hiint(t) + ((k >> 9) << 20), __double2loint(t));
+    return fma(ts, p, ts);
+}
+
+// e = exp(-s^2) / sqrt(pi) and E = erf(s) together, from
+// tab[j] = {exp(-x^2) / sqrt(pi), erf(x)} at the nearest x = j / 1024 to |s|,
+// d = |s| - x (exact, |d| <= 2^-11):
+//   exp(-s^2) = exp(-x^2) exp(-u), u = d (2 x + d), by its series, u^3 on in FP32;
+//   erf(s) = erf(x) + 2/sqrt(pi) d [(f0 + f1) / 2 + d (f0' - f1') / 12],
+// the corrected trapezoid over f = exp(-t^2) (error d^5 f'''' / 720 < 2^-60),
+// its correction, below 2^-24, in FP32.
+__device__ __forceinline__ void gauss_erf(double s, const double2 *__restrict__ tab, double &e, double &E)
+{
+    const unsigned ah = abs_hi(s);
+    if (ah >= 0x40180000u) {  // |s| >= 6 or NaN
+        const double2 v = gauss_erf_slow(s);
+        e = v.x;
+        E = v.y;
+        return;
+    }
+    const double a = __hiloint2double((int)ah, __double2loint(s));
+    const float jf = rintf(d2f(a) * 1024.0f);
+    const double2 t = __ldg(tab + (int)jf);
+    const float xf = jf * 0.0009765625f;
+    const double x = f2d(xf);
+    const double d = a - x;
+    const double u = d * fma(2.0, x, d);
+    const float uf = d2f(u), df = d2f(d);
+    const double h = 0.5 - f2d(uf * fmaf(uf, fmaf(uf, 0.0083333333f, -0.041666667f), 0.16666667f));
+    const double p = u * fma(u, h, -1.0);
+    e = fma(t.x, p, t.x);
+    // 2 d/6 (s e - x e0)
+    const float pf = d2f(p);
+    const float w = 0.33333334f * df * d2f(t.x) * fmaf(df, 1.0f + pf, xf * pf);
+    const double z = (t.x + e) + f2d(w);
+    E = flip(fma(d, z, t.y), (unsigned)__double2hiint(s) & 0x80000000u);
+}
+
+// One component of the limited reconstruction (interior_fluxes_mod.h:72-83,
+// limiters_mod.h:64-104): q + phi dn with dn = -(delx dqx + dely dqy) / 2
+// given; dp = qmax - q (dn > 0) or qmin - q.  The common factor dn of the
+// limiter's numerator and denominator cancels.
+__device__ __forceinline__ double limited(double q, double dn, double dp, double eps2)
+{
+    double phi = 1.0;
+    if (!within_cut(dn)) {
+        const double base = fma(dp, dp, eps2);
+        const double t = ratio64(fma(dn, dp + dp, base), fma(dn, fma(2.0, dn, dp), base));
+        // min(t, 1), 1 for NaN: t is non-negative, so its bits order like its value
+        if ((unsigned long long)__double_as_longlong(t) < 0x3ff0000000000000ULL) phi = t;
+    }
+    return fma(phi, dn, q);
+}
+
+// One edge end: q~ -> prim (q_variables_mod.h:230-253) and the half-range
+// moments (split_fluxes_mod.h:14-26) from q~ turned into the owner's (t, n)
+// frame (interior points' frame is (x, y)).  With b = -2 q~4 = 4 beta,
+// r = 1 / sqrt(b) and h = 1 / b: p / rho = 2 h, u = 2 h q~, S = u sqrt(beta) = r q~,
+// beta |u|^2 = S1^2 + S2^2, rho = exp(q~1 + S1^2 + S2^2) 32 h^2 r, and
+// 1 / (2 sqrt(pi beta)) = r / sqrt(pi).  h is r^2 corrected by its remainder:
+// rho takes it to the power 2.5, and with it the residual's error against a
+// 128-bit run is 0.85-1 times the one of reciprocals and a square root taken
+// one by one (without it 1.2 times).
+struct End {
+    Kin<double> k;
+    double r, e1, e2;  // kept for the reverse: r, exp(-S1^2) and exp(-S2^2) over sqrt(pi)
+};
+
+__device__ __forceinline__ void end(const DevCloud &c, int f, double nx, double ny, const double t[4], End &s)
+{
+    double qs = t[1], qn = t[2];
+    if (f != kInterior) {
+        qs = fma(t[1], ny, -(t[2] * nx));
+        qn = fma(t[1], nx, t[2] * ny);
+    }
+    const double b = -2.0 * t[3];
+    const double r = rsqrt64(b);
+    double h = r * r;
+    h = fma(h, fma(-b, h, 1.0), h);
+    const double S1 = qs * r, S2 = qn * r;
+    s.k.pbr = h + h;
+    s.k.ut = qs * s.k.pbr;
+    s.k.un = qn * s.k.pbr;
+    s.k.usq = fma(s.k.ut, s.k.ut, s.k.un * s.k.un);
+    s.k.rho = exp32(fma(S1, S1, fma(S2, S2, t[0])), c.exp_tab) * (h * h * r);
+    gauss_erf(S1, c.gauss_tab, s.e1, s.k.E1);
+    gauss_erf(S2, c.gauss_tab, s.e2, s.k.E2);
+    s.k.B1 = r * s.e1;
+    s.k.B2 = r * s.e2;
+    s.r = r;
+}
+
+// What the reverse reads back instead of evaluating it again, as planes of ns
+// doubles: rho, sqrt(beta), exp(-S1^2), exp(-S2^2), erf(S1), erf(S2).
+__device__ __forceinline__ void keep_end(double *__restrict__ o, long long ns, double t3, const End &s)
+{
+    o[0] = s.k.rho;
+    o[ns] = -t3 * s.r;
+    o[2 * ns] = 1.7724538509055159 * s.e1;
+    o[3 * ns] = 1.7724538509055159 * s.e2;
+    o[4 * ns] = s.k.E1;
+    o[5 * ns] = s.k.E2;
+}
+
+// Adds one interior end's weighted pair wx Gx(s1) + wy Gy(s2) to v.  With
+// A = (1 + s E) / 2, al = wx rho A1, ga = wy rho A2 and
+// be = wx rho s1 B1 + wy rho s2 B2, the pair (split_fluxes_mod.h:14-84 and
+// :86-164) is
+//   v0 = al ut + ga un + be,  v1 = ut v0 + al p/rho,  v2 = un v0 + ga p/rho,
+//   v3 = (usq v0 + p/rho (7 v0 - be)) / 2;  twice v3 is added.
+// sx, sy: the sign bits of s1, s2 (0 for +1).
+__device__ __forceinline__ void interior_pair(const Kin<double> &k, unsigned sx, unsigned sy, double wx, double wy,
+                                              double v[4])
+{
+    const double wr = wx * k.rho, yr = wy * k.rho;
+    const double al = wr * fma(0.5, flip(k.E1, sx), 0.5), ga = yr * fma(0.5, flip(k.E2, sy), 0.5);
+    const double be = fma(flip(wr, sx), k.B1, flip(yr, sy) * k.B2);
+    const double v0 = fma(al, k.ut, fma(ga, k.un, be));
+    v[0] += v0;
+    v[1] = fma(k.ut, v0, fma(al, k.pbr, v[1]));
+    v[2] = fma(k.un, v0, fma(ga, k.pbr, v[2]));
+    v[3] = fma(k.pbr, fma(7.0, v0, -be), fma(k.usq, v0, v[3]));
+}
+
+}  // namespace fast64
+}  // namespace qlskum

@@ -2,13 +2,11 @@
 //
 // Every formula is the reference's, with FMA contraction on (GB300 runs FP64
 // at 1/64 of the FP32 rate, and a fused multiply-add is one FP64 instruction
-// instead of two), and in the edge ends' hot arithmetic a few expressions
-// rewritten to use fewer FP64 instructions for the same value to a few ulps
-// (edge_qtilde / venkat_r and end_kin in qlskum_math.cuh: one reciprocal
-// square root for sqrt(beta), 1 / sqrt(pi beta) and beta^-2.5, reciprocals
-// instead of divisions).  The results differ from the serial reference by
-// those roundings and the device's exp / log / erf: 1e-10 relative after
-// 1000 iterations (the parity tests).
+// instead of two), and the edge ends in the forms of qlskum_fast64.cuh, which
+// need few FP64 instructions for the same value to a few ulps.  The
+// directional solves are folded into per-edge weights once per cloud.  The
+// results differ from the serial reference by those roundings: 1e-10 relative
+// after 1000 iterations (the parity tests).
 //
 // One thread per point; the point's edges are walked in the reference's
 // neighbour order from the sliced-ELL edge arrays (coalesced across the warp),
@@ -19,6 +17,7 @@
 // operation order, which on this chip trades a few bytes per edge for FP64
 // instructions, its scarce resource.
 #include "qlskum_math.cuh"
+#include "qlskum_fast64.cuh"
 
 namespace qlskum {
 namespace fp64 {
@@ -164,119 +163,188 @@ __global__ void k_func_delta(DevCloud c, const double4_32a *__restrict__ prim, d
 
 // ------------------------------------------------------------- flux
 
-// The four directional flux derivatives of point i (interior_/wall_/
-// outer_fluxes_mod.h), walked edge by edge: each edge's limited end states
-// are reconstructed once and feed every sub-stencil the edge belongs to,
-// in the reference's neighbour order, so the sums are the reference's.
-// G[d] returns the solved derivative of sub-stencil d (xpos, xneg, ypos,
-// yneg); unused directions are left at 0.
-// sums (or NULL): the directional sums {sx[d][0..3], sy[d][0..3]} of each d,
-// 32 doubles per point, kept for the reverse's moment bars.
-__device__ __forceinline__ void point_flux(const DevCloud &c, int i, int f, double nx, double ny,
-                                           const double4_32a *__restrict__ q, const double4_32a *__restrict__ dq,
-                                           const double4_32a *__restrict__ qm, double G[4][4],
-                                           double *__restrict__ sums = nullptr, double *__restrict__ ends = nullptr,
-                                           long long ns = 0)
+// a b - c d with one rounding of the difference (Kahan): the second product's
+// rounding error is added back.
+__device__ __forceinline__ double diff_of_products(double a, double b, double c, double d)
 {
-    double qi[4], dxi[4], dyi[4], mxi[4], mni[4];
-    ld4(q[i], qi);
-    ld4(dq[2 * i], dxi);
-    ld4(dq[2 * i + 1], dyi);
-    ld4(qm[2 * i], mxi);
-    ld4(qm[2 * i + 1], mni);
-    const double e2i = c.eps2[i];
-    double sx[4][4], sy[4][4];
-#pragma unroll
-    for (int d = 0; d < 4; d++)
-#pragma unroll
-        for (int r = 0; r < 4; r++) { sx[d][r] = 0.0; sy[d][r] = 0.0; }
+    const double w = c * d;
+    const double e = fma(-c, d, w);
+    return fma(a, b, -w) + e;
+}
 
-    const int nb = c.nbhs[i];
+// The weight of half-range d's flux difference over an edge with rotated
+// vector sn in point i's residual: the row of the directional 2x2 solve
+// (interior_fluxes_mod.h:140-145 and its likes) times the edge's least-squares
+// weights; twice on the wall (flux_residual_mod.h:29), 0 for a half-range the
+// class does not use.
+__device__ __forceinline__ double flux_weight(const DevCloud &c, int i, int f, int d, double2 sn)
+{
+    if ((f == kWall && d == 2) || (f == kOuter && d == 3)) return 0.0;
+    const double4_32a m = c.fgeo[4 * (size_t)i + d];  // sxx, syy, sxy, 1/det
+    const double w = m.w * (d < 2 ? diff_of_products(m.y, sn.x, m.z, sn.y) : diff_of_products(m.x, sn.y, m.z, sn.x));
+    return f == kWall ? 2.0 * w : w;
+}
+
+// Per edge {weight of its x half-range (xpos if it lies there, else xneg),
+// weight of its y half-range (ypos, else yneg)}, once per cloud.
+__global__ void k_fold_weights(DevCloud c, double2 *__restrict__ e_w64)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= c.n) return;
+    const int f = c.flag[i];
     const long long base = c.slice_base[i >> 5] + (i & 31);
-    for (int j = 0; j < nb; j++) {
+    for (int j = 0; j < c.nbhs[i]; j++) {
         const long long e = base + 32LL * j;
-        const int k = c.e_nbr[e];
-        const double4_32a g = c.e_geo[e];
-        const double2 sw = c.e_sn[e];
         const unsigned dir = c.e_dir[e];
+        const double2 sn = c.e_sn[e];
+        e_w64[e] = make_double2(flux_weight(c, i, f, (dir & kXpos) ? 0 : 1, sn),
+                                flux_weight(c, i, f, (dir & kYpos) ? 2 : 3, sn));
+    }
+}
+
+// The owner's data of the edge walk: q, its gradient, qmax - q, qmin - q and
+// the limiter's eps^2.
+struct Owner {
+    double q[4], dx[4], dy[4], mx[4], mn[4], e2;
+};
+
+__device__ __forceinline__ void load_owner(const DevCloud &c, int i, const double4_32a *__restrict__ q,
+                                           const double4_32a *__restrict__ dq, const double4_32a *__restrict__ qm,
+                                           Owner &o)
+{
+    ld4(q[i], o.q);
+    ld4(dq[2 * i], o.dx);
+    ld4(dq[2 * i + 1], o.dy);
+    ld4(qm[2 * i], o.mx);
+    ld4(qm[2 * i + 1], o.mn);
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+        o.mx[r] -= o.q[r];
+        o.mn[r] -= o.q[r];
+    }
+    o.e2 = c.eps2[i];
+}
+
+// A wall or outer point's half-range flux difference over an edge
+// (wall_fluxes_mod.h, outer_fluxes_mod.h): the class's quadrant flux in x,
+// the split flux in y, times its weight (component 3 twice, as interior_pair).
+__device__ __forceinline__ void boundary_add(int f, const Kin<double> &ki, const Kin<double> &kk, bool x, double s,
+                                             double w, double v[4])
+{
+    double Gi[4], Gk[4];
+    if (x) {
+        const double s2 = f == kOuter ? 1.0 : -1.0;
+        flux_quad(ki, s, s2, Gi);
+        flux_quad(kk, s, s2, Gk);
+    } else {
+        flux_y(ki, s, Gi);
+        flux_y(kk, s, Gk);
+    }
+#pragma unroll
+    for (int r = 0; r < 4; r++) v[r] = fma(r == 3 ? 2.0 * w : w, Gk[r] - Gi[r], v[r]);
+}
+
+// The weighted flux differences of edge e of point i, all half-ranges, in v
+// (component 3 twice): both ends' limited reconstruction and moments once,
+// the edge's x and y half-range by a sign per lane, so that the lanes of a
+// warp do not diverge on their edges' sub-stencils.  An edge with dels == 0
+// (deln == 0) lies in both half-ranges and takes a second, rare pass.
+// ends (or NULL): see flux_residual.
+__device__ __forceinline__ void edge_flux(const DevCloud &c, int i, int f, double nx, double ny, const Owner &o,
+                                          long long e, const double4_32a *__restrict__ q,
+                                          const double4_32a *__restrict__ dq, const double4_32a *__restrict__ qm,
+                                          double v[4], double *__restrict__ ends, long long ns)
+{
+    const int k = c.e_nbr[e];
+    const double4_32a g = c.e_geo[e];
+    const double hx = -0.5 * g.x, hy = -0.5 * g.y;
+    fast64::End si, sk;
+    double t[4];
+    {
         double qk[4], dxk[4], dyk[4], mxk[4], mnk[4];
         ld4(q[k], qk);
         ld4(dq[2 * k], dxk);
         ld4(dq[2 * k + 1], dyk);
         ld4(qm[2 * k], mxk);
         ld4(qm[2 * k + 1], mnk);
-        double ti[4], tk[4];
-        edge_qtilde<double>(g.x, g.y, qi, dxi, dyi, mxi, mni, e2i, qk, dxk, dyk, mxk, mnk, c.eps2[k], ti, tk);
-        Kin<double> ki, kk;
-        double keep_i[3], keep_k[3];
-        end_kin<double>(nx, ny, ti, ki, ends ? keep_i : nullptr);
-        end_kin<double>(nx, ny, tk, kk, ends ? keep_k : nullptr);
-        if (ends) {
-            // planes [12][ns]: per end rho, sqrt(beta), exp(-S1^2), exp(-S2^2), erf(S1), erf(S2)
-            const double v[12] = {ki.rho, keep_i[0], keep_i[1], keep_i[2], ki.E1, ki.E2,
-                                  kk.rho, keep_k[0], keep_k[1], keep_k[2], kk.E1, kk.E2};
+        const double e2k = c.eps2[k];
 #pragma unroll
-            for (int w = 0; w < 12; w++) ends[w * ns + e] = v[w];
+        for (int r = 0; r < 4; r++) {
+            const double dn = fma(hx, dxk[r], hy * dyk[r]);
+            t[r] = fast64::limited(qk[r], dn, (__double2hiint(dn) >= 0 ? mxk[r] : mnk[r]) - qk[r], e2k);
         }
-#define QLSKUM_ACC(D)                                                         \
-        if (dir & (1u << D)) {                                                \
-            double Gi[4], Gk[4];                                              \
-            dir_flux<double, D>(f, ki, Gi);                                   \
-            dir_flux<double, D>(f, kk, Gk);                                   \
-            _Pragma("unroll") for (int r = 0; r < 4; r++) {                   \
-                sx[D][r] = sx[D][r] + (Gk[r] - Gi[r]) * sw.x;                 \
-                sy[D][r] = sy[D][r] + (Gk[r] - Gi[r]) * sw.y;                 \
-            }                                                                 \
-        }
-        QLSKUM_ACC(0)
-        QLSKUM_ACC(1)
-        QLSKUM_ACC(2)
-        QLSKUM_ACC(3)
-#undef QLSKUM_ACC
-    }
-    if (sums) {
-        double *o = sums + 32 * (size_t)i;
-#pragma unroll
-        for (int d = 0; d < 4; d++)
-#pragma unroll
-            for (int r = 0; r < 4; r++) {
-                o[8 * d + r] = sx[d][r];
-                o[8 * d + 4 + r] = sy[d][r];
-            }
+        fast64::end(c, f, nx, ny, t, sk);
+        if (ends) fast64::keep_end(ends + 6 * ns + e, ns, t[3], sk);
     }
 #pragma unroll
-    for (int d = 0; d < 4; d++) {
-        const double4_32a m = c.fgeo[4 * i + d];  // sxx, syy, sxy, 1/det
+    for (int r = 0; r < 4; r++) {
+        const double dn = fma(hx, o.dx[r], hy * o.dy[r]);
+        t[r] = fast64::limited(o.q[r], dn, __double2hiint(dn) >= 0 ? o.mx[r] : o.mn[r], o.e2);
+    }
+    fast64::end(c, f, nx, ny, t, si);
+    if (ends) fast64::keep_end(ends + e, ns, t[3], si);
+
+    const unsigned dir = c.e_dir[e];
+    const double2 w = c.e_w64[e];
+    const bool xp = dir & kXpos, yp = dir & kYpos;
 #pragma unroll
-        for (int r = 0; r < 4; r++)
-            G[d][r] = (d < 2) ? (sx[d][r] * m.y - sy[d][r] * m.z) * m.w
-                              : (sy[d][r] * m.x - sx[d][r] * m.z) * m.w;
+    for (int r = 0; r < 4; r++) v[r] = 0.0;
+    if (f == kInterior) {
+        const unsigned sx = xp ? 0u : 0x80000000u, sy = yp ? 0u : 0x80000000u;
+        fast64::interior_pair(si.k, sx, sy, -w.x, -w.y, v);
+        fast64::interior_pair(sk.k, sx, sy, w.x, w.y, v);
+    } else {
+        boundary_add(f, si.k, sk.k, true, xp ? 1.0 : -1.0, w.x, v);
+        boundary_add(f, si.k, sk.k, false, yp ? 1.0 : -1.0, w.y, v);
+    }
+    if (xp && (dir & kXneg)) {
+        const double w2 = flux_weight(c, i, f, 1, c.e_sn[e]);
+        if (f == kInterior) {
+            fast64::interior_pair(si.k, 0x80000000u, 0u, -w2, 0.0, v);
+            fast64::interior_pair(sk.k, 0x80000000u, 0u, w2, 0.0, v);
+        } else {
+            boundary_add(f, si.k, sk.k, true, -1.0, w2, v);
+        }
+    }
+    if (yp && (dir & kYneg)) {
+        const double w2 = flux_weight(c, i, f, 3, c.e_sn[e]);
+        fast64::interior_pair(si.k, 0u, 0x80000000u, 0.0, -w2, v);
+        fast64::interior_pair(sk.k, 0u, 0x80000000u, 0.0, w2, v);
     }
 }
 
-// flux_residual_mod.h:18-87
-__device__ __forceinline__ void combine(int f, double delta, const double G[4][4], double F[4])
+// The flux residual of point i (flux_residual_mod.h:18-87): delta times the
+// sum of its edges' contributions in the reference's neighbour order.
+__device__ __forceinline__ void point_flux(const DevCloud &c, int i, int f, double nx, double ny, double delta,
+                                           const double4_32a *__restrict__ q, const double4_32a *__restrict__ dq,
+                                           const double4_32a *__restrict__ qm, double F[4],
+                                           double *__restrict__ ends = nullptr, long long ns = 0)
 {
+    Owner o;
+    load_owner(c, i, q, dq, qm, o);
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    const int nb = c.nbhs[i];
+    const long long base = c.slice_base[i >> 5] + (i & 31);
+    for (int j = 0; j < nb; j++) {
+        double v[4];
+        edge_flux(c, i, f, nx, ny, o, base + 32LL * j, q, dq, qm, v, ends, ns);
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        if (f == kWall) F[j] = (2.0 * delta) * (G[0][j] + G[1][j] + G[3][j]);
-        else if (f == kInterior) F[j] = delta * (G[0][j] + G[1][j] + G[2][j] + G[3][j]);
-        else F[j] = delta * (G[0][j] + G[1][j] + G[2][j]);
+        for (int r = 0; r < 4; r++) acc[r] += v[r];
     }
+#pragma unroll
+    for (int r = 0; r < 4; r++) F[r] = (r == 3 ? 0.5 * delta : delta) * acc[r];
 }
 
 __global__ void __launch_bounds__(128) k_flux_residual(DevCloud c, const double4_32a *__restrict__ q,
                                                        const double4_32a *__restrict__ dq, const double4_32a *__restrict__ qm,
                                                        const double *__restrict__ delta, double4_32a *__restrict__ flux_res,
-                                                       double *__restrict__ sums, double *__restrict__ ends, long long ns)
+                                                       double *__restrict__ ends, long long ns)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.n) return;
-    const int f = c.flag[i];
     const double2 nn = c.nrm[i];
-    double G[4][4], F[4];
-    point_flux(c, i, f, nn.x, nn.y, q, dq, qm, G, sums, ends, ns);
-    combine(f, delta[i], G, F);
+    double F[4];
+    point_flux(c, i, c.flag[i], nn.x, nn.y, delta[i], q, dq, qm, F, ends, ns);
     flux_res[i] = mk4(F);
 }
 
@@ -304,6 +372,10 @@ __global__ void __launch_bounds__(BLOCK) k_state_update(DevCloud c, CaseConst K,
 
 // Fused stage: flux residual + SSPRK update of point i, then q and (after the
 // last stage) the wave speed of the new state for the next stage's kernels.
+// Bound by the FP64 pipe, about 240 FP64 instructions per edge and 130 per
+// point.  Measured on 204,800 points (2.05 M edges, inner 3): 2908 us per
+// launch with CUDA's exp / erf / rsqrt, all four half-range fluxes at every
+// edge and 32 directional sums (about 630 per edge), 1066 us in this form.
 template <int BLOCK>
 __global__ void __launch_bounds__(BLOCK) k_flux_update(DevCloud c, CaseConst K, const double4_32a *__restrict__ q,
                                                        const double4_32a *__restrict__ dq,
@@ -320,9 +392,8 @@ __global__ void __launch_bounds__(BLOCK) k_flux_update(DevCloud c, CaseConst K, 
     if (i < c.n) {
         const int f = c.flag[i];
         const double2 nn = c.nrm[i];
-        double G[4][4], F[4], P[4], Q[4];
-        point_flux(c, i, f, nn.x, nn.y, q, dq, qm, G);
-        combine(f, delta[i], G, F);
+        double F[4], P[4], Q[4];
+        point_flux(c, i, f, nn.x, nn.y, delta[i], q, dq, qm, F);
         ld4(prim[i], P);
         r2 = stage_update(K, f, nn.x, nn.y, P, prim_old + i, F, rk);
         prim_next[i] = mk4(P);
@@ -579,6 +650,12 @@ __global__ void __launch_bounds__(256) k_stagnation(int n, const double4_32a *__
 #define QLSKUM_LAUNCHED(L) \
     do { if ((L).launches) ++*(L).launches; } while (0)
 
+void fold_weights(const Launch &L, const DevCloud &c, double2 *e_w64)
+{
+    k_fold_weights<<<grid_for(c.n, 128), 128, 0, L.stream>>>(c, e_w64);
+    QLSKUM_LAUNCHED(L);
+}
+
 void q_variables(const Launch &L, const DevCloud &c, const double4_32a *prim, double4_32a *q)
 {
     k_q_variables<<<grid_for(c.n, 256), 256, 0, L.stream>>>(c.n, prim, q);
@@ -611,9 +688,9 @@ void func_delta(const Launch &L, const DevCloud &c, const double4_32a *prim, dou
 }
 
 void flux_residual(const Launch &L, const DevCloud &c, const double4_32a *q, const double4_32a *dq, const double4_32a *qm,
-                   const double *delta, double4_32a *flux_res, double *sums, double *ends, long long ns)
+                   const double *delta, double4_32a *flux_res, double *ends, long long ns)
 {
-    k_flux_residual<<<grid_for(c.n, 128), 128, 0, L.stream>>>(c, q, dq, qm, delta, flux_res, sums, ends, ns);
+    k_flux_residual<<<grid_for(c.n, 128), 128, 0, L.stream>>>(c, q, dq, qm, delta, flux_res, ends, ns);
     QLSKUM_LAUNCHED(L);
 }
 

@@ -339,6 +339,29 @@ qlskum_status precompute(const qlskum_cloud *c, const qlskum_params *p, Precomp 
     return QLSKUM_OK;
 }
 
+// The tables of the fast FP64 functions (qlskum_fast64.cuh), rounded once from
+// long double (64 or 113 significant bits): computed on first use, the same
+// for every handle.
+struct FastTables {
+    std::vector<double2> gauss;
+    std::vector<double> exp;
+    FastTables() : gauss(kGaussTab), exp(kExpTab)
+    {
+        const long double rpi = 0.564189583547756286948079451560772586L;  // 1 / sqrt(pi)
+        for (int j = 0; j < kGaussTab; j++) {
+            const long double x = j / 1024.0L;
+            gauss[j] = make_double2((double)(rpi * expl(-x * x)), (double)erfl(x));
+        }
+        for (int i = 0; i < kExpTab; i++) exp[i] = (double)exp2l(5.0L + i / 512.0L);
+    }
+};
+
+const FastTables &fast_tables()
+{
+    static const FastTables t;
+    return t;
+}
+
 // parameter_mod.h:4-30: the free stream of a case
 CaseConst case_of(const qlskum_params &p)
 {
@@ -825,12 +848,29 @@ qlskum_status build_geometry(const qlskum_cloud *c, const qlskum_params *p, int 
     up(d_edist, e_dist); up(d_edir, e_dir); up(d_nrm, nrm); up(d_eps2, eps2); up(d_ggeo, ggeo); up(d_fgeo, fgeo);
     up(d_egeo32, e_geo32); up(d_esn32, e_sn32); up(d_eps32, eps2_32); up(d_edist32, e_dist32); up(d_ew32, e_w32); up(d_ew32b, e_w32b);
     up(d_exy32, e_xy32); up(d_egw32, e_gw32);
+    double2 *d_ew64 = nullptr, *d_gauss = nullptr;
+    double *d_exp = nullptr;
+    if (need_fp64) {
+        const FastTables &T = fast_tables();
+        d_ew64 = A.alloc<double2>(ne);
+        d_gauss = A.alloc<double2>(T.gauss.size());
+        d_exp = A.alloc<double>(T.exp.size());
+        up(d_gauss, T.gauss);
+        up(d_exp, T.exp);
+    }
     DevCloud &dc = G.dc;
     dc.n = n; dc.np = G.np; dc.flag = d_flag; dc.nbhs = d_nb; dc.slice_base = d_sb; dc.e_nbr = d_enbr;
     dc.e_geo = d_egeo; dc.e_sn = d_esn; dc.e_dist = d_edist; dc.e_dir = d_edir; dc.nrm = d_nrm; dc.eps2 = d_eps2;
     dc.ggeo = d_ggeo; dc.fgeo = d_fgeo; dc.e_geo32 = d_egeo32; dc.e_sn32 = d_esn32; dc.eps2_32 = d_eps32;
     dc.e_dist32 = d_edist32; dc.e_w32 = d_ew32; dc.e_w32b = d_ew32b; dc.unit_w = unit_w ? 1 : 0; dc.e_xy32 = d_exy32;
     dc.e_gw32 = d_egw32;
+    dc.gauss_tab = d_gauss; dc.exp_tab = d_exp;
+    if (need_fp64 && A.err == cudaSuccess) {
+        Launch L;
+        L.stream = stream;
+        fp64::fold_weights(L, dc, d_ew64);
+        dc.e_w64 = d_ew64;
+    }
     dc.max_nb = 0;
     for (int pp = 0; pp < n; pp++) dc.max_nb = std::max(dc.max_nb, c->nbhs[G.iperm[pp]]);
 
@@ -2876,7 +2916,6 @@ struct Set64 {
     double4_32a *qm[4] = {};
     double *delta = nullptr;
     double4_32a *flux[4] = {};         // each stage's flux residual
-    double *sums[4] = {};              // each stage's directional sums (wall gradients only), [n][32]
     double *ends[4] = {};              // each stage's edge-end transcendentals, [12][ne] (fp64::flux_residual)
 };
 
@@ -2912,7 +2951,6 @@ struct AdjBuf {
     Set32 set0;
     std::vector<Set32> sets;
     DeviceArena set_arena;             // the on-demand sets (FP32 or FP64, one kind at a time)
-    bool sets_geo = false;             // the FP64 sets carry the directional sums
     float4 *bF32 = nullptr;            // bar of the flux residual
     float4 *bs32 = nullptr;            // bar of the weighted sums (delta * bF)
     AdjT T;                            // the edge list transposed (mixed reverse)
@@ -3070,12 +3108,9 @@ void alloc_set32(DeviceArena &A, size_t np, int ni, Set32 &st)
     st.cs32 = A.alloc<float>(np);
 }
 
-// The FP64 arrays of one stage-data set (its states are assigned by the
-// caller); geo: also the directional sums of the wall-gradient reverse.
-void alloc_set64(DeviceArena &A, size_t np, size_t ne, int ni, Set64 &st, bool geo)
+// The FP64 arrays of one stage-data set (its states are assigned by the caller).
+void alloc_set64(DeviceArena &A, size_t np, size_t ne, int ni, Set64 &st)
 {
-    if (geo)
-        for (auto &p : st.sums) p = A.alloc<double>(32 * np);
     for (auto &p : st.ends) p = A.alloc<double>(12 * ne);
     for (auto &p : st.q) p = A.alloc<double4_32a>(np);
     for (auto &p : st.qm) p = A.alloc<double4_32a>(2 * np);
@@ -3085,10 +3120,9 @@ void alloc_set64(DeviceArena &A, size_t np, size_t ne, int ni, Set64 &st, bool g
     for (auto &p : st.flux) p = A.alloc<double4_32a>(np);
 }
 
-size_t set64_bytes(size_t np, size_t ne, int ni, bool geo)
+size_t set64_bytes(size_t np, size_t ne, int ni)
 {
-    return np * (5 * sizeof(double4_32a) + 4 * 32 + 4 * 64 + 4 * (size_t)(ni + 1) * 64 + 8 + 4 * 32 +
-                 (geo ? 4 * 32 * sizeof(double) : 0)) +
+    return np * (5 * sizeof(double4_32a) + 4 * 32 + 4 * 64 + 4 * (size_t)(ni + 1) * 64 + 8 + 4 * 32) +
            4 * 12 * ne * sizeof(double);
 }
 
@@ -3123,7 +3157,7 @@ qlskum_status adj_alloc(qlskum_handle *h, bool geo, bool need64, bool need32)
     a->buinf = A.alloc<double>(4);  // free-stream velocity bars, then the initial-state sums
     slice_bases(h, &a->ne);
     if (need64) {
-        alloc_set64(A, np, a->ne, a->ni, a->set64, geo);
+        alloc_set64(A, np, a->ne, a->ni, a->set64);
         for (int k = 0; k < 5; k++) a->set64.P[k] = a->P[k];
         a->bq = A.alloc<double4_32a>(np);
         for (auto *p : {&a->bdqA, &a->bdqB, &a->bqm}) *p = A.alloc<double4_32a>(2 * np);
@@ -3231,8 +3265,8 @@ void adj_stage_forward(qlskum_handle *h, Set64 &st, int s)
     fp64::q_variables(h->L, c, st.P[s], st.q[s]);
     fp64::q_derivatives(h->L, c, st.q[s], adj_dq(st, ni, s, 0), st.qm[s], nullptr, nullptr, 0.0);
     for (int j = 1; j <= ni; j++) fp64::q_inner(h->L, c, st.q[s], adj_dq(st, ni, s, j - 1), adj_dq(st, ni, s, j));
-    fp64::flux_residual(h->L, c, st.q[s], adj_dq(st, ni, s, ni), st.qm[s], st.delta, st.flux[s], st.sums[s],
-                        st.ends[s], (long long)h->adj->ne);
+    fp64::flux_residual(h->L, c, st.q[s], adj_dq(st, ni, s, ni), st.qm[s], st.delta, st.flux[s], st.ends[s],
+                        (long long)h->adj->ne);
 }
 
 // The four stage states of one iteration from st.P[0] (fpi_solver_mod.h:14-40)
@@ -3264,7 +3298,7 @@ void adj_stage_reverse(qlskum_handle *h, const Set64 &st, int s, const AdjView &
     zero(h, a->bq, sizeof(double4_32a) * np);
     zero(h, a->bdqA, sizeof(double4_32a) * 2 * np);
     zero(h, a->bqm, sizeof(double4_32a) * 2 * np);
-    adjl::flux(h->L, v, st.q[s], adj_dq(st, ni, s, ni), st.qm[s], st.delta, st.flux[s], st.sums[s], st.ends[s],
+    adjl::flux(h->L, v, st.q[s], adj_dq(st, ni, s, ni), st.qm[s], st.delta, st.flux[s], st.ends[s],
                (long long)a->ne, a->bF, a->bq,
                a->bdqA, a->bqm, a->bdelta);
     for (int j = ni; j >= 1; j--) {
@@ -3301,8 +3335,7 @@ float4 *adj_dq32(const Set32 &st, int ni, int s, int j) { return st.dq32[(size_t
 bool adj_sets(qlskum_handle *h, int count, bool f64)
 {
     AdjBuf *a = h->adj;
-    const bool geo = f64 && a->geo;
-    if ((f64 ? (int)a->sets64.size() : (int)a->sets.size()) >= count && (!geo || a->sets_geo)) return true;
+    if ((f64 ? (int)a->sets64.size() : (int)a->sets.size()) >= count) return true;
     auto drop = [&]() {
         a->sets.clear();
         a->sets64.clear();
@@ -3313,13 +3346,13 @@ bool adj_sets(qlskum_handle *h, int count, bool f64)
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return false;
     // keep a quarter of the free memory for everything else
-    const size_t each = f64 ? set64_bytes(h->np, a->ne, a->ni, geo) : set32_bytes(h->np, a->ni);
+    const size_t each = f64 ? set64_bytes(h->np, a->ne, a->ni) : set32_bytes(h->np, a->ni);
     if ((double)each * count > 0.75 * (double)free_b) return false;
     std::vector<double4_32a *> p0;
     if (f64) {
         a->sets64.resize(count);
         for (auto &st : a->sets64) {
-            alloc_set64(a->set_arena, h->np, a->ne, a->ni, st, geo);
+            alloc_set64(a->set_arena, h->np, a->ne, a->ni, st);
             for (auto &p : st.P) p = a->set_arena.alloc<double4_32a>(h->np);
             p0.push_back(st.P[0]);
         }
@@ -3337,7 +3370,6 @@ bool adj_sets(qlskum_handle *h, int count, bool f64)
         return false;
     }
     for (auto *p : p0) zero(h, p, sizeof(double4_32a) * h->np);
-    a->sets_geo = geo;
     return true;
 }
 

@@ -23,6 +23,7 @@
 namespace qlskum {
 
 enum : int { kWall = 0, kInterior = 1, kOuter = 2 };
+constexpr int kGaussTab = 6145, kExpTab = 512;
 enum : unsigned { kXpos = 1u, kXneg = 2u, kYpos = 4u, kYneg = 8u };
 
 struct CaseConst;
@@ -42,6 +43,11 @@ struct DevCloud {
     const double *eps2 = nullptr;
     const double4_32a *ggeo = nullptr;           // [np]
     const double4_32a *fgeo = nullptr;           // [np][4]
+    // FP64 form: the folded flux weights of e_w32 (below) in FP64, and the
+    // tables of the fast FP64 functions (qlskum_fast64.cuh)
+    const double2 *e_w64 = nullptr;
+    const double2 *gauss_tab = nullptr;      // [kGaussTab]
+    const double *exp_tab = nullptr;         // [kExpTab]
     // mixed-precision copies of the per-edge geometry (FP32)
     const float4 *e_geo32 = nullptr;         // delx, dely, w*delx, w*dely
     const float2 *e_sn32 = nullptr;          // dels*w, deln*w
@@ -200,11 +206,10 @@ namespace adjl {
 void update(const Launch &L, const AdjView &a, const CaseConst &K, const double4_32a *Pin, const double4_32a *Pold,
             const double4_32a *Pout, int rk, double4_32a *bP, double4_32a *bPold, double4_32a *bF, double *buinf);
 // flux: the stage's flux residual (the bar of delta without geometry bars);
-// sums: its directional sums (fp64::flux_residual) for the geometry bars, or
-// NULL (recomputed); ends: the edge ends' kept transcendentals
+// ends: the edge ends' kept transcendentals
 // (fp64::flux_residual's ends, ns slots), or NULL (recomputed)
 void flux(const Launch &L, const AdjView &a, const double4_32a *q, const double4_32a *dq, const double4_32a *qm,
-          const double *delta, const double4_32a *flux, const double *sums, const double *ends, long long ns,
+          const double *delta, const double4_32a *flux, const double *ends, long long ns,
           const double4_32a *bF, double4_32a *bq, double4_32a *bdq, double4_32a *bqm, double *bdelta);
 void inner(const Launch &L, const AdjView &a, const double4_32a *q, const double4_32a *dq_in,
            const double4_32a *bdq_out, double4_32a *bq, double4_32a *bdq_in);
@@ -271,19 +276,19 @@ void delta(const Launch &L, const DevCloud &c, const double4_32a *P, const float
 
 // ---------------------------------------------------------- FP64 kernels (qlskum_fp64.cu)
 namespace fp64 {
+// the folded flux weights DevCloud::e_w64 from the cloud's moments and rotated edge vectors
+void fold_weights(const Launch &L, const DevCloud &c, double2 *e_w64);
 void q_variables(const Launch &L, const DevCloud &c, const double4_32a *prim, double4_32a *q);
 void derived(const Launch &L, const DevCloud &c, const double4_32a *prim, double4_32a *q, double *cspeed);
 void q_derivatives(const Launch &L, const DevCloud &c, const double4_32a *q, double4_32a *dq, double4_32a *qm,
                    const double *cspeed, double *delta, double cfl);
 void q_inner(const Launch &L, const DevCloud &c, const double4_32a *q, const double4_32a *dq_in, double4_32a *dq_out);
 void func_delta(const Launch &L, const DevCloud &c, const double4_32a *prim, double *delta, double cfl);
-// sums (or NULL): each point's directional sums {sx[d][r], sy[d][r]}, [n][32] doubles.
 // ends (or NULL): per edge slot of the ns slots, the owner's and the
 // neighbour's end's rho, sqrt(beta), exp(-S1^2), exp(-S2^2), erf(S1),
 // erf(S2), as 12 planes of ns doubles (read back by the flux reverse).
 void flux_residual(const Launch &L, const DevCloud &c, const double4_32a *q, const double4_32a *dq, const double4_32a *qm,
-                   const double *delta, double4_32a *flux_res, double *sums = nullptr, double *ends = nullptr,
-                   long long ns = 0);
+                   const double *delta, double4_32a *flux_res, double *ends = nullptr, long long ns = 0);
 void state_update(const Launch &L, const DevCloud &c, const CaseConst &k, double4_32a *prim, const double4_32a *prim_old,
                   const double4_32a *flux_res, int rk, const Reduce &R);
 void flux_update(const Launch &L, const DevCloud &c, const CaseConst &k, const double4_32a *q, const double4_32a *dq,

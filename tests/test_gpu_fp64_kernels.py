@@ -1,0 +1,90 @@
+"""The FP64 flux kernels' fast functions and launch forms against the oracle.
+
+Bound of the flux residual: delta sum_e c_e (G_k - G_i) over a point's edges,
+each flux G correct to about 10 ulps of its scale and 8 S^2 more for the
+density, exp of a sum whose terms are S^2 large (S^2 = beta |u|^2); the
+weights c_e of a half range sum to at most 2.5 / min_dist (the cloud
+generator's bound); four half ranges, two ends: 20 (10 + 8 S^2) ulps of
+(delta / min_dist) max |G|.  The disturbances are small against the speed of
+sound, so that an edge end's state stays near the points' at every Mach number.
+"""
+import numpy as np
+import pytest
+
+import qlskum_oracle
+
+pytestmark = pytest.mark.gpu
+
+EPS = 2.0 ** -53
+
+
+def disturbed(cloud, mach, seed=5):
+    rng = np.random.default_rng(seed)
+    P = np.empty((cloud.n, 4))
+    P[:, 0] = 1.0 + 0.05 * rng.uniform(-1, 1, cloud.n)
+    P[:, 1] = 0.97 * mach + 0.02 * rng.uniform(-1, 1, cloud.n)
+    P[:, 2] = 0.15 * mach + 0.02 * rng.uniform(-1, 1, cloud.n)
+    P[:, 3] = (1.0 + 0.05 * rng.uniform(-1, 1, cloud.n)) / 1.4
+    return P
+
+
+def flux_bound(cloud, P, delta):
+    """Per component: the module's bound with |u| + 3 sqrt(p / rho) as the speed of the largest flux."""
+    U = float((np.hypot(P[:, 1], P[:, 2]) + 3 * np.sqrt(P[:, 3] / P[:, 0])).max())
+    G = P[:, 0].max() * U * np.array([1.0, U, U, U * U])
+    S2 = float((0.5 * P[:, 0] / P[:, 3] * (P[:, 1] ** 2 + P[:, 2] ** 2)).max())
+    return 20 * (10 + 8 * S2) * EPS * float((delta / cloud.min_dist).max()) * G
+
+
+def stage(s, P, inner):
+    s.set_prim(P)
+    s.func_delta()
+    s.eval_q_variables()
+    s.eval_q_derivatives()
+    for _ in range(inner):
+        s.eval_q_inner_loop()
+        s.eval_update_innerloop()
+    s.cal_flux_residual()
+
+
+# 9: |S| beyond the tables (the library's exp and erf); 0.01: |S| next to 0.
+# Without jitter the cloud has edges on both sides of an axis (dels or deln == 0).
+@pytest.mark.parametrize("mach", [0.01, 0.85, 3.0, 9.0])
+@pytest.mark.parametrize("power", [0.0, -2.0])
+def test_flux_residual_over_the_mach_range(mach, power):
+    import qlskum
+    from qlskum import cloudgen
+    c = cloudgen.make_cloud(n_wall=48, n_layers=21, first_spacing=5e-3, radius=5.0, seed=3, jitter=0.0)
+    kw = dict(mach=mach, aoa=2.0, cfl=0.2, vl_const=50.0, power=power, inner_iterations=1)
+    P = disturbed(c, mach)
+    s, o = qlskum.Solver(c, **kw), qlskum_oracle.Oracle(c, **kw)
+    o.set_prim(P)
+    o.func_delta()
+    o.eval_q_variables()
+    o.eval_q_derivatives()
+    o.eval_q_inner_loop()
+    o.eval_update_innerloop()
+    o.cal_flux_residual()
+    counts, _ = s.connectivity()
+    interior = c.flag_1 == 1
+    assert (counts[interior].sum(1) > 2 * c.nbhs[interior]).any()  # both-sides edges
+    stage(s, P, 1)
+    err = np.abs(s.field(qlskum.FIELD_FLUX_RES) - o.flux_res).max(0)
+    assert (err <= flux_bound(c, P, o.delta)).all(), (err, flux_bound(c, P, o.delta))
+
+
+def test_nonfinite_state_is_reported():
+    """A NaN in the state goes through the fast functions' library paths and is reported."""
+    import qlskum
+    from conftest import golden_cloud
+    c = golden_cloud("cloud_small")
+    s = qlskum.Solver(c, mach=0.63, aoa=2.0, cfl=0.2, vl_const=50.0, inner_iterations=0)
+    P = disturbed(c, 0.63)
+    P[c.n // 2, 3] = np.nan
+    s.set_prim(P)
+    with pytest.raises(qlskum.QlskumError) as e:
+        s.q_lskum(1)
+    assert e.value.status == 3
+    s.set_prim(disturbed(c, 0.63))
+    s.q_lskum(1)
+    assert np.isfinite(s.prim).all()
