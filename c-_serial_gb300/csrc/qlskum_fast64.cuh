@@ -150,8 +150,8 @@ __device__ __forceinline__ void end(const DevCloud &c, int f, double nx, double 
 {
     double qs = t[1], qn = t[2];
     if (f != kInterior) {
-        qs = fma(t[1], ny, -(t[2] * nx));
-        qn = fma(t[1], nx, t[2] * ny);
+        qs = fma(t[1], ny, -__dmul_rn(t[2], nx));
+        qn = fma(t[1], nx, __dmul_rn(t[2], ny));
     }
     const double b = -2.0 * t[3];
     const double r = rsqrt64(b);
@@ -161,7 +161,7 @@ __device__ __forceinline__ void end(const DevCloud &c, int f, double nx, double 
     s.k.pbr = h + h;
     s.k.ut = qs * s.k.pbr;
     s.k.un = qn * s.k.pbr;
-    s.k.usq = fma(s.k.ut, s.k.ut, s.k.un * s.k.un);
+    s.k.usq = fma(s.k.ut, s.k.ut, __dmul_rn(s.k.un, s.k.un));
     s.k.rho = exp32(fma(S1, S1, fma(S2, S2, t[0])), c.exp_tab) * (h * h * r);
     gauss_erf(S1, c.gauss_tab, s.e1, s.k.E1);
     gauss_erf(S2, c.gauss_tab, s.e2, s.k.E2);
@@ -182,24 +182,130 @@ __device__ __forceinline__ void keep_end(double *__restrict__ o, long long ns, d
     o[5 * ns] = s.k.E2;
 }
 
-// Adds one interior end's weighted pair wx Gx(s1) + wy Gy(s2) to v.  With
+// Adds one end's weighted split-flux pair wx Gx(s1) + wy Gy(s2) to v.  With
 // A = (1 + s E) / 2, al = wx rho A1, ga = wy rho A2 and
 // be = wx rho s1 B1 + wy rho s2 B2, the pair (split_fluxes_mod.h:14-84 and
 // :86-164) is
 //   v0 = al ut + ga un + be,  v1 = ut v0 + al p/rho,  v2 = un v0 + ga p/rho,
 //   v3 = (usq v0 + p/rho (7 v0 - be)) / 2;  twice v3 is added.
-// sx, sy: the sign bits of s1, s2 (0 for +1).
-__device__ __forceinline__ void interior_pair(const Kin<double> &k, unsigned sx, unsigned sy, double wx, double wy,
-                                              double v[4])
+// sx, sy: the sign bits of s1, s2 (0 for +1).  Every product is in an explicit
+// fma or alone, here and below, so that no kernel contracts it differently.
+__device__ __forceinline__ void split_pair(const Kin<double> &k, unsigned sx, unsigned sy, double wx, double wy,
+                                           double v[4])
 {
     const double wr = wx * k.rho, yr = wy * k.rho;
     const double al = wr * fma(0.5, flip(k.E1, sx), 0.5), ga = yr * fma(0.5, flip(k.E2, sy), 0.5);
-    const double be = fma(flip(wr, sx), k.B1, flip(yr, sy) * k.B2);
+    const double be = fma(flip(wr, sx), k.B1, __dmul_rn(flip(yr, sy), k.B2));
     const double v0 = fma(al, k.ut, fma(ga, k.un, be));
     v[0] += v0;
     v[1] = fma(k.ut, v0, fma(al, k.pbr, v[1]));
     v[2] = fma(k.un, v0, fma(ga, k.pbr, v[2]));
     v[3] = fma(k.pbr, fma(7.0, v0, -be), fma(k.usq, v0, v[3]));
+}
+
+// Adds w times a boundary end's quadrant flux (quadrant_fluxes_mod.h:6-211),
+// the t half range of sign bit sx times the n half range of sign bit sn:
+//   f = ut A1 + s1 B1,  m = un A2 + s2 B2,
+//   G0 = rho A2 f,  G1 = rho A2 (ut f + p/rho A1),  G2 = rho f m,
+//   G3 = rho (A2 (usq f + p/rho (7 f - s1 B1)) + s2 un B2 f) / 2; twice G3 is added.
+__device__ __forceinline__ void quad_x(const Kin<double> &k, unsigned sx, unsigned sn, double w, double v[4])
+{
+    const double A1 = fma(0.5, flip(k.E1, sx), 0.5), A2 = fma(0.5, flip(k.E2, sn), 0.5);
+    const double B1 = flip(k.B1, sx), B2 = flip(k.B2, sn);
+    const double wr = w * k.rho, wa = wr * A2;
+    const double f = fma(k.ut, A1, B1);
+    const double wf = wr * f;
+    v[0] = fma(wa, f, v[0]);
+    v[1] = fma(wa, fma(k.ut, f, __dmul_rn(k.pbr, A1)), v[1]);
+    v[2] = fma(wf, fma(k.un, A2, B2), v[2]);
+    v[3] = fma(wa, fma(k.usq, f, __dmul_rn(k.pbr, fma(7.0, f, -B1))), fma(wf, __dmul_rn(k.un, B2), v[3]));
+}
+
+// ------------------------------------------------------------ points
+// The point formulas of qlskum_math.cuh with every multiply-add explicit, so
+// that the module, fused and recording kernels, whatever the compiler inlines
+// around them, give the same bits.
+
+// q_variables_mod.h:19-33
+__device__ __forceinline__ void q_of(const double P[4], double Q[4])
+{
+    const double beta = ratio64(0.5 * P[0], P[3]);
+    const double usq = fma(P[1], P[1], __dmul_rn(P[2], P[2]));
+    Q[0] = fma(-beta, usq, fma(2.5, log(beta), log(P[0])));
+    const double b2 = 2.0 * beta;
+    Q[1] = b2 * P[1];
+    Q[2] = b2 * P[2];
+    Q[3] = -b2;
+}
+
+// |u| + 3 sqrt(p / rho) of state_update_mod.h:483-485
+__device__ __forceinline__ double wave_speed(const double P[4])
+{
+    const double u = __dsqrt_rn(fma(P[1], P[1], __dmul_rn(P[2], P[2])));
+    return fma(3.0, __dsqrt_rn(ratio64(P[3], P[0])), u);
+}
+
+// primitive_to_conserved (state_update_mod.h:18-33), conserved_vector_Ubar
+// (:35-90: the free stream's inflowing half range plus the state's outflowing
+// one) for an outer point.
+__device__ __forceinline__ void conserved(const CaseConst &K, int f, double nx, double ny, const double P[4], double U[4])
+{
+    if (f != kOuter) {
+        const double t1 = P[0] * P[1], t2 = P[0] * P[2];
+        U[0] = P[0];
+        U[3] = fma(2.5, P[3], 0.5 * fma(t1, P[1], __dmul_rn(t2, P[2])));
+        U[1] = fma(t1, ny, -__dmul_rn(t2, nx));
+        U[2] = fma(t1, nx, __dmul_rn(t2, ny));
+        return;
+    }
+#pragma unroll
+    for (int r = 0; r < 4; r++) U[r] = 0.0;
+#pragma unroll 1
+    for (int h = 0; h < 2; h++) {
+        const double s = h ? 1.0 : -1.0;
+        const double rho = h ? P[0] : K.rho_inf, u1 = h ? P[1] : K.u1_inf, u2 = h ? P[2] : K.u2_inf,
+                     p = h ? P[3] : K.pr_inf;
+        const double ut = fma(u1, ny, -__dmul_rn(u2, nx)), un = fma(u1, nx, __dmul_rn(u2, ny));
+        const double beta = ratio64(0.5 * rho, p);
+        const double S = un * __dsqrt_rn(beta);
+        const double B = s * ratio64(exp(-__dmul_rn(S, S)), 2.0 * __dsqrt_rn(K.pi * beta));
+        const double A = fma(s, 0.5 * erf(S), 0.5);
+        const double e = ratio64(p, rho * (K.gamma - 1.0)) + 0.5 * fma(ut, ut, __dmul_rn(un, un));
+        const double m = rho * A;
+        U[0] += m;
+        U[1] = fma(m, ut, U[1]);
+        U[2] = fma(rho, fma(un, A, B), U[2]);
+        U[3] = fma(m, e, fma(0.5 * rho, __dmul_rn(un, B), U[3]));
+    }
+}
+
+// One SSPRK stage of one point (state_update_mod.h:111-282): P is updated in
+// place; returns the point's res_sqr (0 on outer points).
+__device__ __forceinline__ double stage(const CaseConst &K, int f, double nx, double ny, double P[4],
+                                        const double4_32a *__restrict__ prim_old_i, const double F[4], int rk)
+{
+    double U[4];
+    conserved(K, f, nx, ny, P, U);
+    const double rho = U[0];
+    if (rk != 3) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) U[j] = fma(-0.5, F[j], U[j]);
+    } else {
+        double Po[4], Uo[4];
+        ld4(*prim_old_i, Po);
+        conserved(K, f, nx, ny, Po, Uo);
+#pragma unroll
+        for (int j = 0; j < 4; j++) U[j] = fma(2.0 / 3.0, Uo[j], __dmul_rn(1.0 / 3.0, fma(-0.5, F[j], U[j])));
+    }
+    if (f == kWall) U[2] = 0.0;
+    const double m1 = fma(U[1], ny, __dmul_rn(U[2], nx)), m2 = fma(U[2], ny, -__dmul_rn(U[1], nx));
+    const double d = U[0] - rho;
+    const double inv = rcp64(U[0]);
+    P[0] = U[0];
+    P[1] = m1 * inv;
+    P[2] = m2 * inv;
+    P[3] = fma(0.4, U[3], -__dmul_rn(0.2 * inv, fma(m1, m1, __dmul_rn(m2, m2))));
+    return f == kOuter ? 0.0 : __dmul_rn(d, d);
 }
 
 }  // namespace fast64

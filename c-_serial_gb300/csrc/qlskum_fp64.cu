@@ -8,9 +8,9 @@
 // results differ from the serial reference by those roundings: 1e-10 relative
 // after 1000 iterations (the parity tests).
 //
-// One thread per point; the point's edges are walked in the reference's
-// neighbour order from the sliced-ELL edge arrays (coalesced across the warp),
-// neighbour state is gathered through L1/L2 (points are Morton ordered, so
+// One thread per point, or in the flux kernels several (flux_shape); a point's
+// edges are summed in the reference's neighbour order, read from the
+// sliced-ELL edge arrays (coalesced across the warp); neighbour state is gathered through L1/L2 (points are Morton ordered, so
 // most neighbours of a block's points are cache-resident).  All geometry that
 // does not change between iterations (edge vectors, least-squares moments,
 // 1/det, limiter epsilon) is precomputed on the host in the reference's
@@ -18,6 +18,7 @@
 // instructions, its scarce resource.
 #include "qlskum_math.cuh"
 #include "qlskum_fast64.cuh"
+#include <type_traits>
 
 namespace qlskum {
 namespace fp64 {
@@ -33,7 +34,7 @@ __global__ void k_q_variables(int n, const double4_32a *__restrict__ prim, doubl
     if (i >= n) return;
     double P[4], Q[4];
     ld4(prim[i], P);
-    prim_to_q(P[0], P[1], P[2], P[3], Q);
+    fast64::q_of(P, Q);
     q[i] = mk4(Q);
 }
 
@@ -45,9 +46,9 @@ __global__ void k_derived(int n, const double4_32a *__restrict__ prim, double4_3
     if (i >= n) return;
     double P[4], Q[4];
     ld4(prim[i], P);
-    prim_to_q(P[0], P[1], P[2], P[3], Q);
+    fast64::q_of(P, Q);
     q[i] = mk4(Q);
-    cs[i] = wave_speed(P);
+    cs[i] = fast64::wave_speed(P);
 }
 
 // ----------------------------------------------------------- gradients
@@ -154,7 +155,7 @@ __global__ void k_func_delta(DevCloud c, const double4_32a *__restrict__ prim, d
         const long long e = base + 32LL * j;
         double P[4];
         ld4(prim[c.e_nbr[e]], P);
-        double delta_t = c.e_dist[e] / wave_speed(P);
+        double delta_t = c.e_dist[e] / fast64::wave_speed(P);
         delta_t = cfl * delta_t;
         if (min_delt > delta_t) min_delt = delta_t;
     }
@@ -225,25 +226,6 @@ __device__ __forceinline__ void load_owner(const DevCloud &c, int i, const doubl
     o.e2 = c.eps2[i];
 }
 
-// A wall or outer point's half-range flux difference over an edge
-// (wall_fluxes_mod.h, outer_fluxes_mod.h): the class's quadrant flux in x,
-// the split flux in y, times its weight (component 3 twice, as interior_pair).
-__device__ __forceinline__ void boundary_add(int f, const Kin<double> &ki, const Kin<double> &kk, bool x, double s,
-                                             double w, double v[4])
-{
-    double Gi[4], Gk[4];
-    if (x) {
-        const double s2 = f == kOuter ? 1.0 : -1.0;
-        flux_quad(ki, s, s2, Gi);
-        flux_quad(kk, s, s2, Gk);
-    } else {
-        flux_y(ki, s, Gi);
-        flux_y(kk, s, Gk);
-    }
-#pragma unroll
-    for (int r = 0; r < 4; r++) v[r] = fma(r == 3 ? 2.0 * w : w, Gk[r] - Gi[r], v[r]);
-}
-
 // The weighted flux differences of edge e of point i, all half-ranges, in v
 // (component 3 twice): both ends' limited reconstruction and moments once,
 // the edge's x and y half-range by a sign per lane, so that the lanes of a
@@ -270,7 +252,7 @@ __device__ __forceinline__ void edge_flux(const DevCloud &c, int i, int f, doubl
         const double e2k = c.eps2[k];
 #pragma unroll
         for (int r = 0; r < 4; r++) {
-            const double dn = fma(hx, dxk[r], hy * dyk[r]);
+            const double dn = fma(hx, dxk[r], __dmul_rn(hy, dyk[r]));
             t[r] = fast64::limited(qk[r], dn, (__double2hiint(dn) >= 0 ? mxk[r] : mnk[r]) - qk[r], e2k);
         }
         fast64::end(c, f, nx, ny, t, sk);
@@ -278,7 +260,7 @@ __device__ __forceinline__ void edge_flux(const DevCloud &c, int i, int f, doubl
     }
 #pragma unroll
     for (int r = 0; r < 4; r++) {
-        const double dn = fma(hx, o.dx[r], hy * o.dy[r]);
+        const double dn = fma(hx, o.dx[r], __dmul_rn(hy, o.dy[r]));
         t[r] = fast64::limited(o.q[r], dn, __double2hiint(dn) >= 0 ? o.mx[r] : o.mn[r], o.e2);
     }
     fast64::end(c, f, nx, ny, t, si);
@@ -286,122 +268,165 @@ __device__ __forceinline__ void edge_flux(const DevCloud &c, int i, int f, doubl
 
     const unsigned dir = c.e_dir[e];
     const double2 w = c.e_w64[e];
-    const bool xp = dir & kXpos, yp = dir & kYpos;
+    const unsigned neg = 0x80000000u;
+    const unsigned sx = (dir & kXpos) ? 0u : neg, sy = (dir & kYpos) ? 0u : neg;
+    const bool inner = f == kInterior;
+    const unsigned s2 = f == kOuter ? 0u : neg;  // the n half range of the quadrant flux
 #pragma unroll
     for (int r = 0; r < 4; r++) v[r] = 0.0;
-    if (f == kInterior) {
-        const unsigned sx = xp ? 0u : 0x80000000u, sy = yp ? 0u : 0x80000000u;
-        fast64::interior_pair(si.k, sx, sy, -w.x, -w.y, v);
-        fast64::interior_pair(sk.k, sx, sy, w.x, w.y, v);
-    } else {
-        boundary_add(f, si.k, sk.k, true, xp ? 1.0 : -1.0, w.x, v);
-        boundary_add(f, si.k, sk.k, false, yp ? 1.0 : -1.0, w.y, v);
+    const double wx = inner ? w.x : 0.0;
+    fast64::split_pair(si.k, sx, sy, -wx, -w.y, v);
+    fast64::split_pair(sk.k, sx, sy, wx, w.y, v);
+    if (!inner) {
+        fast64::quad_x(si.k, sx, s2, -w.x, v);
+        fast64::quad_x(sk.k, sx, s2, w.x, v);
     }
-    if (xp && (dir & kXneg)) {
+    if ((dir & (kXpos | kXneg)) == (kXpos | kXneg)) {
         const double w2 = flux_weight(c, i, f, 1, c.e_sn[e]);
-        if (f == kInterior) {
-            fast64::interior_pair(si.k, 0x80000000u, 0u, -w2, 0.0, v);
-            fast64::interior_pair(sk.k, 0x80000000u, 0u, w2, 0.0, v);
+        if (inner) {
+            fast64::split_pair(si.k, neg, 0u, -w2, 0.0, v);
+            fast64::split_pair(sk.k, neg, 0u, w2, 0.0, v);
         } else {
-            boundary_add(f, si.k, sk.k, true, -1.0, w2, v);
+            fast64::quad_x(si.k, neg, s2, -w2, v);
+            fast64::quad_x(sk.k, neg, s2, w2, v);
         }
     }
-    if (yp && (dir & kYneg)) {
+    if ((dir & (kYpos | kYneg)) == (kYpos | kYneg)) {
         const double w2 = flux_weight(c, i, f, 3, c.e_sn[e]);
-        fast64::interior_pair(si.k, 0u, 0x80000000u, 0.0, -w2, v);
-        fast64::interior_pair(sk.k, 0u, 0x80000000u, 0.0, w2, v);
+        fast64::split_pair(si.k, 0u, neg, 0.0, -w2, v);
+        fast64::split_pair(sk.k, 0u, neg, 0.0, w2, v);
     }
 }
 
-// The flux residual of point i (flux_residual_mod.h:18-87): delta times the
-// sum of its edges' contributions in the reference's neighbour order.
-__device__ __forceinline__ void point_flux(const DevCloud &c, int i, int f, double nx, double ny, double delta,
-                                           const double4_32a *__restrict__ q, const double4_32a *__restrict__ dq,
-                                           const double4_32a *__restrict__ qm, double F[4],
-                                           double *__restrict__ ends = nullptr, long long ns = 0)
+// The flux residual of the block's P points (flux_residual_mod.h:18-87):
+// delta times the sum of a point's edge contributions.  Thread t takes point
+// t % P and every T / P-th of its edges from t / P on; the contributions meet
+// in shared memory and are added in the reference's neighbour order, so the
+// result does not depend on P.  Returns true to the thread that holds its
+// point's F (threads below P with a point).
+constexpr int kFluxThreads = 128;
+
+template <int P>
+__device__ __forceinline__ bool block_flux(const DevCloud &c, const double4_32a *__restrict__ q,
+                                           const double4_32a *__restrict__ dq, const double4_32a *__restrict__ qm,
+                                           const double *__restrict__ delta, double F[4], double *__restrict__ ends,
+                                           long long ns)
 {
-    Owner o;
-    load_owner(c, i, q, dq, qm, o);
-    double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    const int nb = c.nbhs[i];
-    const long long base = c.slice_base[i >> 5] + (i & 31);
-    for (int j = 0; j < nb; j++) {
-        double v[4];
-        edge_flux(c, i, f, nx, ny, o, base + 32LL * j, q, dq, qm, v, ends, ns);
+    constexpr int T = kFluxThreads;
+    __shared__ double sv[4 * P * kMaxNbhs];
+    const int p = threadIdx.x % P, i = blockIdx.x * P + p;
+    const bool has = i < c.n;
+    const int nb = has ? c.nbhs[i] : 0;
+    if (has) {
+        const int f = c.flag[i];
+        const double2 nn = c.nrm[i];
+        const long long base = c.slice_base[i >> 5] + (i & 31);
+        Owner o;
+        load_owner(c, i, q, dq, qm, o);
+        for (int j = threadIdx.x / P; j < nb; j += T / P) {
+            double v[4];
+            edge_flux(c, i, f, nn.x, nn.y, o, base + 32LL * j, q, dq, qm, v, ends, ns);
 #pragma unroll
-        for (int r = 0; r < 4; r++) acc[r] += v[r];
+            for (int r = 0; r < 4; r++) sv[(4 * j + r) * P + p] = v[r];
+        }
     }
+    // component r = t / P of point t % P; its sum replaces edge 0's contribution
+    __syncthreads();
+    for (int r = threadIdx.x / P; r < 4; r += T / P) {
+        double a = 0.0;
+        for (int j = 0; j < nb; j++) a += sv[(4 * j + r) * P + p];
+        sv[r * P + p] = a;
+    }
+    __syncthreads();
+    if (threadIdx.x >= P || !has) return false;
+    const double dl = delta[i];
 #pragma unroll
-    for (int r = 0; r < 4; r++) F[r] = (r == 3 ? 0.5 * delta : delta) * acc[r];
+    for (int r = 0; r < 4; r++) F[r] = (r == 3 ? 0.5 * dl : dl) * sv[r * P + p];
+    return true;
 }
 
-__global__ void __launch_bounds__(128) k_flux_residual(DevCloud c, const double4_32a *__restrict__ q,
-                                                       const double4_32a *__restrict__ dq, const double4_32a *__restrict__ qm,
-                                                       const double *__restrict__ delta, double4_32a *__restrict__ flux_res,
-                                                       double *__restrict__ ends, long long ns)
+template <int P>
+__global__ void __launch_bounds__(kFluxThreads, 4) k_flux_residual(DevCloud c, const double4_32a *__restrict__ q,
+                                                     const double4_32a *__restrict__ dq, const double4_32a *__restrict__ qm,
+                                                     const double *__restrict__ delta, double4_32a *__restrict__ flux_res,
+                                                     double *__restrict__ ends, long long ns)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
-    const double2 nn = c.nrm[i];
     double F[4];
-    point_flux(c, i, c.flag[i], nn.x, nn.y, delta[i], q, dq, qm, F, ends, ns);
-    flux_res[i] = mk4(F);
+    if (block_flux<P>(c, q, dq, qm, delta, F, ends, ns)) flux_res[blockIdx.x * P + threadIdx.x] = mk4(F);
 }
 
-// state_update_mod.h:92-283 over all points, prim in place, with the
-// residual partial sums of each block.
-template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK) k_state_update(DevCloud c, CaseConst K, double4_32a *__restrict__ prim,
-                                                        const double4_32a *__restrict__ prim_old,
-                                                        const double4_32a *__restrict__ flux_res, int rk,
-                                                        double *__restrict__ psum, double *__restrict__ pmax)
+// Sum and maximum of res_sqr over each 8 consecutive points (lanes of one
+// aligned group of 8, all of them calling), the partials the residual norm is
+// reduced from: the same grouping under every launch shape.
+__device__ __forceinline__ void partial8(double v, int i, int n, double *__restrict__ psum, double *__restrict__ pmax)
 {
-    int i = blockIdx.x * BLOCK + threadIdx.x;
+    const unsigned mask = 0xffu << (threadIdx.x & 24u);
+    double m = v;
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+        v += __shfl_down_sync(mask, v, o, 8);
+        const double t = __shfl_down_sync(mask, m, o, 8);
+        m = t > m ? t : m;
+    }
+    if ((i & 7) == 0 && i < n) {
+        psum[i >> 3] = v;
+        pmax[i >> 3] = m;
+    }
+}
+
+// state_update_mod.h:92-283 over all points, with the residual's partial sums
+// (prim_next may be prim).
+__global__ void __launch_bounds__(128) k_state_update(DevCloud c, CaseConst K, const double4_32a *prim,
+                                                      const double4_32a *__restrict__ prim_old,
+                                                      const double4_32a *__restrict__ flux_res,
+                                                      double4_32a *prim_next, int rk, double *__restrict__ psum,
+                                                      double *__restrict__ pmax)
+{
+    const int i = blockIdx.x * 128 + threadIdx.x;
     double r2 = 0.0;
     if (i < c.n) {
-        const int f = c.flag[i];
         const double2 nn = c.nrm[i];
         double P[4], F[4];
         ld4(prim[i], P);
         ld4(flux_res[i], F);
-        r2 = stage_update(K, f, nn.x, nn.y, P, prim_old + i, F, rk);
-        prim[i] = mk4(P);
+        r2 = fast64::stage(K, c.flag[i], nn.x, nn.y, P, prim_old + i, F, rk);
+        prim_next[i] = mk4(P);
     }
-    block_sum_max<BLOCK>(r2, r2, psum + blockIdx.x, pmax + blockIdx.x);
+    partial8(r2, i, c.n, psum, pmax);
 }
 
-// Fused stage: flux residual + SSPRK update of point i, then q and (after the
-// last stage) the wave speed of the new state for the next stage's kernels.
-// Bound by the FP64 pipe, about 240 FP64 instructions per edge and 130 per
-// point.  Measured on 204,800 points (2.05 M edges, inner 3): 2908 us per
-// launch with CUDA's exp / erf / rsqrt, all four half-range fluxes at every
-// edge and 32 directional sums (about 630 per edge), 1066 us in this form.
-template <int BLOCK>
-__global__ void __launch_bounds__(BLOCK) k_flux_update(DevCloud c, CaseConst K, const double4_32a *__restrict__ q,
-                                                       const double4_32a *__restrict__ dq,
-                                                       const double4_32a *__restrict__ qm,
-                                                       const double *__restrict__ delta,
-                                                       const double4_32a *__restrict__ prim,
-                                                       const double4_32a *__restrict__ prim_old,
-                                                       double4_32a *__restrict__ prim_next, double4_32a *__restrict__ q_next,
-                                                       double *__restrict__ cs_next, int rk,
-                                                       double *__restrict__ psum, double *__restrict__ pmax)
+// Fused stage: flux residual + SSPRK update of the block's points, then q and
+// (after the last stage) the wave speed of the new state for the next stage's
+// kernels.  Bound by the FP64 pipe, about 240 FP64 instructions per edge and
+// 110 per point.  Measured on 204,800 points (2.05 M edges, inner 3): 2908 us
+// per launch with CUDA's exp / erf / rsqrt, all four half-range fluxes at every
+// edge and 32 directional sums (about 630 per edge), 1066 us in this form with
+// a thread per point, 951 us with the edges spread (flux_shape).  Four blocks
+// of 128 registers a thread per SM: 5% over three blocks at 146.
+template <int P>
+__global__ void __launch_bounds__(kFluxThreads, 4) k_flux_update(DevCloud c, CaseConst K, const double4_32a *__restrict__ q,
+                                                   const double4_32a *__restrict__ dq,
+                                                   const double4_32a *__restrict__ qm,
+                                                   const double *__restrict__ delta,
+                                                   const double4_32a *__restrict__ prim,
+                                                   const double4_32a *__restrict__ prim_old,
+                                                   double4_32a *__restrict__ prim_next, double4_32a *__restrict__ q_next,
+                                                   double *__restrict__ cs_next, int rk,
+                                                   double *__restrict__ psum, double *__restrict__ pmax)
 {
-    int i = blockIdx.x * BLOCK + threadIdx.x;
-    double r2 = 0.0;
-    if (i < c.n) {
-        const int f = c.flag[i];
+    double F[4], r2 = 0.0;
+    const int i = blockIdx.x * P + threadIdx.x;
+    if (block_flux<P>(c, q, dq, qm, delta, F, nullptr, 0)) {
         const double2 nn = c.nrm[i];
-        double F[4], P[4], Q[4];
-        point_flux(c, i, f, nn.x, nn.y, delta[i], q, dq, qm, F);
-        ld4(prim[i], P);
-        r2 = stage_update(K, f, nn.x, nn.y, P, prim_old + i, F, rk);
-        prim_next[i] = mk4(P);
-        prim_to_q(P[0], P[1], P[2], P[3], Q);
+        double S[4], Q[4];
+        ld4(prim[i], S);
+        r2 = fast64::stage(K, c.flag[i], nn.x, nn.y, S, prim_old + i, F, rk);
+        prim_next[i] = mk4(S);
+        fast64::q_of(S, Q);
         q_next[i] = mk4(Q);
-        if (cs_next) cs_next[i] = wave_speed(P);
+        if (cs_next) cs_next[i] = fast64::wave_speed(S);
     }
-    if (psum) block_sum_max<BLOCK>(r2, r2, psum + blockIdx.x, pmax + blockIdx.x);
+    if (psum && threadIdx.x < P) partial8(r2, i, c.n, psum, pmax);
 }
 
 // fpi_solver_mod.h:138-147: res_new = sqrt(sum)/n, residue against res_old
@@ -647,6 +672,26 @@ __global__ void __launch_bounds__(256) k_stagnation(int n, const double4_32a *__
 
 // ------------------------------------------------------------- launchers
 
+// Points per block (of 128 threads) of the flux kernels by the number of
+// points; the result is the same under each.  The kernels are bound by the FP64
+// pipe, so what counts is that all SMs have work and end together: with one
+// thread walking a point's edges, a small cloud keeps few SMs busy for the 10
+// to 20 edges of its longest lists; with fewer points per block the last edges
+// and the update leave lanes idle, which costs where every SM is full anyway.
+// Measured per launch (us, inner 0):
+//   points                       960  9,600  30,720  51,200  102,400  204,800
+//   a thread per point           228    217     281     329      649     1061
+//   8 per block, 128 threads      34     81     210     331      645     1260
+//   16                            45     86     182     277      524     1012
+//   32                            68     90     209     281      507      951
+template <typename F> void flux_shape(int n, F &&launch)
+{
+    using std::integral_constant;
+    if (n <= 12288) launch(integral_constant<int, 8>{});
+    else if (n <= 65536) launch(integral_constant<int, 16>{});
+    else launch(integral_constant<int, 32>{});
+}
+
 #define QLSKUM_LAUNCHED(L) \
     do { if ((L).launches) ++*(L).launches; } while (0)
 
@@ -690,15 +735,19 @@ void func_delta(const Launch &L, const DevCloud &c, const double4_32a *prim, dou
 void flux_residual(const Launch &L, const DevCloud &c, const double4_32a *q, const double4_32a *dq, const double4_32a *qm,
                    const double *delta, double4_32a *flux_res, double *ends, long long ns)
 {
-    k_flux_residual<<<grid_for(c.n, 128), 128, 0, L.stream>>>(c, q, dq, qm, delta, flux_res, ends, ns);
+    flux_shape(c.n, [&](auto p) {
+        constexpr int P = decltype(p)::value;
+        k_flux_residual<P><<<grid_for(c.n, P), kFluxThreads, 0, L.stream>>>(c, q, dq, qm, delta, flux_res, ends, ns);
+    });
     QLSKUM_LAUNCHED(L);
 }
 
-void state_update(const Launch &L, const DevCloud &c, const CaseConst &k, double4_32a *prim, const double4_32a *prim_old,
-                  const double4_32a *flux_res, int rk, const Reduce &R)
+void state_update(const Launch &L, const DevCloud &c, const CaseConst &k, const double4_32a *prim,
+                  const double4_32a *prim_old, const double4_32a *flux_res, double4_32a *prim_next, int rk,
+                  const Reduce &R)
 {
-    k_state_update<128><<<grid_for(c.n, 128), 128, 0, L.stream>>>(c, k, prim, prim_old, flux_res, rk,
-                                                                   R.partial_sum, R.partial_max);
+    k_state_update<<<grid_for(c.n, 128), 128, 0, L.stream>>>(c, k, prim, prim_old, flux_res, prim_next, rk,
+                                                             R.partial_sum, R.partial_max);
     QLSKUM_LAUNCHED(L);
 }
 
@@ -706,9 +755,12 @@ void flux_update(const Launch &L, const DevCloud &c, const CaseConst &k, const d
                  const double4_32a *qm, const double *delta, const double4_32a *prim, const double4_32a *prim_old,
                  double4_32a *prim_next, double4_32a *q_next, double *cspeed_next, int rk, const Reduce &R)
 {
-    k_flux_update<128><<<grid_for(c.n, 128), 128, 0, L.stream>>>(c, k, q, dq, qm, delta, prim, prim_old, prim_next,
-                                                                  q_next, cspeed_next, rk, R.partial_sum,
-                                                                  R.partial_max);
+    flux_shape(c.n, [&](auto p) {
+        constexpr int P = decltype(p)::value;
+        k_flux_update<P><<<grid_for(c.n, P), kFluxThreads, 0, L.stream>>>(c, k, q, dq, qm, delta, prim, prim_old,
+                                                                          prim_next, q_next, cspeed_next, rk,
+                                                                          R.partial_sum, R.partial_max);
+    });
     QLSKUM_LAUNCHED(L);
 }
 

@@ -583,7 +583,7 @@ void enqueue_iteration(qlskum_handle *h, int o, int it_arg)
     }
     Reduce R = h->R;
     R.blocks = h->prm.precision == QLSKUM_MIXED ? mixed::flux_grid_blocks(h->flux_variant, h->n)
-                                                 : (h->n + 127) / 128;
+                                                 : fp64::partials(h->n);
     timed(h, QLSKUM_KERNEL_REDUCE, [&] { fp64::reduce_residual(L, R, h->n, it_arg); });
 }
 
@@ -1005,8 +1005,7 @@ qlskum_status qlskum_create(const qlskum_cloud *c, const qlskum_params *p, qlsku
         h->s32.delta = A.alloc<float>(h->np);
         h->s32.cspeed = A.alloc<float>(h->np);
     }
-    h->R.blocks = (n + 127) / 128;
-    h->R.max_blocks = (n + 31) / 32;  // one partial per block of the smallest launch shape (32 threads)
+    h->R.blocks = h->R.max_blocks = fp64::partials(n);  // (the mixed form has one per block of at least 32 points)
     h->R.partial_sum = A.alloc<double>(h->R.max_blocks);
     h->R.partial_max = A.alloc<double>(h->R.max_blocks);
     h->R.res_old = A.alloc<double>(1);
@@ -1134,7 +1133,8 @@ qlskum_status qlskum_state_update(qlskum_handle *h, int rk)
 {
     NEED(h);
     if (rk < 1 || rk > 4) return fail(h, QLSKUM_ERR_INVALID, fmt("rk=%d not in 1..4", rk));
-    fp64::state_update(h->L, h->dc, h->K, h->s64.prim[h->pcur], h->s64.prim[h->pold], h->s64.flux_res, rk, h->R);
+    fp64::state_update(h->L, h->dc, h->K, h->s64.prim[h->pcur], h->s64.prim[h->pold], h->s64.flux_res,
+                       h->s64.prim[h->pcur], rk, h->R);
     h->derived_valid = false;
     return check_launch(h, "state_update");
 }
@@ -2204,7 +2204,7 @@ void part_reduce_layout(qlskum_partition *P)
     int off = 0;
     for (PartDev *d : P->parts) {
         d->red_off = off;
-        d->red_blocks = mx ? mixed::flux_grid_blocks(P->flux_variant, d->G.n) : (d->G.n + 127) / 128;
+        d->red_blocks = mx ? mixed::flux_grid_blocks(P->flux_variant, d->G.n) : fp64::partials(d->G.n);
         off += d->red_blocks;
     }
     P->R.blocks = off;
@@ -2525,7 +2525,7 @@ qlskum_status qlskum_partition_create(const qlskum_cloud *c, const qlskum_params
             if (peer[q][o] && o != q) P->parts[q]->peers.push_back(o);
     // the shared residual arrays: a partial per 32 points of each partition is enough for any launch shape
     int maxp = 0;
-    for (PartDev *d : P->parts) maxp += (d->G.n + 31) / 32;
+    for (PartDev *d : P->parts) maxp += fp64::partials(d->G.n);
     P->R.max_blocks = maxp;
     P->R.partial_sum = P->A.alloc<double>(maxp);
     P->R.partial_max = P->A.alloc<double>(maxp);
@@ -3278,12 +3278,11 @@ void adj_iteration_forward64(qlskum_handle *h, Set64 &st, int it_rec = 0)
     fp64::func_delta(h->L, h->dc, st.P[0], st.delta, h->K.cfl);
     for (int s = 0; s < 4; s++) {
         adj_stage_forward(h, st, s);
-        fp64::copy_prim(h->L, h->n, st.P[s], st.P[s + 1]);
-        fp64::state_update(h->L, h->dc, h->K, st.P[s + 1], st.P[0], st.flux[s], s + 1, h->R);
+        fp64::state_update(h->L, h->dc, h->K, st.P[s], st.P[0], st.flux[s], st.P[s + 1], s + 1, h->R);
     }
     if (it_rec > 0) {
         Reduce R = h->R;
-        R.blocks = (h->n + 127) / 128;
+        R.blocks = fp64::partials(h->n);
         fp64::reduce_residual(h->L, R, h->n, it_rec);
     }
 }

@@ -23,6 +23,7 @@
 namespace qlskum {
 
 enum : int { kWall = 0, kInterior = 1, kOuter = 2 };
+constexpr int kMaxNbhs = 20;                   // QLSKUM_MAX_NBHS
 constexpr int kGaussTab = 6145, kExpTab = 512;
 enum : unsigned { kXpos = 1u, kXneg = 2u, kYpos = 4u, kYneg = 8u };
 
@@ -160,7 +161,7 @@ struct Reduce {
     int *status = nullptr;                   // [1] 0 ok, 1 non-finite residual
     int capacity = 0;
     int blocks = 0;                          // partials written by the last stage kernel
-    int max_blocks = 0;                      // partials allocated (n / 32 rounded up)
+    int max_blocks = 0;                      // partials allocated
     // res_old latches at iterations 1 and 2 unless the run continues from a
     // restart file, which carries its own (fpi_solver_mod.h:139)
     int latch = 1;
@@ -276,6 +277,8 @@ void delta(const Launch &L, const DevCloud &c, const double4_32a *P, const float
 
 // ---------------------------------------------------------- FP64 kernels (qlskum_fp64.cu)
 namespace fp64 {
+// residual partials of one launch over n points (one per 8 points)
+inline int partials(int n) { return (n + 7) / 8; }
 // the folded flux weights DevCloud::e_w64 from the cloud's moments and rotated edge vectors
 void fold_weights(const Launch &L, const DevCloud &c, double2 *e_w64);
 void q_variables(const Launch &L, const DevCloud &c, const double4_32a *prim, double4_32a *q);
@@ -289,8 +292,10 @@ void func_delta(const Launch &L, const DevCloud &c, const double4_32a *prim, dou
 // erf(S2), as 12 planes of ns doubles (read back by the flux reverse).
 void flux_residual(const Launch &L, const DevCloud &c, const double4_32a *q, const double4_32a *dq, const double4_32a *qm,
                    const double *delta, double4_32a *flux_res, double *ends = nullptr, long long ns = 0);
-void state_update(const Launch &L, const DevCloud &c, const CaseConst &k, double4_32a *prim, const double4_32a *prim_old,
-                  const double4_32a *flux_res, int rk, const Reduce &R);
+// one SSPRK stage of every point (prim_next may be prim)
+void state_update(const Launch &L, const DevCloud &c, const CaseConst &k, const double4_32a *prim,
+                  const double4_32a *prim_old, const double4_32a *flux_res, double4_32a *prim_next, int rk,
+                  const Reduce &R);
 void flux_update(const Launch &L, const DevCloud &c, const CaseConst &k, const double4_32a *q, const double4_32a *dq,
                  const double4_32a *qm, const double *delta, const double4_32a *prim, const double4_32a *prim_old,
                  double4_32a *prim_next, double4_32a *q_next, double *cspeed_next, int rk, const Reduce &R);

@@ -88,3 +88,45 @@ def test_nonfinite_state_is_reported():
     s.set_prim(disturbed(c, 0.63))
     s.q_lskum(1)
     assert np.isfinite(s.prim).all()
+
+
+# the flux kernels' three launch shapes, each with a remainder
+@pytest.mark.parametrize("wall, layers", [(49, 21), (113, 111), (257, 259)])
+def test_flux_launch_shapes(wall, layers):
+    """Fused and module path agree bit for bit, and both with the oracle."""
+    import qlskum
+    from qlskum import cloudgen
+    c = cloudgen.make_cloud(n_wall=wall, n_layers=layers, first_spacing=5e-3, radius=5.0 if wall < 50 else 20.0, seed=4)
+    kw = dict(mach=0.63, aoa=2.0, cfl=0.2, vl_const=50.0, inner_iterations=1)
+    P = disturbed(c, 0.63)
+    o = qlskum_oracle.Oracle(c, threads=16, **kw)
+    o.set_prim(P)
+    s = qlskum.Solver(c, **kw)
+    stage(s, P, 1)
+    flux = s.field(qlskum.FIELD_FLUX_RES)
+    s.snapshot_prim_old()
+    for rk in (1, 2, 3, 4):
+        if rk > 1:
+            s.eval_q_variables()
+            s.eval_q_derivatives()
+            s.eval_q_inner_loop()
+            s.eval_update_innerloop()
+            s.cal_flux_residual()
+        s.state_update(rk)
+    f = qlskum.Solver(c, **kw)
+    f.set_prim(P)
+    f.q_lskum(1)
+    assert np.array_equal(f.prim, s.prim)
+    o.func_delta()
+    o.eval_q_variables()
+    o.eval_q_derivatives()
+    o.eval_q_inner_loop()
+    o.eval_update_innerloop()
+    o.cal_flux_residual()
+    assert (np.abs(flux - o.flux_res).max(0) <= flux_bound(c, P, o.delta)).all()
+    o.set_prim(P)
+    res, _, top = o.fpi_solver()
+    h = f.residual_history()[-1]
+    assert np.allclose([h[0], h[2]], [res, top], rtol=1e-10, atol=0)
+    # four stages, each within the bound of its flux residual
+    assert (np.abs(f.prim - o.prim).max(0) <= 4 * flux_bound(c, P, o.delta) + 8 * EPS * np.abs(P).max(0)).all()
