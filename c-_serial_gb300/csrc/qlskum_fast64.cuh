@@ -300,7 +300,7 @@ __device__ __forceinline__ double stage(const CaseConst &K, int f, double nx, do
     if (f == kWall) U[2] = 0.0;
     const double m1 = fma(U[1], ny, __dmul_rn(U[2], nx)), m2 = fma(U[2], ny, -__dmul_rn(U[1], nx));
     const double d = U[0] - rho;
-    const double inv = rcp64(U[0]);
+    const double inv = __drcp_rn(U[0]);
     P[0] = U[0];
     P[1] = m1 * inv;
     P[2] = m2 * inv;

@@ -23,7 +23,7 @@
 namespace qlskum {
 namespace fp64 {
 
-static inline int grid_for(int n, int block) { return (n + block - 1) / block; }
+static inline int grid_for(long long n, int block) { return (int)((n + block - 1) / block); }
 
 // ----------------------------------------------------------------- q, c
 
@@ -53,94 +53,114 @@ __global__ void k_derived(int n, const double4_32a *__restrict__ prim, double4_3
 
 // ----------------------------------------------------------- gradients
 
-// q_variables_mod.h:36-118 (+ state_update_mod.h:448-496 when delta != null):
-// qm = neighbour max/min, dq = least-squares gradient with the precomputed
-// moments {sxx, syy, sxy, 1/det}.
-__global__ void k_q_derivatives(DevCloud c, const double4_32a *__restrict__ q, double4_32a *__restrict__ dq,
-                                double4_32a *__restrict__ qm, const double *__restrict__ cs, double *__restrict__ delta,
-                                double cfl)
+// The gradient and inner-step kernels take four lanes per point, one per
+// component: a lane walks all edges in the reference's neighbour order, the
+// four lanes gather the 32 bytes of a neighbour's q (or of each half of its
+// gradient) in one sector, and a small cloud fills four times the warps.
+
+// Doubles in the order of signed integers (for max / min off the FP64 pipe);
+// its own inverse.
+__device__ __forceinline__ long long order_key(long long b) { return b ^ ((b >> 63) & 0x7fffffffffffffffLL); }
+
+// dist / speed * cfl of one edge (state_update_mod.h:483-488)
+__device__ __forceinline__ double edge_dt(double dist, double speed, double cfl)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
-    double qi[4], qmax[4], qmin[4], sdx[4] = {0, 0, 0, 0}, sdy[4] = {0, 0, 0, 0};
-    ld4(q[i], qi);
-#pragma unroll
-    for (int r = 0; r < 4; r++) { qmax[r] = qi[r]; qmin[r] = qi[r]; }
-    double min_delt = 1.0;
-    const int nb = c.nbhs[i];
-    const long long base = c.slice_base[i >> 5] + (i & 31);
-    for (int j = 0; j < nb; j++) {
-        const long long e = base + 32LL * j;
-        const int k = c.e_nbr[e];
-        const double4_32a g = c.e_geo[e];
-        double qk[4];
-        ld4(q[k], qk);
-#pragma unroll
-        for (int r = 0; r < 4; r++) {
-            if (qk[r] > qmax[r]) qmax[r] = qk[r];
-            if (qk[r] < qmin[r]) qmin[r] = qk[r];
-            sdx[r] = sdx[r] + g.z * (qk[r] - qi[r]);
-            sdy[r] = sdy[r] + g.w * (qk[r] - qi[r]);
-        }
-        if (delta) {
-            double delta_t = c.e_dist[e] / cs[k];
-            delta_t = cfl * delta_t;
-            if (min_delt > delta_t) min_delt = delta_t;
-        }
-    }
-    const double4_32a m = c.ggeo[i];  // sxx, syy, sxy, 1/det
-    double dx[4], dy[4];
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-        dx[r] = (sdx[r] * m.y - sdy[r] * m.z) * m.w;
-        dy[r] = (sdy[r] * m.x - sdx[r] * m.z) * m.w;
-    }
-    dq[2 * i] = mk4(dx);
-    dq[2 * i + 1] = mk4(dy);
-    qm[2 * i] = mk4(qmax);
-    qm[2 * i + 1] = mk4(qmin);
-    if (delta) delta[i] = min_delt;
+    return cfl * fast64::ratio64(dist, speed);
 }
 
-// q_variables_mod.h:120-213: defect-corrected gradient from q shifted half an
-// edge on both ends; writes to dq_out (ping-pong replaces the copy-back of
-// eval_update_innerloop).
-__global__ void k_q_inner(DevCloud c, const double4_32a *__restrict__ q, const double4_32a *__restrict__ dq_in,
-                          double4_32a *__restrict__ dq_out)
+// q_variables_mod.h:36-118 (+ state_update_mod.h:448-496 when delta != null):
+// qm = neighbour max/min, dq = the least-squares gradient through its folded
+// per-edge weights.  960 / 204,800 points: 29 / 113 us per launch with one
+// thread per point, the moments' solve per point and comparisons on the FP64
+// pipe, 12 / 62 us in this form.
+template <bool DT>
+__global__ void k_q_derivatives(DevCloud c, const double *__restrict__ q, double *__restrict__ dq,
+                                double *__restrict__ qm, const double *__restrict__ cs, double *__restrict__ delta,
+                                double cfl)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = t >> 2, r = t & 3;
     if (i >= c.n) return;
-    double qi[4], dxi[4], dyi[4], sdx[4] = {0, 0, 0, 0}, sdy[4] = {0, 0, 0, 0};
-    ld4(q[i], qi);
-    ld4(dq_in[2 * i], dxi);
-    ld4(dq_in[2 * i + 1], dyi);
+    const double qi = q[4 * (size_t)i + r];
+    long long kmax = order_key(__double_as_longlong(qi)), kmin = kmax;
+    double dx = 0.0, dy = 0.0;
     const int nb = c.nbhs[i];
     const long long base = c.slice_base[i >> 5] + (i & 31);
+#pragma unroll 2
     for (int j = 0; j < nb; j++) {
         const long long e = base + 32LL * j;
-        const int k = c.e_nbr[e];
-        const double4_32a g = c.e_geo[e];
-        double qk[4], dxk[4], dyk[4];
-        ld4(q[k], qk);
-        ld4(dq_in[2 * k], dxk);
-        ld4(dq_in[2 * k + 1], dyk);
+        const double2 gw = c.e_gw64[e];
+        const double qk = q[4 * (size_t)c.e_nbr[e] + r];
+        const long long key = order_key(__double_as_longlong(qk));
+        kmax = key > kmax ? key : kmax;
+        kmin = key < kmin ? key : kmin;
+        const double d = qk - qi;
+        dx = fma(gw.x, d, dx);
+        dy = fma(gw.y, d, dy);
+    }
+    const size_t o = 8 * (size_t)i + r;
+    dq[o] = dx;
+    dq[o + 4] = dy;
+    qm[o] = __longlong_as_double(order_key(kmax));
+    qm[o + 4] = __longlong_as_double(order_key(kmin));
+    if (DT) {
+        double m = 1.0;
+        for (int j = r; j < nb; j += 4) {
+            const long long e = base + 32LL * j;
+            const double dt = edge_dt(c.e_dist[e], cs[c.e_nbr[e]], cfl);
+            if (m > dt) m = dt;
+        }
+        const unsigned mask = 0xfu << (threadIdx.x & 28u);
 #pragma unroll
-        for (int r = 0; r < 4; r++) {
-            double temp1 = qi[r] - 0.5 * (g.x * dxi[r] + g.y * dyi[r]);
-            double temp2 = qk[r] - 0.5 * (g.x * dxk[r] + g.y * dyk[r]);
-            sdx[r] = sdx[r] + (g.z * (temp2 - temp1));
-            sdy[r] = sdy[r] + (g.w * (temp2 - temp1));
+        for (int s = 1; s < 4; s <<= 1) {
+            const double x = __shfl_xor_sync(mask, m, s);
+            if (m > x) m = x;
+        }
+        if (r == 0) delta[i] = m;
+    }
+}
+
+// q_variables_mod.h:120-213: the reference's sums over w d (t_k - t_i),
+// t = q - d.dq / 2, by linearity: the solve of the sum over w d (q_k - q_i) is
+// the first-order gradient dq0, the solve of the sum over w d (d.dq_i) is dq_i,
+// so dq_out = dq0 + (dq_i - sum_e g_e (d_e.dq_k)) / 2 with the folded weights
+// g_e: one gather and 4 FP64 instructions per edge and component instead of
+// two and 9.  FIRST: dq0 is not at hand (a call of the inner step alone) and
+// is formed here, with k_q_derivatives' sum.  204,800 points: 167 us per
+// launch before, 73 us now.
+template <bool FIRST>
+__global__ void k_q_inner(DevCloud c, const double *__restrict__ q, const double *__restrict__ dq0,
+                          const double *__restrict__ dq_in, double *__restrict__ dq_out)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = t >> 2, r = t & 3;
+    if (i >= c.n) return;
+    double ax = 0.0, ay = 0.0, d0x = 0.0, d0y = 0.0;
+    const double qi = FIRST ? q[4 * (size_t)i + r] : 0.0;
+    const int nb = c.nbhs[i];
+    const long long base = c.slice_base[i >> 5] + (i & 31);
+#pragma unroll 2
+    for (int j = 0; j < nb; j++) {
+        const long long e = base + 32LL * j;
+        const double2 gw = c.e_gw64[e];
+        const double2 d = *reinterpret_cast<const double2 *>(c.e_geo + e);  // delx, dely
+        const size_t k = (size_t)c.e_nbr[e];
+        const double u = fma(d.x, dq_in[8 * k + r], __dmul_rn(d.y, dq_in[8 * k + 4 + r]));
+        ax = fma(gw.x, u, ax);
+        ay = fma(gw.y, u, ay);
+        if (FIRST) {
+            const double dk = q[4 * k + r] - qi;
+            d0x = fma(gw.x, dk, d0x);
+            d0y = fma(gw.y, dk, d0y);
         }
     }
-    const double4_32a m = c.ggeo[i];
-    double dx[4], dy[4];
-#pragma unroll
-    for (int r = 0; r < 4; r++) {
-        dx[r] = m.w * (sdx[r] * m.y - sdy[r] * m.z);
-        dy[r] = m.w * (sdy[r] * m.x - sdx[r] * m.z);
+    const size_t o = 8 * (size_t)i + r;
+    if (!FIRST) {
+        d0x = dq0[o];
+        d0y = dq0[o + 4];
     }
-    dq_out[2 * i] = mk4(dx);
-    dq_out[2 * i + 1] = mk4(dy);
+    dq_out[o] = fma(0.5, dq_in[o] - ax, d0x);
+    dq_out[o + 4] = fma(0.5, dq_in[o + 4] - ay, d0y);
 }
 
 // state_update_mod.h:448-496, wave speed evaluated per edge as the reference does.
@@ -155,8 +175,7 @@ __global__ void k_func_delta(DevCloud c, const double4_32a *__restrict__ prim, d
         const long long e = base + 32LL * j;
         double P[4];
         ld4(prim[c.e_nbr[e]], P);
-        double delta_t = c.e_dist[e] / fast64::wave_speed(P);
-        delta_t = cfl * delta_t;
+        const double delta_t = edge_dt(c.e_dist[e], fast64::wave_speed(P), cfl);
         if (min_delt > delta_t) min_delt = delta_t;
     }
     delta[i] = min_delt;
@@ -186,20 +205,24 @@ __device__ __forceinline__ double flux_weight(const DevCloud &c, int i, int f, i
     return f == kWall ? 2.0 * w : w;
 }
 
-// Per edge {weight of its x half-range (xpos if it lies there, else xneg),
-// weight of its y half-range (ypos, else yneg)}, once per cloud.
-__global__ void k_fold_weights(DevCloud c, double2 *__restrict__ e_w64)
+// Once per cloud: per edge {weight of its x half-range (xpos if it lies there,
+// else xneg), weight of its y half-range (ypos, else yneg)}, and the gradient's
+// 2x2 solve (q_variables_mod.h:112-116) times the edge's weights.
+__global__ void k_fold_weights(DevCloud c, double2 *__restrict__ e_w64, double2 *__restrict__ e_gw64)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.n) return;
     const int f = c.flag[i];
+    const double4_32a m = c.ggeo[i];  // sxx, syy, sxy, 1/det
     const long long base = c.slice_base[i >> 5] + (i & 31);
     for (int j = 0; j < c.nbhs[i]; j++) {
         const long long e = base + 32LL * j;
         const unsigned dir = c.e_dir[e];
         const double2 sn = c.e_sn[e];
+        const double4_32a g = c.e_geo[e];
         e_w64[e] = make_double2(flux_weight(c, i, f, (dir & kXpos) ? 0 : 1, sn),
                                 flux_weight(c, i, f, (dir & kYpos) ? 2 : 3, sn));
+        e_gw64[e] = make_double2(m.w * diff_of_products(m.y, g.z, m.z, g.w), m.w * diff_of_products(m.x, g.w, m.z, g.z));
     }
 }
 
@@ -695,9 +718,9 @@ template <typename F> void flux_shape(int n, F &&launch)
 #define QLSKUM_LAUNCHED(L) \
     do { if ((L).launches) ++*(L).launches; } while (0)
 
-void fold_weights(const Launch &L, const DevCloud &c, double2 *e_w64)
+void fold_weights(const Launch &L, const DevCloud &c, double2 *e_w64, double2 *e_gw64)
 {
-    k_fold_weights<<<grid_for(c.n, 128), 128, 0, L.stream>>>(c, e_w64);
+    k_fold_weights<<<grid_for(c.n, 128), 128, 0, L.stream>>>(c, e_w64, e_gw64);
     QLSKUM_LAUNCHED(L);
 }
 
@@ -716,13 +739,23 @@ void derived(const Launch &L, const DevCloud &c, const double4_32a *prim, double
 void q_derivatives(const Launch &L, const DevCloud &c, const double4_32a *q, double4_32a *dq, double4_32a *qm,
                    const double *cspeed, double *delta, double cfl)
 {
-    k_q_derivatives<<<grid_for(c.n, L.block), L.block, 0, L.stream>>>(c, q, dq, qm, cspeed, delta, cfl);
+    const double *q1 = reinterpret_cast<const double *>(q);
+    double *dq1 = reinterpret_cast<double *>(dq), *qm1 = reinterpret_cast<double *>(qm);
+    const int g = grid_for(4 * (long long)c.n, L.block);
+    if (delta) k_q_derivatives<true><<<g, L.block, 0, L.stream>>>(c, q1, dq1, qm1, cspeed, delta, cfl);
+    else k_q_derivatives<false><<<g, L.block, 0, L.stream>>>(c, q1, dq1, qm1, nullptr, nullptr, cfl);
     QLSKUM_LAUNCHED(L);
 }
 
-void q_inner(const Launch &L, const DevCloud &c, const double4_32a *q, const double4_32a *dq_in, double4_32a *dq_out)
+void q_inner(const Launch &L, const DevCloud &c, const double4_32a *q, const double4_32a *dq0, const double4_32a *dq_in,
+             double4_32a *dq_out)
 {
-    k_q_inner<<<grid_for(c.n, L.block), L.block, 0, L.stream>>>(c, q, dq_in, dq_out);
+    const double *q1 = reinterpret_cast<const double *>(q), *d0 = reinterpret_cast<const double *>(dq0),
+                 *in = reinterpret_cast<const double *>(dq_in);
+    double *out = reinterpret_cast<double *>(dq_out);
+    const int g = grid_for(4 * (long long)c.n, L.block);
+    if (dq0) k_q_inner<false><<<g, L.block, 0, L.stream>>>(c, nullptr, d0, in, out);
+    else k_q_inner<true><<<g, L.block, 0, L.stream>>>(c, q1, nullptr, in, out);
     QLSKUM_LAUNCHED(L);
 }
 

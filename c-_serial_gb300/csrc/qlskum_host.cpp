@@ -563,9 +563,9 @@ void enqueue_iteration(qlskum_handle *h, int o, int it_arg)
             });
             for (int j = 0; j < ni; j++)
                 timed(h, QLSKUM_KERNEL_INNER,
-                      [&] { mixed::q_inner(L, c, S.dq[0], S.dq[mixed_dq_in(j)], S.dq[mixed_dq_out(j)]); });
+                      [&] { mixed::q_inner(L, c, S.dq[0], S.dq[dq_in_of(j)], S.dq[dq_out_of(j)]); });
             timed(h, QLSKUM_KERNEL_FLUX_UPDATE, [&] {
-                mixed::flux_update(L, c, h->K, S.q[qa], S.dq[mixed_dq_final(ni)], S.qm, S.delta, pin, pold, pout, S.q[qb], cs32,
+                mixed::flux_update(L, c, h->K, S.q[qa], S.dq[dq_final_of(ni)], S.qm, S.delta, pin, pold, pout, S.q[qb], cs32,
                                    rk, Rk, h->flux_variant);
             });
         } else {
@@ -574,10 +574,11 @@ void enqueue_iteration(qlskum_handle *h, int o, int it_arg)
                 fp64::q_derivatives(L, c, S.q[qa], S.dq[0], S.qm, S.cspeed, dl, h->K.cfl);
             });
             for (int j = 0; j < ni; j++)
-                timed(h, QLSKUM_KERNEL_INNER, [&] { fp64::q_inner(L, c, S.q[qa], S.dq[j & 1], S.dq[(j + 1) & 1]); });
+                timed(h, QLSKUM_KERNEL_INNER, 
+                      [&] { fp64::q_inner(L, c, S.q[qa], S.dq[0], S.dq[dq_in_of(j)], S.dq[dq_out_of(j)]); });
             timed(h, QLSKUM_KERNEL_FLUX_UPDATE, [&] {
-                fp64::flux_update(L, c, h->K, S.q[qa], S.dq[ni & 1], S.qm, S.delta, pin, pold, pout, S.q[qb], cs, rk,
-                                  Rk);
+                fp64::flux_update(L, c, h->K, S.q[qa], S.dq[dq_final_of(ni)], S.qm, S.delta, pin, pold, pout, S.q[qb],
+                                  cs, rk, Rk);
             });
         }
     }
@@ -587,11 +588,15 @@ void enqueue_iteration(qlskum_handle *h, int o, int it_arg)
     timed(h, QLSKUM_KERNEL_REDUCE, [&] { fp64::reduce_residual(L, R, h->n, it_arg); });
 }
 
+// The buffer a module-path inner step from dq[d] writes.
+int dq_other(int d) { return d == 1 ? 0 : 1; }
+
 void after_iteration(qlskum_handle *h, int o)
 {
     h->pold = o;
     h->pcur = (o + 2) % 3;
-    h->dcur = h->prm.inner_iterations & 1;
+    if (h->prm.precision != QLSKUM_MIXED) h->dcur = dq_final_of(h->prm.inner_iterations);
+    else h->dcur = h->prm.inner_iterations & 1;
     h->inner_pending = false;
     h->derived_valid = true;
 }
@@ -848,11 +853,12 @@ qlskum_status build_geometry(const qlskum_cloud *c, const qlskum_params *p, int 
     up(d_edist, e_dist); up(d_edir, e_dir); up(d_nrm, nrm); up(d_eps2, eps2); up(d_ggeo, ggeo); up(d_fgeo, fgeo);
     up(d_egeo32, e_geo32); up(d_esn32, e_sn32); up(d_eps32, eps2_32); up(d_edist32, e_dist32); up(d_ew32, e_w32); up(d_ew32b, e_w32b);
     up(d_exy32, e_xy32); up(d_egw32, e_gw32);
-    double2 *d_ew64 = nullptr, *d_gauss = nullptr;
+    double2 *d_ew64 = nullptr, *d_egw64 = nullptr, *d_gauss = nullptr;
     double *d_exp = nullptr;
     if (need_fp64) {
         const FastTables &T = fast_tables();
         d_ew64 = A.alloc<double2>(ne);
+        d_egw64 = A.alloc<double2>(ne);
         d_gauss = A.alloc<double2>(T.gauss.size());
         d_exp = A.alloc<double>(T.exp.size());
         up(d_gauss, T.gauss);
@@ -868,8 +874,9 @@ qlskum_status build_geometry(const qlskum_cloud *c, const qlskum_params *p, int 
     if (need_fp64 && A.err == cudaSuccess) {
         Launch L;
         L.stream = stream;
-        fp64::fold_weights(L, dc, d_ew64);
+        fp64::fold_weights(L, dc, d_ew64, d_egw64);
         dc.e_w64 = d_ew64;
+        dc.e_gw64 = d_egw64;
     }
     dc.max_nb = 0;
     for (int pp = 0; pp < n; pp++) dc.max_nb = std::max(dc.max_nb, c->nbhs[G.iperm[pp]]);
@@ -994,6 +1001,7 @@ qlskum_status qlskum_create(const qlskum_cloud *c, const qlskum_params *p, qlsku
         h->s64.q[b] = A.alloc<double4_32a>(h->np);
         h->s64.dq[b] = A.alloc<double4_32a>((size_t)h->np * 2);
     }
+    if (p->precision != QLSKUM_MIXED) h->s64.dq[2] = A.alloc<double4_32a>((size_t)h->np * 2);
     h->s64.qm = A.alloc<double4_32a>((size_t)h->np * 2);
     h->s64.flux_res = A.alloc<double4_32a>(h->np);
     h->s64.delta = A.alloc<double>(h->np);
@@ -1108,7 +1116,7 @@ qlskum_status qlskum_eval_q_derivatives(qlskum_handle *h)
 qlskum_status qlskum_eval_q_inner_loop(qlskum_handle *h)
 {
     NEED(h);
-    fp64::q_inner(h->L, h->dc, h->s64.q[0], h->s64.dq[h->dcur], h->s64.dq[1 - h->dcur]);
+    fp64::q_inner(h->L, h->dc, h->s64.q[0], nullptr, h->s64.dq[h->dcur], h->s64.dq[dq_other(h->dcur)]);
     h->inner_pending = true;
     return check_launch(h, "eval_q_inner_loop");
 }
@@ -1117,7 +1125,7 @@ qlskum_status qlskum_eval_update_innerloop(qlskum_handle *h)
 {
     NEED(h);
     // the inner loop wrote the other buffer: make it current instead of copying
-    if (h->inner_pending) h->dcur = 1 - h->dcur;
+    if (h->inner_pending) h->dcur = dq_other(h->dcur);
     h->inner_pending = false;
     return QLSKUM_OK;
 }
@@ -1282,7 +1290,7 @@ qlskum_status qlskum_get_field(qlskum_handle *h, int field, double *out)
         break;
     case QLSKUM_FIELD_DQ:
         if (h->prm.precision == QLSKUM_MIXED && h->derived_valid) {
-            src = h->s32.dq[mixed_dq_final(h->prm.inner_iterations)];
+            src = h->s32.dq[dq_final_of(h->prm.inner_iterations)];
             f32 = true;
         }
         else src = h->s64.dq[h->dcur];
@@ -1555,8 +1563,8 @@ void batch_enqueue_iteration(qlskum_batch *b, int o)
         const int qa = (rk - 1) & 1, qb = rk & 1;
         mixed::q_derivatives(b->L, b->sc, b->q[qa], b->dq[0], b->qm, b->cspeed, rk == 1 ? b->delta : nullptr, b->cfl);
         for (int j = 0; j < ni; j++)
-            mixed::q_inner(b->L, b->sc, b->dq[0], b->dq[mixed_dq_in(j)], b->dq[mixed_dq_out(j)]);
-        mixed::flux_update(b->L, b->sc, b->cases[0].K, b->q[qa], b->dq[mixed_dq_final(ni)], b->qm, b->delta,
+            mixed::q_inner(b->L, b->sc, b->dq[0], b->dq[dq_in_of(j)], b->dq[dq_out_of(j)]);
+        mixed::flux_update(b->L, b->sc, b->cases[0].K, b->q[qa], b->dq[dq_final_of(ni)], b->qm, b->delta,
                            b->prim[src[rk - 1]], b->prim[o], b->prim[dst[rk - 1]], b->q[qb],
                            rk == 4 ? b->cspeed : nullptr, rk, rk == 4 ? R : none, b->flux_variant);
     }
@@ -2250,15 +2258,16 @@ void part_iteration(qlskum_partition *P, int o)
         for (int j = 0; j < ni; j++) {
             for (PartDev *d : P->parts) {
                 if (mx)
-                    mixed::q_inner(d->L, d->G.dc, d->s32.dq[0], d->s32.dq[mixed_dq_in(j)],
-                                   d->s32.dq[mixed_dq_out(j)]);
+                    mixed::q_inner(d->L, d->G.dc, d->s32.dq[0], d->s32.dq[dq_in_of(j)],
+                                   d->s32.dq[dq_out_of(j)]);
                 else
-                    fp64::q_inner(d->L, d->G.dc, d->s64.q[qa], d->s64.dq[j & 1], d->s64.dq[(j + 1) & 1]);
+                    fp64::q_inner(d->L, d->G.dc, d->s64.q[qa], d->s64.dq[0], d->s64.dq[dq_in_of(j)],
+                                  d->s64.dq[dq_out_of(j)]);
             }
             if (mx)
-                part_exchange(P, 1, [&](PartDev &d, int) { return FieldRef{d.s32.dq[mixed_dq_out(j)], 32}; });
+                part_exchange(P, 1, [&](PartDev &d, int) { return FieldRef{d.s32.dq[dq_out_of(j)], 32}; });
             else
-                part_exchange(P, 1, [&](PartDev &d, int) { return FieldRef{d.s64.dq[(j + 1) & 1], 64}; });
+                part_exchange(P, 1, [&](PartDev &d, int) { return FieldRef{d.s64.dq[dq_out_of(j)], 64}; });
         }
         for (PartDev *d : P->parts) {
             // only the last stage's residual is reported (fpi_solver_mod.h:138)
@@ -2271,11 +2280,11 @@ void part_iteration(qlskum_partition *P, int o)
             }
             double4_32a *const *prim = d->s64.prim;
             if (mx)
-                mixed::flux_update(d->L, d->G.dc, P->K, d->s32.q[qa], d->s32.dq[mixed_dq_final(ni)], d->s32.qm,
+                mixed::flux_update(d->L, d->G.dc, P->K, d->s32.q[qa], d->s32.dq[dq_final_of(ni)], d->s32.qm,
                                    d->s32.delta, prim[src[rk - 1]], prim[o], prim[dst[rk - 1]], d->s32.q[qb],
                                    rk == 4 ? d->s32.cspeed : nullptr, rk, Rk, P->flux_variant);
             else
-                fp64::flux_update(d->L, d->G.dc, P->K, d->s64.q[qa], d->s64.dq[ni & 1], d->s64.qm, d->s64.delta,
+                fp64::flux_update(d->L, d->G.dc, P->K, d->s64.q[qa], d->s64.dq[dq_final_of(ni)], d->s64.qm, d->s64.delta,
                                   prim[src[rk - 1]], prim[o], prim[dst[rk - 1]], d->s64.q[qb],
                                   rk == 4 ? d->s64.cspeed : nullptr, rk, Rk);
         }
@@ -2456,6 +2465,7 @@ qlskum_status qlskum_partition_create(const qlskum_cloud *c, const qlskum_params
             d->s64.q[b] = A.alloc<double4_32a>(np);
             d->s64.dq[b] = A.alloc<double4_32a>(np * 2);
         }
+        if (!mx) d->s64.dq[2] = A.alloc<double4_32a>(np * 2);
         d->s64.qm = A.alloc<double4_32a>(np * 2);
         d->s64.flux_res = A.alloc<double4_32a>(np);
         d->s64.delta = A.alloc<double>(np);
@@ -3264,7 +3274,8 @@ void adj_stage_forward(qlskum_handle *h, Set64 &st, int s)
     const DevCloud &c = h->dc;
     fp64::q_variables(h->L, c, st.P[s], st.q[s]);
     fp64::q_derivatives(h->L, c, st.q[s], adj_dq(st, ni, s, 0), st.qm[s], nullptr, nullptr, 0.0);
-    for (int j = 1; j <= ni; j++) fp64::q_inner(h->L, c, st.q[s], adj_dq(st, ni, s, j - 1), adj_dq(st, ni, s, j));
+    for (int j = 1; j <= ni; j++) 
+        fp64::q_inner(h->L, c, st.q[s], adj_dq(st, ni, s, 0), adj_dq(st, ni, s, j - 1), adj_dq(st, ni, s, j));
     fp64::flux_residual(h->L, c, st.q[s], adj_dq(st, ni, s, ni), st.qm[s], st.delta, st.flux[s], st.ends[s],
                         (long long)h->adj->ne);
 }

@@ -44,9 +44,10 @@ struct DevCloud {
     const double *eps2 = nullptr;
     const double4_32a *ggeo = nullptr;           // [np]
     const double4_32a *fgeo = nullptr;           // [np][4]
-    // FP64 form: the folded flux weights of e_w32 (below) in FP64, and the
+    // FP64 form: the folded weights of e_w32 and e_gw32 (below) in FP64, and the
     // tables of the fast FP64 functions (qlskum_fast64.cuh)
     const double2 *e_w64 = nullptr;
+    const double2 *e_gw64 = nullptr;
     const double2 *gauss_tab = nullptr;      // [kGaussTab]
     const double *exp_tab = nullptr;         // [kExpTab]
     // mixed-precision copies of the per-edge geometry (FP32)
@@ -125,7 +126,10 @@ struct BatchView {
 struct State64 {
     double4_32a *prim[3] = {nullptr, nullptr, nullptr};
     double4_32a *q[2] = {nullptr, nullptr};
-    double4_32a *dq[2] = {nullptr, nullptr};     // [np][2] each
+    // [np][2] each: in the fused iteration dq[0] the stage's first-order
+    // gradient, dq[1] / dq[2] the inner steps' outputs in turn (dq_in_of /
+    // dq_out_of); the module path's steps swap dq[0] and dq[1] (dq[2]: FP64 handles only)
+    double4_32a *dq[3] = {nullptr, nullptr, nullptr};
     double4_32a *qm = nullptr;                   // [np][2]
     double4_32a *flux_res = nullptr;
     double *delta = nullptr;
@@ -138,18 +142,18 @@ struct State64 {
 struct State32 {
     float4 *q[2] = {nullptr, nullptr};
     // [np][2] each: dq[0] the stage's first-order gradient, dq[1] / dq[2]
-    // the inner steps' outputs in turn (mixed_dq_in / mixed_dq_out)
+    // the inner steps' outputs in turn (dq_in_of / dq_out_of)
     float4 *dq[3] = {nullptr, nullptr, nullptr};
     float4 *qm = nullptr;                    // [np][2]
     float *delta = nullptr;
     float *cspeed = nullptr;
 };
 
-// Buffers of the mixed inner loop: step j (0-based) reads dq[mixed_dq_in(j)]
-// and writes dq[mixed_dq_out(j)]; the flux kernel reads dq[mixed_dq_final(ni)].
-inline int mixed_dq_in(int j) { return j == 0 ? 0 : 1 + ((j - 1) & 1); }
-inline int mixed_dq_out(int j) { return 1 + (j & 1); }
-inline int mixed_dq_final(int ni) { return ni == 0 ? 0 : mixed_dq_out(ni - 1); }
+// Buffers of the inner loop: step j (0-based) reads dq[dq_in_of(j)]
+// and writes dq[dq_out_of(j)]; the flux kernel reads dq[dq_final_of(ni)].
+inline int dq_in_of(int j) { return j == 0 ? 0 : 1 + ((j - 1) & 1); }
+inline int dq_out_of(int j) { return 1 + (j & 1); }
+inline int dq_final_of(int ni) { return ni == 0 ? 0 : dq_out_of(ni - 1); }
 
 // Residual reduction scratch.
 struct Reduce {
@@ -279,13 +283,15 @@ void delta(const Launch &L, const DevCloud &c, const double4_32a *P, const float
 namespace fp64 {
 // residual partials of one launch over n points (one per 8 points)
 inline int partials(int n) { return (n + 7) / 8; }
-// the folded flux weights DevCloud::e_w64 from the cloud's moments and rotated edge vectors
-void fold_weights(const Launch &L, const DevCloud &c, double2 *e_w64);
+// the folded weights DevCloud::e_w64 and e_gw64 from the cloud's moments and rotated edge vectors
+void fold_weights(const Launch &L, const DevCloud &c, double2 *e_w64, double2 *e_gw64);
 void q_variables(const Launch &L, const DevCloud &c, const double4_32a *prim, double4_32a *q);
 void derived(const Launch &L, const DevCloud &c, const double4_32a *prim, double4_32a *q, double *cspeed);
 void q_derivatives(const Launch &L, const DevCloud &c, const double4_32a *q, double4_32a *dq, double4_32a *qm,
                    const double *cspeed, double *delta, double cfl);
-void q_inner(const Launch &L, const DevCloud &c, const double4_32a *q, const double4_32a *dq_in, double4_32a *dq_out);
+// one inner step from dq_in; dq0: the first-order gradient of q (q_derivatives'), or NULL (formed again from q)
+void q_inner(const Launch &L, const DevCloud &c, const double4_32a *q, const double4_32a *dq0, const double4_32a *dq_in,
+             double4_32a *dq_out);
 void func_delta(const Launch &L, const DevCloud &c, const double4_32a *prim, double *delta, double cfl);
 // ends (or NULL): per edge slot of the ns slots, the owner's and the
 // neighbour's end's rho, sqrt(beta), exp(-S1^2), exp(-S2^2), erf(S1),

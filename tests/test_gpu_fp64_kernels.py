@@ -130,3 +130,29 @@ def test_flux_launch_shapes(wall, layers):
     assert np.allclose([h[0], h[2]], [res, top], rtol=1e-10, atol=0)
     # four stages, each within the bound of its flux residual
     assert (np.abs(f.prim - o.prim).max(0) <= 4 * flux_bound(c, P, o.delta) + 8 * EPS * np.abs(P).max(0)).all()
+
+
+# 1008, 1029 and 1071 points: the last warp of the four-lanes-per-point kernels full or partly empty
+@pytest.mark.parametrize("wall", [48, 49, 51])
+@pytest.mark.parametrize("power", [0.0, -2.0])
+def test_inner_step_on_its_own(wall, power):
+    """An inner step whose gradient is not that of the current q, as a caller
+    of the modules may order it.  Bound: the weights sum to at most 2.5 /
+    min_dist; q (8 ulps) and the old gradient times an edge (8 ulps) meet them."""
+    import qlskum
+    from qlskum import cloudgen
+    c = cloudgen.make_cloud(n_wall=wall, n_layers=21, first_spacing=5e-3, radius=5.0, seed=4)
+    kw = dict(mach=0.63, aoa=2.0, cfl=0.2, vl_const=50.0, power=power, inner_iterations=1)
+    s, o = qlskum.Solver(c, **kw), qlskum_oracle.Oracle(c, **kw)
+    for x in (s, o):
+        x.set_prim(disturbed(c, 0.63, 1))
+        x.eval_q_variables()
+        x.eval_q_derivatives()
+        x.set_prim(disturbed(c, 0.63, 2))
+        x.eval_q_variables()
+        x.eval_q_inner_loop()
+        x.eval_update_innerloop()
+    d = s.field(qlskum.FIELD_DQ)
+    md = c.min_dist[:, None, None]
+    reach = 2.5 * 3.0 * np.abs(o.dq).max()  # gradient times an edge of up to 3 min_dist, over min_dist
+    assert (np.abs(d - o.dq) <= EPS * (8 * 2.5 * 2 * np.abs(o.q).max() / md + 8 * reach)).all()
