@@ -15,6 +15,7 @@
 // least-squares moments) for the wall-displacement gradient, which the host
 // finishes (qlskum_host.cpp).
 #include "qlskum_adjoint.cuh"
+#include "qlskum_fast64.cuh"
 #include "qlskum_dev.cuh"
 
 namespace qlskum {
@@ -78,219 +79,355 @@ __global__ void k_update(AdjView a, CaseConst K, const double4_32a *__restrict__
     }
 }
 
-// Reverse of the flux residual of every point: F_i = s delta_i sum_d G_d.
-// Adds the bars of q, dq, qm (own and neighbours'), of delta, and (GEO) of the
-// edge geometry, the normal and the directional moments.
-template <int MODE>
-__global__ void __launch_bounds__(128) k_flux(AdjView a, const double4_32a *__restrict__ q,
-                                               const double4_32a *__restrict__ dq, const double4_32a *__restrict__ qm,
-                                               const double *__restrict__ delta, const double4_32a *__restrict__ flux,
-                                               const double *__restrict__ ends, long long ns, const double4_32a *__restrict__ bF,
-                                               double4_32a *__restrict__ bq, double4_32a *__restrict__ bdq,
-                                               double4_32a *__restrict__ bqm, double *__restrict__ bdelta)
+// ------------------------------------------------------ flux reverse, FP64
+// The reverse of fp64::edge_flux: F = delta sum_e v_e, v_e the folded-weight
+// sum of an edge's half-range flux differences, so the bar of v_e is
+// delta F-bar at every edge and the bar of a flux at the neighbour's end that
+// times the edge's weight, at the owner's end its negative.
+
+// The limiter at one component, kept for its reverse: t = num / den and
+// 1 / den where it is active, else t = 1 and 0.
+struct Limiter {
+    double dn, dp, t, rden;
+};
+
+__device__ __forceinline__ double limited(double q, double dn, double dp, double eps2, Limiter &l)
 {
-    // MODE 0: the state bars at every point; 2: only the geometry bars, at
-    // the points AdjView::geo_list names (the geometry's instantiation needs
-    // far more registers, so it runs on those few points alone)
-    constexpr bool GEO = MODE != 0, STATE = MODE != 2;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (MODE == 2 ? a.n_geo : a.c.n)) return;
-    const int i = MODE == 2 ? a.geo_list[t] : t;
+    l.dn = dn;
+    l.dp = dp;
+    l.t = 1.0;
+    l.rden = 0.0;
+    if (!fast64::within_cut(dn)) {
+        const double base = fma(dp, dp, eps2);
+        const double rd = rcp64(fma(dn, fma(2.0, dn, dp), base));
+        const double t = fma(dn, dp + dp, base) * rd;
+        if ((unsigned long long)__double_as_longlong(t) < 0x3ff0000000000000ULL) {
+            l.t = t;
+            l.rden = rd;
+        }
+    }
+    return fma(l.t, dn, q);
+}
+
+// The bars of q~ -> those of dn and dp (dp's enters q and qmax or qmin).
+// q~ = q + t dn, t = (base + 2 dn dp) / (base + dn dp + 2 dn^2), base = dp^2 + eps2.
+__device__ __forceinline__ void limited_vjp(const Limiter &l, double bt, double &bdn, double &bdp)
+{
+    const double g = l.dn * bt * l.rden;
+    const double dp2 = l.dp + l.dp;
+    bdn = fma(l.t, bt, g * fma(-l.t, fma(4.0, l.dn, l.dp), dp2));
+    bdp = g * fma(-l.t, dp2 + l.dn, fma(2.0, l.dn, dp2));
+}
+
+// Bars of one end's log(rho), u_t, u_n, p / rho, erf(S1), erf(S2) and of the
+// moments B1, B2.
+struct EndBar {
+    double ell, ut, un, p, E1, E2, B1, B2;
+};
+
+// Reverse of fast64::split_pair for the bar b of v.
+__device__ __forceinline__ void split_pair_vjp(const Kin<double> &k, unsigned sx, unsigned sy, double wx, double wy,
+                                               const double b[4], EndBar &o)
+{
+    const double wr = wx * k.rho, yr = wy * k.rho, ws = fast64::flip(wr, sx), ys = fast64::flip(yr, sy);
+    const double al = wr * fma(0.5, fast64::flip(k.E1, sx), 0.5), ga = yr * fma(0.5, fast64::flip(k.E2, sy), 0.5);
+    const double be = fma(ws, k.B1, ys * k.B2);
+    const double v0 = fma(al, k.ut, fma(ga, k.un, be));
+    const double h3 = 0.5 * b[3];
+    // the bar of v0 without and with the 3.5 p / rho v0 of v3
+    const double bs = fma(k.ut, b[1], fma(k.un, b[2], fma(k.usq, h3, b[0])));
+    const double bv = fma(7.0 * k.pbr, h3, bs);
+    const double bbe = fma(-k.pbr, h3, bv);
+    const double bp = fma(al, b[1], fma(ga, b[2], h3 * fma(7.0, v0, -be)));
+    o.p += bp;
+    o.ell += fma(v0, bs, k.pbr * bp);
+    o.ut += fma(v0, fma(k.ut, b[3], b[1]), al * bv);
+    o.un += fma(v0, fma(k.un, b[3], b[2]), ga * bv);
+    o.E1 = fma(0.5 * ws, fma(k.pbr, b[1], bv * k.ut), o.E1);
+    o.E2 = fma(0.5 * ys, fma(k.pbr, b[2], bv * k.un), o.E2);
+    o.B1 = fma(ws, bbe, o.B1);
+    o.B2 = fma(ys, bbe, o.B2);
+}
+
+// Reverse of a boundary end's quadrant flux of weight w.
+__device__ __forceinline__ void quad_x_vjp(const Kin<double> &k, double s1, double s2, double w, const double b[4],
+                                           EndBar &o)
+{
+    KinBar kb;
+    const double bG[4] = {w * b[0], w * b[1], w * b[2], w * b[3]};
+    adj::flux_quad_vjp(k, s1, s2, bG, kb);
+    o.ell = fma(k.rho, kb.rho, o.ell);
+    o.ut += fma(2.0 * k.ut, kb.usq, kb.ut);
+    o.un += fma(2.0 * k.un, kb.usq, kb.un);
+    o.p += kb.pbr;
+    o.E1 += kb.E1;
+    o.E2 += kb.E2;
+    o.B1 += kb.B1;
+    o.B2 += kb.B2;
+}
+
+// One end of an edge: its limited reconstruction and the moments from the
+// forward's kept values.
+struct RevEnd {
+    Limiter l[4];
+    double t[4];        // q~
+    double qs, qn, r, e1, e2;
+    Kin<double> k;
+};
+
+__device__ __forceinline__ void rev_end(int f, double nx, double ny, double hx, double hy, const double q[4],
+                                        const double dx[4], const double dy[4], const double mx[4],
+                                        const double mn[4], double e2, const double *__restrict__ kept, long long ns,
+                                        RevEnd &s)
+{
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        const double dn = fma(hx, dx[c], hy * dy[c]);
+        s.t[c] = limited(q[c], dn, (__double2hiint(dn) >= 0 ? mx[c] : mn[c]) - q[c], e2, s.l[c]);
+    }
+    s.k.rho = kept[0];
+    s.r = kept[ns];
+    s.e1 = kept[2 * ns];
+    s.e2 = kept[3 * ns];
+    s.k.E1 = kept[4 * ns];
+    s.k.E2 = kept[5 * ns];
+    s.qs = s.t[1];
+    s.qn = s.t[2];
+    if (f != kInterior) {
+        s.qs = fma(s.t[1], ny, -(s.t[2] * nx));
+        s.qn = fma(s.t[1], nx, s.t[2] * ny);
+    }
+    s.k.pbr = 2.0 * s.r * s.r;
+    s.k.ut = s.qs * s.k.pbr;
+    s.k.un = s.qn * s.k.pbr;
+    s.k.usq = fma(s.k.ut, s.k.ut, s.k.un * s.k.un);
+    s.k.B1 = s.r * s.e1;
+    s.k.B2 = s.r * s.e2;
+}
+
+// Reverse of fast64::end: the bars of the end's moments -> those of q~ in the
+// point's (t, n) frame: bt[1], bt[2] are the bars of qs, qn.
+//   S = r q, r = b^-1/2, p / rho = 2 / b, u = q p / rho,
+//   log(rho) = q~1 + S1^2 + S2^2 - 2.5 log b, b = -2 q~4, erf' = 2 e, B = r e.
+__device__ __forceinline__ void end_vjp(const RevEnd &s, const EndBar &o, double bt[4])
+{
+    const double S1 = s.r * s.qs, S2 = s.r * s.qn;
+    const double bS1 = 2.0 * fma(s.e1, o.E1, S1 * fma(-s.k.B1, o.B1, o.ell));
+    const double bS2 = 2.0 * fma(s.e2, o.E2, S2 * fma(-s.k.B2, o.B2, o.ell));
+    const double br = fma(s.e1, o.B1, fma(s.e2, o.B2, fma(s.qs, bS1, s.qn * bS2)));
+    const double bp = fma(s.qs, o.ut, fma(s.qn, o.un, o.p));
+    bt[0] = o.ell;
+    bt[1] = fma(s.k.pbr, o.ut, s.r * bS1);
+    bt[2] = fma(s.k.pbr, o.un, s.r * bS2);
+    bt[3] = 0.5 * s.k.pbr * fma(s.r, br, fma(2.0 * s.k.pbr, bp, 5.0 * o.ell));
+}
+
+// The bars of an end's moments for the weights (wx, wy) of the edge, w2x / w2y
+// those of the second half range of an edge on both sides of an axis.
+__device__ __forceinline__ void flux_bars(int f, unsigned dir, const Kin<double> &k, double wx, double wy, double w2x,
+                                          double w2y, const double b[4], EndBar &o)
+{
+    const unsigned neg = 0x80000000u;
+    const unsigned sx = (dir & kXpos) ? 0u : neg, sy = (dir & kYpos) ? 0u : neg;
+    const bool inner = f == kInterior;
+    const double s2 = f == kOuter ? 1.0 : -1.0;
+    o = EndBar{0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    split_pair_vjp(k, sx, sy, inner ? wx : 0.0, wy, b, o);
+    if (!inner) quad_x_vjp(k, sx ? -1.0 : 1.0, s2, wx, b, o);
+    if (w2x != 0.0) {
+        if (inner) split_pair_vjp(k, neg, 0u, w2x, 0.0, b, o);
+        else quad_x_vjp(k, -1.0, s2, w2x, b, o);
+    }
+    if (w2y != 0.0) split_pair_vjp(k, 0u, neg, 0.0, w2y, b, o);
+}
+
+// Reverse of the flux residual.  GEO false: adds the bars of q, dq, qm (own
+// and neighbours') and of delta, at every point.  GEO true: the bars of the
+// edge geometry, the normal and the directional moments, at the points
+// AdjView::geo_list names.  P points per block of kRevThreads threads, a
+// point's edges spread over kRevThreads / P of them as in fp64::block_flux;
+// each thread adds its edges' owner bars to its own slots of shared memory,
+// which the block sums at the end.
+// Bound by the FP64 pipe: about 400 FP64 instructions per edge, 16 FP64
+// reductions to L2.  51,200 points (512,000 edges): 1707 us with one thread
+// per point and all four half ranges at every edge, 448 us in this form; the
+// geometry bars of a 20,480-point cloud (128 wall points) 922 and 37 us.  Four blocks
+// of 128 registers per SM: 3-8% over two at 178.
+constexpr int kRevThreads = 128;
+
+template <int P, bool GEO>
+__global__ void __launch_bounds__(kRevThreads, GEO ? 1 : 4) k_flux(AdjView a, const double4_32a *__restrict__ q,
+                                                      const double4_32a *__restrict__ dq,
+                                                      const double4_32a *__restrict__ qm,
+                                                      const double *__restrict__ delta,
+                                                      const double4_32a *__restrict__ flux,
+                                                      const double *__restrict__ ends, long long ns,
+                                                      const double4_32a *__restrict__ bF, double4_32a *__restrict__ bq,
+                                                      double4_32a *__restrict__ bdq, double4_32a *__restrict__ bqm,
+                                                      double *__restrict__ bdelta)
+{
+    constexpr int T = kRevThreads;
+    // GEO false: bars of q, dq x, dq y, qmax, qmin; true: per half range the
+    // x and y sums of the moments' bars, then the normal's
+    constexpr int NS = GEO ? 10 : 20;
+    __shared__ double sum[NS][T];
     const DevCloud &c = a.c;
-    const int f = c.flag[i];
-    const double2 nn = c.nrm[i];
-    const double nx = nn.x, ny = nn.y;
-    double qi[4], dxi[4], dyi[4], mxi[4], mni[4];
-    ld4(q[i], qi);
-    ld4(dq[2 * i], dxi);
-    ld4(dq[2 * i + 1], dyi);
-    ld4(qm[2 * i], mxi);
-    ld4(qm[2 * i + 1], mni);
-    const double e2i = c.eps2[i];
-    const int nb = c.nbhs[i];
-    const long long base = c.slice_base[i >> 5] + (i & 31);
-    const double scale = (f == kWall) ? 2.0 : 1.0;
-    const bool used[4] = {true, true, f != kWall, f != kOuter};
-    const bool geo = GEO;
-
-    // forward: the directional sums, for the bars of the moments (GEO only;
-    // without them the bar of delta comes from the stage's flux residual,
-    // F = delta * scale * sum_d G_d, so dF/ddelta = F / delta)
-    double sx[4][4], sy[4][4];
-    for (int d = 0; d < 4; d++)
-        for (int r = 0; r < 4; r++) sx[d][r] = sy[d][r] = 0.0;
-    for (int j = 0; geo && j < nb; j++) {
-        const long long e = base + 32LL * j;
-        const int k = c.e_nbr[e];
-        const double4_32a g = c.e_geo[e];
-        const double2 sw = c.e_sn[e];
-        const unsigned dir = c.e_dir[e];
-        double qk[4], dxk[4], dyk[4], mxk[4], mnk[4], kept[12];
-        ld4(q[k], qk);
-        ld4(dq[2 * k], dxk);
-        ld4(dq[2 * k + 1], dyk);
-        ld4(qm[2 * k], mxk);
-        ld4(qm[2 * k + 1], mnk);
-        for (int w = 0; ends && w < 12; w++) kept[w] = ends[w * ns + e];
-        adj::End64 s;
-        adj::end64(nx, ny, g.x, g.y, qi, dxi, dyi, mxi, mni, e2i, s, ends ? kept : nullptr);
-        const Kin<double> ki = s.k;
-        adj::end64(nx, ny, g.x, g.y, qk, dxk, dyk, mxk, mnk, c.eps2[k], s, ends ? kept + 6 : nullptr);
-        const Kin<double> kk = s.k;
-#define QLSKUM_FWD(D)                                                                \
-        if (dir & (1u << D)) {                                                       \
-            double Gi[4], Gk[4];                                                     \
-            dir_flux<double, D>(f, ki, Gi);                                          \
-            dir_flux<double, D>(f, kk, Gk);                                          \
-            for (int r = 0; r < 4; r++) {                                            \
-                sx[D][r] += (Gk[r] - Gi[r]) * sw.x;                                  \
-                sy[D][r] += (Gk[r] - Gi[r]) * sw.y;                                  \
-            }                                                                        \
+    const int p = threadIdx.x % P, at = blockIdx.x * P + p, n = GEO ? a.n_geo : c.n;
+    const bool has = at < n;
+    const int i = !has ? 0 : GEO ? a.geo_list[at] : at;
+#pragma unroll
+    for (int w = 0; w < NS; w++) sum[w][threadIdx.x] = 0.0;
+    if (has) {
+        const int f = c.flag[i];
+        const double2 nn = c.nrm[i];
+        const double nx = nn.x, ny = nn.y, dl = delta[i];
+        const int nb = c.nbhs[i];
+        const long long base = c.slice_base[i >> 5] + (i & 31);
+        double b[4];
+        ld4(bF[i], b);
+        if (!GEO && threadIdx.x < P) {
+            // F = delta * sum, so dF / ddelta = F / delta
+            double F[4];
+            ld4(flux[i], F);
+            bdelta[i] += (b[0] * F[0] + b[1] * F[1] + b[2] * F[2] + b[3] * F[3]) / dl;
         }
-        QLSKUM_FWD(0)
-        QLSKUM_FWD(1)
-        QLSKUM_FWD(2)
-        QLSKUM_FWD(3)
-#undef QLSKUM_FWD
-    }
-    double bFi[4];
-    ld4(bF[i], bFi);
-    const double dl = delta[i];
-    // bars of the directional sums: the solve is linear in them, so the bar
-    // of sum x (y) of half-range d, component r, is bG[r] ax[d] (bG[r] ay[d])
-    // with bG = scale delta F-bar
-    double bG4[4], ax[4], ay[4];
-    for (int r = 0; r < 4; r++) bG4[r] = scale * dl * bFi[r];
-    double bdl = 0.0;
-    for (int d = 0; d < 4; d++) {
-        const double4_32a m = c.fgeo[4 * i + d];
-        ax[d] = ay[d] = 0.0;
-        if (!used[d]) continue;
-        if (d < 2) {
-            ax[d] = m.y * m.w;
-            ay[d] = -m.z * m.w;
-        } else {
-            ax[d] = -m.z * m.w;
-            ay[d] = m.x * m.w;
-        }
-        if (!geo) continue;
-        double bm[4] = {0, 0, 0, 0};
-        for (int r = 0; r < 4; r++) {
-            const double bG = bG4[r];
-            if (d < 2) {
-                const double G = (sx[d][r] * m.y - sy[d][r] * m.z) * m.w;
-                bdl += scale * bFi[r] * G;
-                bm[1] += bG * sx[d][r] * m.w;
-                bm[2] -= bG * sy[d][r] * m.w;
-                bm[3] += bG * (sx[d][r] * m.y - sy[d][r] * m.z);
-            } else {
-                const double G = (sy[d][r] * m.x - sx[d][r] * m.z) * m.w;
-                bdl += scale * bFi[r] * G;
-                bm[0] += bG * sy[d][r] * m.w;
-                bm[2] -= bG * sx[d][r] * m.w;
-                bm[3] += bG * (sy[d][r] * m.x - sx[d][r] * m.z);
+#pragma unroll
+        for (int r = 0; r < 4; r++) b[r] *= dl;
+        for (int j = threadIdx.x / P; j < nb; j += T / P) {
+            const long long e = base + 32LL * j;
+            const double4_32a g = c.e_geo[e];
+            const double hx = -0.5 * g.x, hy = -0.5 * g.y;
+            const double2 w = c.e_w64[e];
+            const unsigned dir = c.e_dir[e];
+            double w2x = 0.0, w2y = 0.0;
+            if ((dir & (kXpos | kXneg)) == (kXpos | kXneg)) w2x = fast64::flux_weight(c, i, f, 1, c.e_sn[e]);
+            if ((dir & (kYpos | kYneg)) == (kYpos | kYneg)) w2y = fast64::flux_weight(c, i, f, 3, c.e_sn[e]);
+            double bdelx = 0.0, bdely = 0.0, bnx = 0.0, bny = 0.0;
+            double dot[4] = {0.0, 0.0, 0.0, 0.0};  // b . (G_k - G_i) per half range
+            // the neighbour's end, then the owner's
+#pragma unroll 1
+            for (int own = 0; own < 2; own++) {
+                const int k = own ? i : c.e_nbr[e];
+                const double sg = own ? -1.0 : 1.0;
+                double qk[4], dx[4], dy[4], mx[4], mn[4], bt[4];
+                ld4(q[k], qk);
+                ld4(dq[2 * k], dx);
+                ld4(dq[2 * k + 1], dy);
+                ld4(qm[2 * k], mx);
+                ld4(qm[2 * k + 1], mn);
+                RevEnd s;
+                EndBar o;
+                rev_end(f, nx, ny, hx, hy, qk, dx, dy, mx, mn, c.eps2[k], ends + (own ? 0 : 6) * ns + e, ns, s);
+                flux_bars(f, dir, s.k, sg * w.x, sg * w.y, sg * w2x, sg * w2y, b, o);
+                end_vjp(s, o, bt);
+                if (GEO) {
+                    bnx += fma(s.t[1], bt[2], -(s.t[2] * bt[1]));
+                    bny += fma(s.t[1], bt[1], s.t[2] * bt[2]);
+                    double G[4];
+#define QLSKUM_DOT(D)                                                                           \
+                    if (dir & (1u << D)) {                                                      \
+                        dir_flux<double, D>(f, s.k, G);                                         \
+                        dot[D] += sg * (b[0] * G[0] + b[1] * G[1] + b[2] * G[2] + b[3] * G[3]); \
+                    }
+                    QLSKUM_DOT(0)
+                    QLSKUM_DOT(1)
+                    QLSKUM_DOT(2)
+                    QLSKUM_DOT(3)
+#undef QLSKUM_DOT
+                }
+                if (f != kInterior) {
+                    const double bs = bt[1], bn = bt[2];
+                    bt[1] = fma(bs, ny, bn * nx);
+                    bt[2] = fma(bn, ny, -(bs * nx));
+                }
+#pragma unroll
+                for (int r = 0; r < 4; r++) {
+                    double bdn, bdp;
+                    limited_vjp(s.l[r], bt[r], bdn, bdp);
+                    if (GEO) {
+                        bdelx = fma(-0.5 * bdn, dx[r], bdelx);
+                        bdely = fma(-0.5 * bdn, dy[r], bdely);
+                    } else {
+                        const bool up = __double2hiint(s.l[r].dn) >= 0;
+                        if (own) {
+                            const int t = threadIdx.x;
+                            sum[r][t] += bt[r] - bdp;
+                            sum[4 + r][t] = fma(hx, bdn, sum[4 + r][t]);
+                            sum[8 + r][t] = fma(hy, bdn, sum[8 + r][t]);
+                            sum[(up ? 12 : 16) + r][t] += bdp;
+                        } else {
+                            atomicAdd(reinterpret_cast<double *>(bq + k) + r, bt[r] - bdp);
+                            atomicAdd(reinterpret_cast<double *>(bdq + 2 * k) + r, hx * bdn);
+                            atomicAdd(reinterpret_cast<double *>(bdq + 2 * k + 1) + r, hy * bdn);
+                            if (bdp != 0.0) atomicAdd(reinterpret_cast<double *>(bqm + 2 * k + (up ? 0 : 1)) + r, bdp);
+                        }
+                    }
+                }
+            }
+            if (GEO) {
+                const double2 sw = c.e_sn[e];
+                const double sc = f == kWall ? 2.0 : 1.0;
+                double bsx = 0.0, bsy = 0.0;
+#pragma unroll
+                for (int d = 0; d < 4; d++) {
+                    if ((d == 2 && f == kWall) || (d == 3 && f == kOuter)) continue;
+                    const double4_32a m = c.fgeo[4 * (size_t)i + d];
+                    const double gd = sc * dot[d];
+                    const double ax = d < 2 ? m.y * m.w : -m.z * m.w, ay = d < 2 ? -m.z * m.w : m.x * m.w;
+                    bsx += ax * gd;
+                    bsy += ay * gd;
+                    sum[2 * d][threadIdx.x] += gd * sw.x;
+                    sum[2 * d + 1][threadIdx.x] += gd * sw.y;
+                }
+                sum[8][threadIdx.x] += bnx;
+                sum[9][threadIdx.x] += bny;
+                double4_32a &ge = a.bedge[e];
+                ge.x += bdelx;
+                ge.y += bdely;
+                ge.z += bsx;
+                ge.w += bsy;
             }
         }
-        double4_32a &acc = a.bfmom[4 * i + d];
-        acc.x += bm[0];
-        acc.y += bm[1];
-        acc.z += bm[2];
-        acc.w += bm[3];
     }
-    if (!geo) {
-        double F[4];
-        ld4(flux[i], F);
-        bdl = (bFi[0] * F[0] + bFi[1] * F[1] + bFi[2] * F[2] + bFi[3] * F[3]) / dl;
-    }
-    if (STATE) bdelta[i] += bdl;
-
-    // reverse over the edges, one end at a time (end64 / end64_vjp): the
-    // neighbour's end first, its bars scattered, then the owner's
-    double bqi[4] = {0, 0, 0, 0}, bdxi[4] = {0, 0, 0, 0}, bdyi[4] = {0, 0, 0, 0}, bmxi[4] = {0, 0, 0, 0},
-           bmni[4] = {0, 0, 0, 0};
-    double bnx = 0.0, bny = 0.0;
-    for (int j = 0; j < nb; j++) {
-        const long long e = base + 32LL * j;
-        const int k = c.e_nbr[e];
-        const double4_32a g = c.e_geo[e];
-        const double2 sw = c.e_sn[e];
-        const unsigned dir = c.e_dir[e];
-        double bdelx = 0.0, bdely = 0.0, bsw_x = 0.0, bsw_y = 0.0;
-        // the bar of G_k on half-range D is bG (ax sw.x + ay sw.y), that of G_i its negative
-#define QLSKUM_REV(D, SGN, KIN, KB)                                                  \
-        if (dir & (1u << D)) {                                                       \
-            const double fw = SGN * (ax[D] * sw.x + ay[D] * sw.y);                   \
-            double bG[4];                                                            \
-            for (int r = 0; r < 4; r++) bG[r] = fw * bG4[r];                         \
-            adj::dir_flux_vjp<D>(f, KIN, bG, KB);                                    \
-            if (geo) {                                                               \
-                double G[4];                                                         \
-                dir_flux<double, D>(f, KIN, G);                                      \
-                const double gb = bG4[0] * G[0] + bG4[1] * G[1] + bG4[2] * G[2] + bG4[3] * G[3]; \
-                bsw_x += SGN * ax[D] * gb;                                           \
-                bsw_y += SGN * ay[D] * gb;                                           \
-            }                                                                        \
+    __syncthreads();
+    for (int w = threadIdx.x; w < NS * P; w += T) {
+        const int s = w / P, pp = w % P, to = blockIdx.x * P + pp;
+        double v = 0.0;
+#pragma unroll
+        for (int g = 0; g < T / P; g++) v += sum[s][g * P + pp];
+        if (GEO) {
+            sum[s][pp] = v;  // read and written by this thread alone
+        } else if (to < n) {
+            const int r = s & 3;
+            double4_32a *dst = s < 4 ? bq + to : s < 8 ? bdq + 2 * to : s < 12 ? bdq + 2 * to + 1 : s < 16 ? bqm + 2 * to : bqm + 2 * to + 1;
+            if (s < 12 || v != 0.0) atomicAdd(reinterpret_cast<double *>(dst) + r, v);
         }
-        {
-            double qk[4], dxk[4], dyk[4], mxk[4], mnk[4];
-            ld4(q[k], qk);
-            ld4(dq[2 * k], dxk);
-            ld4(dq[2 * k + 1], dyk);
-            ld4(qm[2 * k], mxk);
-            ld4(qm[2 * k + 1], mnk);
-            adj::End64 s;
-            double kept[6];
-            if (ends)
-                for (int w = 0; w < 6; w++) kept[w] = ends[(6 + w) * ns + e];
-            adj::end64(nx, ny, g.x, g.y, qk, dxk, dyk, mxk, mnk, c.eps2[k], s, ends ? kept : nullptr);
-            KinBar kb;
-            QLSKUM_REV(0, 1.0, s.k, kb)
-            QLSKUM_REV(1, 1.0, s.k, kb)
-            QLSKUM_REV(2, 1.0, s.k, kb)
-            QLSKUM_REV(3, 1.0, s.k, kb)
-            double bqk[4] = {0, 0, 0, 0}, bdxk[4] = {0, 0, 0, 0}, bdyk[4] = {0, 0, 0, 0}, bmxk[4] = {0, 0, 0, 0},
-                   bmnk[4] = {0, 0, 0, 0};
-            adj::end64_vjp(s, nx, ny, g.x, g.y, dxk, dyk, kb, bqk, bdxk, bdyk, bmxk, bmnk, bdelx, bdely, bnx, bny);
-            if (STATE) {
-                atomic_add4(bq + k, bqk);
-                atomic_add4(bdq + 2 * k, bdxk);
-                atomic_add4(bdq + 2 * k + 1, bdyk);
-                atomic_add4(bqm + 2 * k, bmxk);
-                atomic_add4(bqm + 2 * k + 1, bmnk);
+    }
+    if (GEO) {
+        __syncthreads();
+        if (has && threadIdx.x < P) {
+#pragma unroll
+            for (int d = 0; d < 4; d++) {
+                const int f = c.flag[i];
+                if ((d == 2 && f == kWall) || (d == 3 && f == kOuter)) continue;
+                const double4_32a m = c.fgeo[4 * (size_t)i + d];
+                const double X = sum[2 * d][p], Y = sum[2 * d + 1][p];
+                double4_32a &o = a.bfmom[4 * (size_t)i + d];
+                if (d < 2) {
+                    o.y += X * m.w;
+                    o.z -= Y * m.w;
+                    o.w += X * m.y - Y * m.z;
+                } else {
+                    o.x += Y * m.w;
+                    o.z -= X * m.w;
+                    o.w += Y * m.x - X * m.z;
+                }
+            }
+            if (a.bnrm) {
+                a.bnrm[i].x += sum[8][p];
+                a.bnrm[i].y += sum[9][p];
             }
         }
-        {
-            adj::End64 s;
-            double kept[6];
-            if (ends)
-                for (int w = 0; w < 6; w++) kept[w] = ends[w * ns + e];
-            adj::end64(nx, ny, g.x, g.y, qi, dxi, dyi, mxi, mni, e2i, s, ends ? kept : nullptr);
-            KinBar kb;
-            QLSKUM_REV(0, -1.0, s.k, kb)
-            QLSKUM_REV(1, -1.0, s.k, kb)
-            QLSKUM_REV(2, -1.0, s.k, kb)
-            QLSKUM_REV(3, -1.0, s.k, kb)
-            adj::end64_vjp(s, nx, ny, g.x, g.y, dxi, dyi, kb, bqi, bdxi, bdyi, bmxi, bmni, bdelx, bdely, bnx, bny);
-        }
-#undef QLSKUM_REV
-        if (geo) {
-            double4_32a &ge = a.bedge[e];
-            ge.x += bdelx;
-            ge.y += bdely;
-            ge.z += bsw_x;
-            ge.w += bsw_y;
-        }
-    }
-    if (STATE) {
-        atomic_add4(bq + i, bqi);
-        atomic_add4(bdq + 2 * i, bdxi);
-        atomic_add4(bdq + 2 * i + 1, bdyi);
-        atomic_add4(bqm + 2 * i, bmxi);
-        atomic_add4(bqm + 2 * i + 1, bmni);
-    }
-    if (geo && a.bnrm) {
-        a.bnrm[i].x += bnx;
-        a.bnrm[i].y += bny;
     }
 }
 
@@ -1156,11 +1293,16 @@ void flux(const Launch &L, const AdjView &a, const double4_32a *q, const double4
           const double *delta, const double4_32a *flux, const double *ends, long long ns, const double4_32a *bF,
           double4_32a *bq, double4_32a *bdq, double4_32a *bqm, double *bdelta)
 {
-    adjk::k_flux<0><<<adjk::grid_for(a.c.n, 128), 128, 0, L.stream>>>(a, q, dq, qm, delta, flux, ends, ns, bF,
-                                                                       bq, bdq, bqm, bdelta);
-    if (a.bedge && a.n_geo > 0)
-        adjk::k_flux<2><<<adjk::grid_for(a.n_geo, 128), 128, 0, L.stream>>>(a, q, dq, qm, delta, flux, ends, ns,
-                                                                            bF, bq, bdq, bqm, bdelta);
+    const int n = a.c.n;
+#define QLSKUM_FLUX(P, GEO, N)                                                                                   \
+    adjk::k_flux<P, GEO><<<adjk::grid_for(N, P), adjk::kRevThreads, 0, L.stream>>>(a, q, dq, qm, delta, flux, ends, \
+                                                                                 ns, bF, bq, bdq, bqm, bdelta)
+    // as fp64::flux_shape
+    if (n <= 12288) QLSKUM_FLUX(8, false, n);
+    else if (n <= 65536) QLSKUM_FLUX(16, false, n);
+    else QLSKUM_FLUX(32, false, n);
+    if (a.bedge && a.n_geo > 0) QLSKUM_FLUX(8, true, a.n_geo);
+#undef QLSKUM_FLUX
 }
 
 void inner(const Launch &L, const AdjView &a, const double4_32a *q, const double4_32a *dq_in,

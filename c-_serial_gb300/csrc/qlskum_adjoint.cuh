@@ -212,8 +212,9 @@ template <typename R> QLSKUM_HD void edge_end_vjp(R delx, R dely, const R q[4], 
     }
 }
 
-// One edge end of the FP64 reverse, evaluated once per edge and end: the
-// limited reconstruction (interior_fluxes_mod.h:72-83, limiters_mod.h:64-104),
+// One edge end and its reverse in one piece, checked on the CPU against the
+// functions above; the device's flux reverse (adjk::k_flux) takes the same
+// steps in the forms of qlskum_fast64.cuh.  The limited reconstruction (interior_fluxes_mod.h:72-83, limiters_mod.h:64-104),
 // q~ -> prim (q_variables_mod.h:230-253) and the half-range moments
 // (split_fluxes_mod.h:14-26), keeping what end64_vjp reads.  The functions
 // above recompute each quantity they need (an edge end then costs 33 FP64

@@ -37,10 +37,10 @@ __device__ __forceinline__ bool within_cut(double x)
 // A finite seed that FP32 holds as a normal number.
 __device__ __forceinline__ bool seed_ok(float s) { return fabsf(s) > 1e-37f && fabsf(s) < 1e37f; }
 
-__device__ __noinline__ double div_slow(double a, double b) { return a / b; }
-__device__ __noinline__ double rsqrt_slow(double x) { return rsqrt(x); }
-__device__ __noinline__ double exp32_slow(double x) { return 32.0 * exp(x); }
-__device__ __noinline__ double2 gauss_erf_slow(double s) { return make_double2(0.5641895835477563 * exp(-s * s), erf(s)); }
+static __device__ __noinline__ double div_slow(double a, double b) { return a / b; }
+static __device__ __noinline__ double rsqrt_slow(double x) { return rsqrt(x); }
+static __device__ __noinline__ double exp32_slow(double x) { return 32.0 * exp(x); }
+static __device__ __noinline__ double2 gauss_erf_slow(double s) { return make_double2(0.5641895835477563 * exp(-s * s), erf(s)); }
 
 // num / den: the FP32 quotient corrected twice by its FP64 remainder.
 __device__ __forceinline__ double ratio64(double num, double den)
@@ -171,13 +171,13 @@ __device__ __forceinline__ void end(const DevCloud &c, int f, double nx, double 
 }
 
 // What the reverse reads back instead of evaluating it again, as planes of ns
-// doubles: rho, sqrt(beta), exp(-S1^2), exp(-S2^2), erf(S1), erf(S2).
-__device__ __forceinline__ void keep_end(double *__restrict__ o, long long ns, double t3, const End &s)
+// doubles: rho, r, exp(-S1^2) and exp(-S2^2) over sqrt(pi), erf(S1), erf(S2).
+__device__ __forceinline__ void keep_end(double *__restrict__ o, long long ns, const End &s)
 {
     o[0] = s.k.rho;
-    o[ns] = -t3 * s.r;
-    o[2 * ns] = 1.7724538509055159 * s.e1;
-    o[3 * ns] = 1.7724538509055159 * s.e2;
+    o[ns] = s.r;
+    o[2 * ns] = s.e1;
+    o[3 * ns] = s.e2;
     o[4 * ns] = s.k.E1;
     o[5 * ns] = s.k.E2;
 }
@@ -219,6 +219,28 @@ __device__ __forceinline__ void quad_x(const Kin<double> &k, unsigned sx, unsign
     v[1] = fma(wa, fma(k.ut, f, __dmul_rn(k.pbr, A1)), v[1]);
     v[2] = fma(wf, fma(k.un, A2, B2), v[2]);
     v[3] = fma(wa, fma(k.usq, f, __dmul_rn(k.pbr, fma(7.0, f, -B1))), fma(wf, __dmul_rn(k.un, B2), v[3]));
+}
+
+// a b - c d with one rounding of the difference (Kahan): the second product's
+// rounding error is added back.
+__device__ __forceinline__ double diff_of_products(double a, double b, double c, double d)
+{
+    const double w = c * d;
+    const double e = fma(-c, d, w);
+    return fma(a, b, -w) + e;
+}
+
+// The weight of half-range d's flux difference over an edge with rotated
+// vector sn in point i's residual: the row of the directional 2x2 solve
+// (interior_fluxes_mod.h:140-145 and its likes) times the edge's least-squares
+// weights; twice on the wall (flux_residual_mod.h:29), 0 for a half-range the
+// class does not use.
+__device__ __forceinline__ double flux_weight(const DevCloud &c, int i, int f, int d, double2 sn)
+{
+    if ((f == kWall && d == 2) || (f == kOuter && d == 3)) return 0.0;
+    const double4_32a m = c.fgeo[4 * (size_t)i + d];  // sxx, syy, sxy, 1/det
+    const double w = m.w * (d < 2 ? diff_of_products(m.y, sn.x, m.z, sn.y) : diff_of_products(m.x, sn.y, m.z, sn.x));
+    return f == kWall ? 2.0 * w : w;
 }
 
 // ------------------------------------------------------------ points

@@ -183,28 +183,6 @@ __global__ void k_func_delta(DevCloud c, const double4_32a *__restrict__ prim, d
 
 // ------------------------------------------------------------- flux
 
-// a b - c d with one rounding of the difference (Kahan): the second product's
-// rounding error is added back.
-__device__ __forceinline__ double diff_of_products(double a, double b, double c, double d)
-{
-    const double w = c * d;
-    const double e = fma(-c, d, w);
-    return fma(a, b, -w) + e;
-}
-
-// The weight of half-range d's flux difference over an edge with rotated
-// vector sn in point i's residual: the row of the directional 2x2 solve
-// (interior_fluxes_mod.h:140-145 and its likes) times the edge's least-squares
-// weights; twice on the wall (flux_residual_mod.h:29), 0 for a half-range the
-// class does not use.
-__device__ __forceinline__ double flux_weight(const DevCloud &c, int i, int f, int d, double2 sn)
-{
-    if ((f == kWall && d == 2) || (f == kOuter && d == 3)) return 0.0;
-    const double4_32a m = c.fgeo[4 * (size_t)i + d];  // sxx, syy, sxy, 1/det
-    const double w = m.w * (d < 2 ? diff_of_products(m.y, sn.x, m.z, sn.y) : diff_of_products(m.x, sn.y, m.z, sn.x));
-    return f == kWall ? 2.0 * w : w;
-}
-
 // Once per cloud: per edge {weight of its x half-range (xpos if it lies there,
 // else xneg), weight of its y half-range (ypos, else yneg)}, and the gradient's
 // 2x2 solve (q_variables_mod.h:112-116) times the edge's weights.
@@ -220,9 +198,9 @@ __global__ void k_fold_weights(DevCloud c, double2 *__restrict__ e_w64, double2 
         const unsigned dir = c.e_dir[e];
         const double2 sn = c.e_sn[e];
         const double4_32a g = c.e_geo[e];
-        e_w64[e] = make_double2(flux_weight(c, i, f, (dir & kXpos) ? 0 : 1, sn),
-                                flux_weight(c, i, f, (dir & kYpos) ? 2 : 3, sn));
-        e_gw64[e] = make_double2(m.w * diff_of_products(m.y, g.z, m.z, g.w), m.w * diff_of_products(m.x, g.w, m.z, g.z));
+        e_w64[e] = make_double2(fast64::flux_weight(c, i, f, (dir & kXpos) ? 0 : 1, sn),
+                                fast64::flux_weight(c, i, f, (dir & kYpos) ? 2 : 3, sn));
+        e_gw64[e] = make_double2(m.w * fast64::diff_of_products(m.y, g.z, m.z, g.w), m.w * fast64::diff_of_products(m.x, g.w, m.z, g.z));
     }
 }
 
@@ -279,7 +257,7 @@ __device__ __forceinline__ void edge_flux(const DevCloud &c, int i, int f, doubl
             t[r] = fast64::limited(qk[r], dn, (__double2hiint(dn) >= 0 ? mxk[r] : mnk[r]) - qk[r], e2k);
         }
         fast64::end(c, f, nx, ny, t, sk);
-        if (ends) fast64::keep_end(ends + 6 * ns + e, ns, t[3], sk);
+        if (ends) fast64::keep_end(ends + 6 * ns + e, ns, sk);
     }
 #pragma unroll
     for (int r = 0; r < 4; r++) {
@@ -287,7 +265,7 @@ __device__ __forceinline__ void edge_flux(const DevCloud &c, int i, int f, doubl
         t[r] = fast64::limited(o.q[r], dn, __double2hiint(dn) >= 0 ? o.mx[r] : o.mn[r], o.e2);
     }
     fast64::end(c, f, nx, ny, t, si);
-    if (ends) fast64::keep_end(ends + e, ns, t[3], si);
+    if (ends) fast64::keep_end(ends + e, ns, si);
 
     const unsigned dir = c.e_dir[e];
     const double2 w = c.e_w64[e];
@@ -305,7 +283,7 @@ __device__ __forceinline__ void edge_flux(const DevCloud &c, int i, int f, doubl
         fast64::quad_x(sk.k, sx, s2, w.x, v);
     }
     if ((dir & (kXpos | kXneg)) == (kXpos | kXneg)) {
-        const double w2 = flux_weight(c, i, f, 1, c.e_sn[e]);
+        const double w2 = fast64::flux_weight(c, i, f, 1, c.e_sn[e]);
         if (inner) {
             fast64::split_pair(si.k, neg, 0u, -w2, 0.0, v);
             fast64::split_pair(sk.k, neg, 0u, w2, 0.0, v);
@@ -315,7 +293,7 @@ __device__ __forceinline__ void edge_flux(const DevCloud &c, int i, int f, doubl
         }
     }
     if ((dir & (kYpos | kYneg)) == (kYpos | kYneg)) {
-        const double w2 = flux_weight(c, i, f, 3, c.e_sn[e]);
+        const double w2 = fast64::flux_weight(c, i, f, 3, c.e_sn[e]);
         fast64::split_pair(si.k, 0u, neg, 0.0, -w2, v);
         fast64::split_pair(sk.k, 0u, neg, 0.0, w2, v);
     }

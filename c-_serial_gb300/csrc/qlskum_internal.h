@@ -211,8 +211,7 @@ namespace adjl {
 void update(const Launch &L, const AdjView &a, const CaseConst &K, const double4_32a *Pin, const double4_32a *Pold,
             const double4_32a *Pout, int rk, double4_32a *bP, double4_32a *bPold, double4_32a *bF, double *buinf);
 // flux: the stage's flux residual (the bar of delta without geometry bars);
-// ends: the edge ends' kept transcendentals
-// (fp64::flux_residual's ends, ns slots), or NULL (recomputed)
+// ends: the edge ends' kept transcendentals (fp64::flux_residual's ends, ns slots)
 void flux(const Launch &L, const AdjView &a, const double4_32a *q, const double4_32a *dq, const double4_32a *qm,
           const double *delta, const double4_32a *flux, const double *ends, long long ns,
           const double4_32a *bF, double4_32a *bq, double4_32a *bdq, double4_32a *bqm, double *bdelta);
@@ -294,8 +293,8 @@ void q_inner(const Launch &L, const DevCloud &c, const double4_32a *q, const dou
              double4_32a *dq_out);
 void func_delta(const Launch &L, const DevCloud &c, const double4_32a *prim, double *delta, double cfl);
 // ends (or NULL): per edge slot of the ns slots, the owner's and the
-// neighbour's end's rho, sqrt(beta), exp(-S1^2), exp(-S2^2), erf(S1),
-// erf(S2), as 12 planes of ns doubles (read back by the flux reverse).
+// neighbour's end's values of fast64::keep_end, as 12 planes of ns doubles
+// (read back by the flux reverse).
 void flux_residual(const Launch &L, const DevCloud &c, const double4_32a *q, const double4_32a *dq, const double4_32a *qm,
                    const double *delta, double4_32a *flux_res, double *ends = nullptr, long long ns = 0);
 // one SSPRK stage of every point (prim_next may be prim)
