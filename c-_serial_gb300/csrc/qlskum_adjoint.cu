@@ -23,7 +23,7 @@ namespace adjk {
 
 using adj::KinBar;
 
-static inline int grid_for(int n, int block) { return (n + block - 1) / block; }
+static inline int grid_for(long long n, int block) { return (int)((n + block - 1) / block); }
 
 __device__ __forceinline__ void atomic_add4(double4_32a *p, const double v[4])
 {
@@ -431,185 +431,180 @@ __global__ void __launch_bounds__(kRevThreads, GEO ? 1 : 4) k_flux(AdjView a, co
     }
 }
 
-// Reverse of one inner iteration (q_variables_mod.h:120-213): bdq_out is the
-// bar of its output; adds bars of q and of its input dq.
-template <int MODE>
-__global__ void k_inner(AdjView a, const double4_32a *__restrict__ q, const double4_32a *__restrict__ dq_in,
-                        const double4_32a *__restrict__ bdq_out, double4_32a *__restrict__ bq,
-                        double4_32a *__restrict__ bdq_in)
+// The gradient's and the inner step's reverse: four lanes per point, one per
+// component, through the folded weights, as their forward kernels; the
+// geometry bars take a warp per listed point (eight edges at a time by four
+// components).  51,200 / 20,480 points, per launch: inner step 53 / 31 us with
+// one thread per point (its geometry bars 68), 32 / 16 (geometry 12); gradient 39 / 27
+// (geometry 39), 23 / 14 (geometry 10).
+//
+// One inner step (q_variables_mod.h:120-213) as the forward evaluates it:
+// dq_out = dq0 + (dq_in - sum_e g_e (d_e . dq_in_k)) / 2.  bdq_out is the bar
+// of its output; adds the bar of dq_in and sets (first) or adds that of dq0.
+__global__ void k_inner(DevCloud c, const double *__restrict__ bdq_out, double *__restrict__ bdq_in,
+                        double *__restrict__ bdq0, int first)
 {
-    // MODE 0: state bars everywhere; 2: geometry bars only, at AdjView::geo_list
-    constexpr bool STATE = MODE != 2;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (MODE == 2 ? a.n_geo : a.c.n)) return;
-    const int i = MODE == 2 ? a.geo_list[t] : t;
-    const DevCloud &c = a.c;
-    const bool geo = MODE != 0;
-    const double4_32a m = c.ggeo[i];
-    double bx[4], by[4];
-    ld4(bdq_out[2 * i], bx);
-    ld4(bdq_out[2 * i + 1], by);
-    double bsdx[4], bsdy[4];
-    for (int r = 0; r < 4; r++) {
-        bsdx[r] = m.w * (bx[r] * m.y - by[r] * m.z);
-        bsdy[r] = m.w * (by[r] * m.x - bx[r] * m.z);
-    }
-    double qi[4], dxi[4], dyi[4];
-    ld4(q[i], qi);
-    ld4(dq_in[2 * i], dxi);
-    ld4(dq_in[2 * i + 1], dyi);
+    const int i = t >> 2, r = t & 3;
+    if (i >= c.n) return;
+    const size_t o = 8 * (size_t)i + r;
+    const double bx = bdq_out[o], by = bdq_out[o + 4];
     const int nb = c.nbhs[i];
     const long long base = c.slice_base[i >> 5] + (i & 31);
-    double sdx[4] = {0, 0, 0, 0}, sdy[4] = {0, 0, 0, 0};
-    double bqi[4] = {0, 0, 0, 0}, bdxi[4] = {0, 0, 0, 0}, bdyi[4] = {0, 0, 0, 0};
     for (int j = 0; j < nb; j++) {
         const long long e = base + 32LL * j;
-        const int k = c.e_nbr[e];
-        const double4_32a g = c.e_geo[e];
-        double qk[4], dxk[4], dyk[4];
-        ld4(q[k], qk);
-        ld4(dq_in[2 * k], dxk);
-        ld4(dq_in[2 * k + 1], dyk);
-        double bqk[4], bdxk[4], bdyk[4];
-        double bgx = 0.0, bgy = 0.0, bwx = 0.0, bwy = 0.0;
-        for (int r = 0; r < 4; r++) {
-            const double t1 = qi[r] - 0.5 * (g.x * dxi[r] + g.y * dyi[r]);
-            const double t2 = qk[r] - 0.5 * (g.x * dxk[r] + g.y * dyk[r]);
-            sdx[r] += g.z * (t2 - t1);
-            sdy[r] += g.w * (t2 - t1);
-            const double bt = g.z * bsdx[r] + g.w * bsdy[r];
-            bqk[r] = bt;
-            bdxk[r] = -0.5 * g.x * bt;
-            bdyk[r] = -0.5 * g.y * bt;
-            bqi[r] -= bt;
-            bdxi[r] += 0.5 * g.x * bt;
-            bdyi[r] += 0.5 * g.y * bt;
-            if (geo) {
-                bwx += bsdx[r] * (t2 - t1);
-                bwy += bsdy[r] * (t2 - t1);
-                bgx += -0.5 * bt * (dxk[r] - dxi[r]);
-                bgy += -0.5 * bt * (dyk[r] - dyi[r]);
-            }
-        }
-        if (STATE) {
-            atomic_add4(bq + k, bqk);
-            atomic_add4(bdq_in + 2 * k, bdxk);
-            atomic_add4(bdq_in + 2 * k + 1, bdyk);
-        }
-        if (geo) {
-            // unit weights: w delx == delx
-            double4_32a &ge = a.bedge[e];
-            ge.x += bgx + bwx;
-            ge.y += bgy + bwy;
-        }
+        const double2 gw = c.e_gw64[e];
+        const double2 d = *reinterpret_cast<const double2 *>(c.e_geo + e);
+        const double bs = -0.5 * fma(gw.x, bx, gw.y * by);
+        double *to = bdq_in + 8 * (size_t)c.e_nbr[e] + r;
+        atomicAdd(to, d.x * bs);
+        atomicAdd(to + 4, d.y * bs);
     }
-    if (STATE) {
-        atomic_add4(bq + i, bqi);
-        atomic_add4(bdq_in + 2 * i, bdxi);
-        atomic_add4(bdq_in + 2 * i + 1, bdyi);
-    }
-    if (geo) {
-        double bm[4] = {0, 0, 0, 0};
-        for (int r = 0; r < 4; r++) {
-            // dx = ood (Sx syy - Sy sxy), dy = ood (Sy sxx - Sx sxy)
-            bm[1] += m.w * bx[r] * sdx[r];
-            bm[2] += -m.w * (bx[r] * sdy[r] + by[r] * sdx[r]);
-            bm[0] += m.w * by[r] * sdy[r];
-            bm[3] += bx[r] * (sdx[r] * m.y - sdy[r] * m.z) + by[r] * (sdy[r] * m.x - sdx[r] * m.z);
-        }
-        double4_32a &acc = a.bgmom[i];
-        acc.x += bm[0];
-        acc.y += bm[1];
-        acc.z += bm[2];
-        acc.w += bm[3];
+    atomicAdd(bdq_in + o, 0.5 * bx);
+    atomicAdd(bdq_in + o + 4, 0.5 * by);
+    if (first) {
+        bdq0[o] = bx;
+        bdq0[o + 4] = by;
+    } else {
+        bdq0[o] += bx;
+        bdq0[o + 4] += by;
     }
 }
 
-// Reverse of the least-squares gradient and of the neighbour max / min
-// (q_variables_mod.h:36-118).
-template <int MODE>
-__global__ void k_grad(AdjView a, const double4_32a *__restrict__ q, const double4_32a *__restrict__ bdq,
-                       const double4_32a *__restrict__ bqm, double4_32a *__restrict__ bq)
+// Sum over the four components of a lane group / over the eight edge slots of a warp.
+__device__ __forceinline__ double sum_components(double v)
 {
-    // MODE 0: state bars everywhere; 2: geometry bars only, at AdjView::geo_list
-    constexpr bool STATE = MODE != 2;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (MODE == 2 ? a.n_geo : a.c.n)) return;
-    const int i = MODE == 2 ? a.geo_list[t] : t;
+    const unsigned mask = 0xfu << (threadIdx.x & 28u);
+    v += __shfl_xor_sync(mask, v, 1);
+    return v + __shfl_xor_sync(mask, v, 2);
+}
+
+__device__ __forceinline__ double sum_slots(double v)
+{
+#pragma unroll
+    for (int s = 4; s < 32; s <<= 1) v += __shfl_xor_sync(0xffffffffu, v, s);
+    return v;
+}
+
+// The bars of a point's gradient moments {sxx, syy, sxy, 1/det} for the bar
+// (bx, by) of solve(Sx, Sy), per component; summed and stored by lane 0.
+__device__ __forceinline__ void moment_bars(double4_32a &acc, const double4_32a &m, double bx, double by, double Sx,
+                                            double Sy)
+{
+    const double b0 = sum_components(m.w * by * Sy), b1 = sum_components(m.w * bx * Sx),
+                 b2 = sum_components(-m.w * (bx * Sy + by * Sx)),
+                 b3 = sum_components(bx * (Sx * m.y - Sy * m.z) + by * (Sy * m.x - Sx * m.z));
+    if ((threadIdx.x & 31) == 0) {
+        acc.x += b0;
+        acc.y += b1;
+        acc.z += b2;
+        acc.w += b3;
+    }
+}
+
+// The geometry bars of one inner step (unit weights: w delx == delx): those of
+// solve(sum_e d_e (d_e . dq_in_k)) with the bar -bdq_out / 2.
+__global__ void k_inner_geo(AdjView a, const double *__restrict__ dq_in, const double *__restrict__ bdq_out)
+{
+    const int at = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (at >= a.n_geo) return;
     const DevCloud &c = a.c;
-    const bool geo = MODE != 0;
+    const int i = a.geo_list[at], r = lane & 3;
     const double4_32a m = c.ggeo[i];
-    double bx[4], by[4], bmax[4], bmin[4];
-    ld4(bdq[2 * i], bx);
-    ld4(bdq[2 * i + 1], by);
-    ld4(bqm[2 * i], bmax);
-    ld4(bqm[2 * i + 1], bmin);
-    double bsdx[4], bsdy[4];
-    for (int r = 0; r < 4; r++) {
-        bsdx[r] = (bx[r] * m.y - by[r] * m.z) * m.w;
-        bsdy[r] = (by[r] * m.x - bx[r] * m.z) * m.w;
-    }
-    double qi[4];
-    ld4(q[i], qi);
-    double qmax[4], qmin[4];
-    int amax[4], amin[4];
-    for (int r = 0; r < 4; r++) {
-        qmax[r] = qmin[r] = qi[r];
-        amax[r] = amin[r] = i;
-    }
+    const double bx = -0.5 * bdq_out[8 * (size_t)i + r], by = -0.5 * bdq_out[8 * (size_t)i + 4 + r];
+    const double bsx = m.w * (bx * m.y - by * m.z), bsy = m.w * (by * m.x - bx * m.z);
+    double Sx = 0.0, Sy = 0.0;
     const int nb = c.nbhs[i];
     const long long base = c.slice_base[i >> 5] + (i & 31);
-    double sdx[4] = {0, 0, 0, 0}, sdy[4] = {0, 0, 0, 0};
-    double bqi[4] = {0, 0, 0, 0};
+    for (int j = lane >> 2; j < nb; j += 8) {
+        const long long e = base + 32LL * j;
+        const double2 d = *reinterpret_cast<const double2 *>(c.e_geo + e);
+        const size_t k = 8 * (size_t)c.e_nbr[e] + r;
+        const double gx = dq_in[k], gy = dq_in[k + 4];
+        const double u = d.x * gx + d.y * gy, bu = bsx * d.x + bsy * d.y;
+        Sx += d.x * u;
+        Sy += d.y * u;
+        const double ex = sum_components(bsx * u + bu * gx), ey = sum_components(bsy * u + bu * gy);
+        if (r == 0) {
+            double4_32a &ge = a.bedge[e];
+            ge.x += ex;
+            ge.y += ey;
+        }
+    }
+    moment_bars(a.bgmom[i], m, bx, by, sum_slots(Sx), sum_slots(Sy));
+}
+
+// Reverse of the least-squares gradient and of the neighbour max / min
+// (q_variables_mod.h:36-118): adds the bars of q.  The gradient's bar is
+// bdq + bdq0 (bdq0 NULL: bdq alone).
+__global__ void k_grad(DevCloud c, const double *__restrict__ q, const double *__restrict__ bdq,
+                       const double *__restrict__ bdq0, const double *__restrict__ bqm, double *__restrict__ bq)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = t >> 2, r = t & 3;
+    if (i >= c.n) return;
+    const size_t o = 8 * (size_t)i + r;
+    double bx = bdq[o], by = bdq[o + 4];
+    if (bdq0) {
+        bx += bdq0[o];
+        by += bdq0[o + 4];
+    }
+    const double bmax = bqm[o], bmin = bqm[o + 4];
+    long long kmax = fast64::order_key(__double_as_longlong(q[4 * (size_t)i + r])), kmin = kmax;
+    int amax = i, amin = i;
+    double own = 0.0;
+    const int nb = c.nbhs[i];
+    const long long base = c.slice_base[i >> 5] + (i & 31);
     for (int j = 0; j < nb; j++) {
         const long long e = base + 32LL * j;
         const int k = c.e_nbr[e];
-        const double4_32a g = c.e_geo[e];
-        double qk[4], bqk[4];
-        ld4(q[k], qk);
-        double bwx = 0.0, bwy = 0.0;
-        for (int r = 0; r < 4; r++) {
-            if (qk[r] > qmax[r]) { qmax[r] = qk[r]; amax[r] = k; }
-            if (qk[r] < qmin[r]) { qmin[r] = qk[r]; amin[r] = k; }
-            sdx[r] += g.z * (qk[r] - qi[r]);
-            sdy[r] += g.w * (qk[r] - qi[r]);
-            const double bt = g.z * bsdx[r] + g.w * bsdy[r];
-            bqk[r] = bt;
-            bqi[r] -= bt;
-            if (geo) {
-                bwx += bsdx[r] * (qk[r] - qi[r]);
-                bwy += bsdy[r] * (qk[r] - qi[r]);
-            }
-        }
-        if (STATE) atomic_add4(bq + k, bqk);
-        if (geo) {
+        const double2 gw = c.e_gw64[e];
+        const long long key = fast64::order_key(__double_as_longlong(q[4 * (size_t)k + r]));
+        if (key > kmax) { kmax = key; amax = k; }
+        if (key < kmin) { kmin = key; amin = k; }
+        const double bt = fma(gw.x, bx, gw.y * by);
+        own -= bt;
+        atomicAdd(bq + 4 * (size_t)k + r, bt);
+    }
+    atomicAdd(bq + 4 * (size_t)i + r, own);
+    if (bmax != 0.0) atomicAdd(bq + 4 * (size_t)amax + r, bmax);
+    if (bmin != 0.0) atomicAdd(bq + 4 * (size_t)amin + r, bmin);
+}
+
+// Its geometry bars (unit weights).
+__global__ void k_grad_geo(AdjView a, const double *__restrict__ q, const double *__restrict__ bdq,
+                           const double *__restrict__ bdq0)
+{
+    const int at = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (at >= a.n_geo) return;
+    const DevCloud &c = a.c;
+    const int i = a.geo_list[at], r = lane & 3;
+    const double4_32a m = c.ggeo[i];
+    const size_t o = 8 * (size_t)i + r;
+    double bx = bdq[o], by = bdq[o + 4];
+    if (bdq0) {
+        bx += bdq0[o];
+        by += bdq0[o + 4];
+    }
+    const double bsx = m.w * (bx * m.y - by * m.z), bsy = m.w * (by * m.x - bx * m.z);
+    const double qi = q[4 * (size_t)i + r];
+    double Sx = 0.0, Sy = 0.0;
+    const int nb = c.nbhs[i];
+    const long long base = c.slice_base[i >> 5] + (i & 31);
+    for (int j = lane >> 2; j < nb; j += 8) {
+        const long long e = base + 32LL * j;
+        const double2 d = *reinterpret_cast<const double2 *>(c.e_geo + e);
+        const double u = q[4 * (size_t)c.e_nbr[e] + r] - qi;
+        Sx += d.x * u;
+        Sy += d.y * u;
+        const double ex = sum_components(bsx * u), ey = sum_components(bsy * u);
+        if (r == 0) {
             double4_32a &ge = a.bedge[e];
-            ge.x += bwx;
-            ge.y += bwy;
+            ge.x += ex;
+            ge.y += ey;
         }
     }
-    if (STATE) {
-        atomic_add4(bq + i, bqi);
-        double *bqd = reinterpret_cast<double *>(bq);
-        for (int r = 0; r < 4; r++) {
-            if (bmax[r] != 0.0) atomicAdd(bqd + 4 * (size_t)amax[r] + r, bmax[r]);
-            if (bmin[r] != 0.0) atomicAdd(bqd + 4 * (size_t)amin[r] + r, bmin[r]);
-        }
-    }
-    if (geo) {
-        double bm[4] = {0, 0, 0, 0};
-        for (int r = 0; r < 4; r++) {
-            bm[1] += m.w * bx[r] * sdx[r];
-            bm[2] += -m.w * (bx[r] * sdy[r] + by[r] * sdx[r]);
-            bm[0] += m.w * by[r] * sdy[r];
-            bm[3] += bx[r] * (sdx[r] * m.y - sdy[r] * m.z) + by[r] * (sdy[r] * m.x - sdx[r] * m.z);
-        }
-        double4_32a &acc = a.bgmom[i];
-        acc.x += bm[0];
-        acc.y += bm[1];
-        acc.z += bm[2];
-        acc.w += bm[3];
-    }
+    moment_bars(a.bgmom[i], m, bx, by, sum_slots(Sx), sum_slots(Sy));
 }
 
 // bP += (dq/dP)^T bq  (q_variables_mod.h:19-33)
@@ -627,39 +622,43 @@ __global__ void k_q(int n, const double4_32a *__restrict__ P, const double4_32a 
 }
 
 // Reverse of the local time step (state_update_mod.h:448-496): the bar of
-// delta_i goes to the wave speed of the neighbour that set the minimum.
+// delta_i goes to the wave speed (cs, of the same state) of the neighbour that
+// set the minimum, the first of equals.  Four lanes share a point's edges.
 template <bool GEO>
-__global__ void k_delta(AdjView a, const double4_32a *__restrict__ P, const double *__restrict__ bdelta,
-                        double cfl, double *__restrict__ bc)
+__global__ void k_delta(AdjView a, const double *__restrict__ cs, const double *__restrict__ bdelta, double cfl,
+                        double *__restrict__ bc)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = t >> 2, r = t & 3;
     if (i >= a.c.n) return;
     const DevCloud &c = a.c;
-    double min_delt = 1.0;
-    int arg = -1;
-    long long earg = -1;
-    double carg = 0.0;
+    double m = 1.0;
+    int arg = 0x7fffffff;
     const int nb = c.nbhs[i];
     const long long base = c.slice_base[i >> 5] + (i & 31);
-    for (int j = 0; j < nb; j++) {
+    for (int j = r; j < nb; j += 4) {
         const long long e = base + 32LL * j;
-        const int k = c.e_nbr[e];
-        double p[4];
-        ld4(P[k], p);
-        const double ck = wave_speed(p);
-        double dt = c.e_dist[e] / ck;
-        dt = cfl * dt;
-        if (min_delt > dt) {
-            min_delt = dt;
-            arg = k;
-            earg = e;
-            carg = ck;
+        const double dt = fast64::edge_dt(c.e_dist[e], cs[c.e_nbr[e]], cfl);
+        if (m > dt) {
+            m = dt;
+            arg = j;
         }
     }
-    if (arg >= 0 && bdelta[i] != 0.0) {
-        atomicAdd(bc + arg, -bdelta[i] * cfl * c.e_dist[earg] / (carg * carg));
-        if (GEO && a.geo_pt[i]) a.bdist[earg] += bdelta[i] * cfl / carg;
+    const unsigned mask = 0xfu << (threadIdx.x & 28u);
+#pragma unroll
+    for (int s = 1; s < 4; s <<= 1) {
+        const double x = __shfl_xor_sync(mask, m, s);
+        const int y = __shfl_xor_sync(mask, arg, s);
+        if (x < m || (x == m && y < arg)) {
+            m = x;
+            arg = y;
+        }
     }
+    if (r != 0 || arg == 0x7fffffff || bdelta[i] == 0.0) return;
+    const long long e = base + 32LL * arg;
+    const double ck = cs[c.e_nbr[e]];
+    atomicAdd(bc + c.e_nbr[e], -bdelta[i] * cfl * c.e_dist[e] / (ck * ck));
+    if (GEO && a.geo_pt[i]) a.bdist[e] += bdelta[i] * cfl / ck;
 }
 
 __global__ void k_wave(int n, const double4_32a *__restrict__ P, const double *__restrict__ bc,
@@ -1305,20 +1304,26 @@ void flux(const Launch &L, const AdjView &a, const double4_32a *q, const double4
 #undef QLSKUM_FLUX
 }
 
-void inner(const Launch &L, const AdjView &a, const double4_32a *q, const double4_32a *dq_in,
-           const double4_32a *bdq_out, double4_32a *bq, double4_32a *bdq_in)
+void inner(const Launch &L, const AdjView &a, const double4_32a *dq_in, const double4_32a *bdq_out, double4_32a *bdq_in,
+           double4_32a *bdq0, bool first)
 {
-    adjk::k_inner<0><<<adjk::grid_for(a.c.n, 128), 128, 0, L.stream>>>(a, q, dq_in, bdq_out, bq, bdq_in);
+    const double *b = reinterpret_cast<const double *>(bdq_out);
+    adjk::k_inner<<<adjk::grid_for(4 * (long long)a.c.n, 128), 128, 0, L.stream>>>(
+        a.c, b, reinterpret_cast<double *>(bdq_in), reinterpret_cast<double *>(bdq0), first);
     if (a.bedge && a.n_geo > 0)
-        adjk::k_inner<2><<<adjk::grid_for(a.n_geo, 128), 128, 0, L.stream>>>(a, q, dq_in, bdq_out, bq, bdq_in);
+        adjk::k_inner_geo<<<adjk::grid_for(32LL * a.n_geo, 64), 64, 0, L.stream>>>(
+            a, reinterpret_cast<const double *>(dq_in), b);
 }
 
-void grad(const Launch &L, const AdjView &a, const double4_32a *q, const double4_32a *bdq, const double4_32a *bqm,
-          double4_32a *bq)
+void grad(const Launch &L, const AdjView &a, const double4_32a *q, const double4_32a *bdq, const double4_32a *bdq0,
+          const double4_32a *bqm, double4_32a *bq)
 {
-    adjk::k_grad<0><<<adjk::grid_for(a.c.n, 128), 128, 0, L.stream>>>(a, q, bdq, bqm, bq);
+    const double *q1 = reinterpret_cast<const double *>(q), *b = reinterpret_cast<const double *>(bdq),
+                 *b0 = reinterpret_cast<const double *>(bdq0);
+    adjk::k_grad<<<adjk::grid_for(4 * (long long)a.c.n, 128), 128, 0, L.stream>>>(
+        a.c, q1, b, b0, reinterpret_cast<const double *>(bqm), reinterpret_cast<double *>(bq));
     if (a.bedge && a.n_geo > 0)
-        adjk::k_grad<2><<<adjk::grid_for(a.n_geo, 128), 128, 0, L.stream>>>(a, q, bdq, bqm, bq);
+        adjk::k_grad_geo<<<adjk::grid_for(32LL * a.n_geo, 64), 64, 0, L.stream>>>(a, q1, b, b0);
 }
 
 void qvars(const Launch &L, int n, const double4_32a *P, const double4_32a *bq, double4_32a *bP)
@@ -1326,13 +1331,13 @@ void qvars(const Launch &L, int n, const double4_32a *P, const double4_32a *bq, 
     adjk::k_q<<<adjk::grid_for(n, 256), 256, 0, L.stream>>>(n, P, bq, bP);
 }
 
-void delta(const Launch &L, const AdjView &a, const double4_32a *P, const double *bdelta, double cfl, double *bc,
-           double4_32a *bP)
+void delta(const Launch &L, const AdjView &a, const double4_32a *P, const double *bdelta, double cfl, double *cs,
+           double *bc, double4_32a *bP)
 {
-    if (a.bdist)
-        adjk::k_delta<true><<<adjk::grid_for(a.c.n, 128), 128, 0, L.stream>>>(a, P, bdelta, cfl, bc);
-    else
-        adjk::k_delta<false><<<adjk::grid_for(a.c.n, 128), 128, 0, L.stream>>>(a, P, bdelta, cfl, bc);
+    fp64::wave_speeds(L, a.c.n, P, cs);
+    const int g = adjk::grid_for(4 * (long long)a.c.n, 128);
+    if (a.bdist) adjk::k_delta<true><<<g, 128, 0, L.stream>>>(a, cs, bdelta, cfl, bc);
+    else adjk::k_delta<false><<<g, 128, 0, L.stream>>>(a, cs, bdelta, cfl, bc);
     adjk::k_wave<<<adjk::grid_for(a.c.n, 256), 256, 0, L.stream>>>(a.c.n, P, bc, bP);
 }
 

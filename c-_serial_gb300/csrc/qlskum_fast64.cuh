@@ -243,6 +243,16 @@ __device__ __forceinline__ double flux_weight(const DevCloud &c, int i, int f, i
     return f == kWall ? 2.0 * w : w;
 }
 
+// Doubles in the order of signed integers (for max / min off the FP64 pipe);
+// its own inverse.
+__device__ __forceinline__ long long order_key(long long b) { return b ^ ((b >> 63) & 0x7fffffffffffffffLL); }
+
+// dist / speed * cfl of one edge (state_update_mod.h:483-488)
+__device__ __forceinline__ double edge_dt(double dist, double speed, double cfl)
+{
+    return cfl * ratio64(dist, speed);
+}
+
 // ------------------------------------------------------------ points
 // The point formulas of qlskum_math.cuh with every multiply-add explicit, so
 // that the module, fused and recording kernels, whatever the compiler inlines

@@ -58,14 +58,24 @@ __global__ void k_derived(int n, const double4_32a *__restrict__ prim, double4_3
 // four lanes gather the 32 bytes of a neighbour's q (or of each half of its
 // gradient) in one sector, and a small cloud fills four times the warps.
 
-// Doubles in the order of signed integers (for max / min off the FP64 pipe);
-// its own inverse.
-__device__ __forceinline__ long long order_key(long long b) { return b ^ ((b >> 63) & 0x7fffffffffffffffLL); }
-
-// dist / speed * cfl of one edge (state_update_mod.h:483-488)
-__device__ __forceinline__ double edge_dt(double dist, double speed, double cfl)
+// The local time step of point i (state_update_mod.h:448-496), its edges over
+// the point's four lanes.
+__device__ __forceinline__ void point_dt(const DevCloud &c, int i, int r, long long base, int nb,
+                                         const double *__restrict__ cs, double *__restrict__ delta, double cfl)
 {
-    return cfl * fast64::ratio64(dist, speed);
+    double m = 1.0;
+    for (int j = r; j < nb; j += 4) {
+        const long long e = base + 32LL * j;
+        const double dt = fast64::edge_dt(c.e_dist[e], cs[c.e_nbr[e]], cfl);
+        if (m > dt) m = dt;
+    }
+    const unsigned mask = 0xfu << (threadIdx.x & 28u);
+#pragma unroll
+    for (int s = 1; s < 4; s <<= 1) {
+        const double x = __shfl_xor_sync(mask, m, s);
+        if (m > x) m = x;
+    }
+    if (r == 0) delta[i] = m;
 }
 
 // q_variables_mod.h:36-118 (+ state_update_mod.h:448-496 when delta != null):
@@ -82,7 +92,7 @@ __global__ void k_q_derivatives(DevCloud c, const double *__restrict__ q, double
     const int i = t >> 2, r = t & 3;
     if (i >= c.n) return;
     const double qi = q[4 * (size_t)i + r];
-    long long kmax = order_key(__double_as_longlong(qi)), kmin = kmax;
+    long long kmax = fast64::order_key(__double_as_longlong(qi)), kmin = kmax;
     double dx = 0.0, dy = 0.0;
     const int nb = c.nbhs[i];
     const long long base = c.slice_base[i >> 5] + (i & 31);
@@ -91,7 +101,7 @@ __global__ void k_q_derivatives(DevCloud c, const double *__restrict__ q, double
         const long long e = base + 32LL * j;
         const double2 gw = c.e_gw64[e];
         const double qk = q[4 * (size_t)c.e_nbr[e] + r];
-        const long long key = order_key(__double_as_longlong(qk));
+        const long long key = fast64::order_key(__double_as_longlong(qk));
         kmax = key > kmax ? key : kmax;
         kmin = key < kmin ? key : kmin;
         const double d = qk - qi;
@@ -101,23 +111,9 @@ __global__ void k_q_derivatives(DevCloud c, const double *__restrict__ q, double
     const size_t o = 8 * (size_t)i + r;
     dq[o] = dx;
     dq[o + 4] = dy;
-    qm[o] = __longlong_as_double(order_key(kmax));
-    qm[o + 4] = __longlong_as_double(order_key(kmin));
-    if (DT) {
-        double m = 1.0;
-        for (int j = r; j < nb; j += 4) {
-            const long long e = base + 32LL * j;
-            const double dt = edge_dt(c.e_dist[e], cs[c.e_nbr[e]], cfl);
-            if (m > dt) m = dt;
-        }
-        const unsigned mask = 0xfu << (threadIdx.x & 28u);
-#pragma unroll
-        for (int s = 1; s < 4; s <<= 1) {
-            const double x = __shfl_xor_sync(mask, m, s);
-            if (m > x) m = x;
-        }
-        if (r == 0) delta[i] = m;
-    }
+    qm[o] = __longlong_as_double(fast64::order_key(kmax));
+    qm[o + 4] = __longlong_as_double(fast64::order_key(kmin));
+    if (DT) point_dt(c, i, r, base, nb, cs, delta, cfl);
 }
 
 // q_variables_mod.h:120-213: the reference's sums over w d (t_k - t_i),
@@ -163,22 +159,23 @@ __global__ void k_q_inner(DevCloud c, const double *__restrict__ q, const double
     dq_out[o + 4] = fma(0.5, dq_in[o + 4] - ay, d0y);
 }
 
-// state_update_mod.h:448-496, wave speed evaluated per edge as the reference does.
-__global__ void k_func_delta(DevCloud c, const double4_32a *__restrict__ prim, double *__restrict__ delta, double cfl)
+// state_update_mod.h:448-496 from the points' wave speeds.  51,200 points: 44 us
+// with the neighbour's wave speed evaluated at every edge, 12 us with
+// k_wave_speeds (5 us) before it.
+__global__ void k_func_delta(DevCloud c, const double *__restrict__ cs, double *__restrict__ delta, double cfl)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
-    double min_delt = 1.0;
-    const int nb = c.nbhs[i];
-    const long long base = c.slice_base[i >> 5] + (i & 31);
-    for (int j = 0; j < nb; j++) {
-        const long long e = base + 32LL * j;
-        double P[4];
-        ld4(prim[c.e_nbr[e]], P);
-        const double delta_t = edge_dt(c.e_dist[e], fast64::wave_speed(P), cfl);
-        if (min_delt > delta_t) min_delt = delta_t;
-    }
-    delta[i] = min_delt;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = t >> 2;
+    if (i < c.n) point_dt(c, i, t & 3, c.slice_base[i >> 5] + (i & 31), c.nbhs[i], cs, delta, cfl);
+}
+
+__global__ void k_wave_speeds(int n, const double4_32a *__restrict__ prim, double *__restrict__ cs)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    double P[4];
+    ld4(prim[i], P);
+    cs[i] = fast64::wave_speed(P);
 }
 
 // ------------------------------------------------------------- flux
@@ -737,9 +734,16 @@ void q_inner(const Launch &L, const DevCloud &c, const double4_32a *q, const dou
     QLSKUM_LAUNCHED(L);
 }
 
-void func_delta(const Launch &L, const DevCloud &c, const double4_32a *prim, double *delta, double cfl)
+void wave_speeds(const Launch &L, int n, const double4_32a *prim, double *cs)
 {
-    k_func_delta<<<grid_for(c.n, L.block), L.block, 0, L.stream>>>(c, prim, delta, cfl);
+    k_wave_speeds<<<grid_for(n, 64), 64, 0, L.stream>>>(n, prim, cs);
+    QLSKUM_LAUNCHED(L);
+}
+
+void func_delta(const Launch &L, const DevCloud &c, const double4_32a *prim, double *cs, double *delta, double cfl)
+{
+    wave_speeds(L, c.n, prim, cs);
+    k_func_delta<<<grid_for(4 * (long long)c.n, L.block), L.block, 0, L.stream>>>(c, cs, delta, cfl);
     QLSKUM_LAUNCHED(L);
 }
 

@@ -1093,7 +1093,8 @@ qlskum_status qlskum_destroy(qlskum_handle *h)
 qlskum_status qlskum_func_delta(qlskum_handle *h)
 {
     NEED(h);
-    fp64::func_delta(h->L, h->dc, h->s64.prim[h->pcur], h->s64.delta, h->K.cfl);
+    // s64.cspeed holds this same state's wave speeds whenever the fused iteration reads it
+    fp64::func_delta(h->L, h->dc, h->s64.prim[h->pcur], h->s64.cspeed, h->s64.delta, h->K.cfl);
     return check_launch(h, "func_delta");
 }
 
@@ -2938,8 +2939,8 @@ struct AdjBuf {
     Set64 set64;                       // the FP64 stage data of one iteration (its states are P)
     std::vector<Set64> sets64;         // one per iteration of a segment, on demand (set_arena)
     double4_32a *bP = nullptr, *bPacc = nullptr, *bF = nullptr, *bq = nullptr, *bdqA = nullptr, *bdqB = nullptr,
-                *bqm = nullptr, *lam = nullptr, *lam_prev = nullptr, *seed = nullptr;
-    double *bdelta = nullptr, *bc = nullptr, *buinf = nullptr;
+                *bdq0 = nullptr, *bqm = nullptr, *lam = nullptr, *lam_prev = nullptr, *seed = nullptr;
+    double *bdelta = nullptr, *bc = nullptr, *cs = nullptr, *buinf = nullptr;
     // geometry adjoints (wall-displacement gradients only)
     double4_32a *bedge = nullptr;
     double *bdist = nullptr;
@@ -3170,9 +3171,10 @@ qlskum_status adj_alloc(qlskum_handle *h, bool geo, bool need64, bool need32)
         alloc_set64(A, np, a->ne, a->ni, a->set64);
         for (int k = 0; k < 5; k++) a->set64.P[k] = a->P[k];
         a->bq = A.alloc<double4_32a>(np);
-        for (auto *p : {&a->bdqA, &a->bdqB, &a->bqm}) *p = A.alloc<double4_32a>(2 * np);
+        for (auto *p : {&a->bdqA, &a->bdqB, &a->bdq0, &a->bqm}) *p = A.alloc<double4_32a>(2 * np);
         a->bdelta = A.alloc<double>(np);
         a->bc = A.alloc<double>(np);
+        a->cs = A.alloc<double>(np);
     }
     if (need32) {
         alloc_set32(A, np, a->ni, a->set0);
@@ -3286,7 +3288,7 @@ void adj_stage_forward(qlskum_handle *h, Set64 &st, int s)
 // residual row is reduced and recorded, as qlskum_fpi_solver does).
 void adj_iteration_forward64(qlskum_handle *h, Set64 &st, int it_rec = 0)
 {
-    fp64::func_delta(h->L, h->dc, st.P[0], st.delta, h->K.cfl);
+    fp64::func_delta(h->L, h->dc, st.P[0], h->adj->cs, st.delta, h->K.cfl);
     for (int s = 0; s < 4; s++) {
         adj_stage_forward(h, st, s);
         fp64::state_update(h->L, h->dc, h->K, st.P[s], st.P[0], st.flux[s], st.P[s + 1], s + 1, h->R);
@@ -3313,10 +3315,10 @@ void adj_stage_reverse(qlskum_handle *h, const Set64 &st, int s, const AdjView &
                a->bdqA, a->bqm, a->bdelta);
     for (int j = ni; j >= 1; j--) {
         zero(h, a->bdqB, sizeof(double4_32a) * 2 * np);
-        adjl::inner(h->L, v, st.q[s], adj_dq(st, ni, s, j - 1), a->bdqA, a->bq, a->bdqB);
+        adjl::inner(h->L, v, adj_dq(st, ni, s, j - 1), a->bdqA, a->bdqB, a->bdq0, j == ni);
         std::swap(a->bdqA, a->bdqB);
     }
-    adjl::grad(h->L, v, st.q[s], a->bdqA, a->bqm, a->bq);
+    adjl::grad(h->L, v, st.q[s], a->bdqA, ni > 0 ? a->bdq0 : nullptr, a->bqm, a->bq);
     adjl::qvars(h->L, h->n, st.P[s], a->bq, a->bP);
 }
 
@@ -3334,7 +3336,7 @@ void adj_iteration_reverse64(qlskum_handle *h, const Set64 &st, const AdjView &v
         adj_stage_reverse(h, st, s, v);
     }
     zero(h, a->bc, sizeof(double) * np);
-    adjl::delta(h->L, v, st.P[0], a->bdelta, h->K.cfl, a->bc, a->bPacc);
+    adjl::delta(h->L, v, st.P[0], a->bdelta, h->K.cfl, a->cs, a->bc, a->bPacc);
     fp64::add_prim(h->L, h->n, a->bPacc, a->bP);
 }
 
@@ -3639,7 +3641,7 @@ qlskum_status qlskum_residual_forward(qlskum_handle *h, const double *prim, doub
     if (st) return st;
     AdjBuf *a = h->adj;
     if ((st = upload_points(h, prim, a->P[0], 1.0))) return st;
-    fp64::func_delta(h->L, h->dc, a->P[0], a->set64.delta, h->K.cfl);
+    fp64::func_delta(h->L, h->dc, a->P[0], a->cs, a->set64.delta, h->K.cfl);
     adj_stage_forward(h, a->set64, 0);
     if ((st = check_launch(h, "residual_forward"))) return st;
     return download_points(h, a->set64.flux[0], flux_res);
@@ -3654,14 +3656,14 @@ qlskum_status qlskum_residual_vjp(qlskum_handle *h, const double *prim, const do
     AdjBuf *a = h->adj;
     if ((st = upload_points(h, prim, a->P[0], 1.0))) return st;
     if ((st = upload_points(h, bar_flux_res, a->bF, 0.0))) return st;
-    fp64::func_delta(h->L, h->dc, a->P[0], a->set64.delta, h->K.cfl);
+    fp64::func_delta(h->L, h->dc, a->P[0], a->cs, a->set64.delta, h->K.cfl);
     adj_stage_forward(h, a->set64, 0);
     const AdjView v = adj_view(h, false);
     zero(h, a->bP, sizeof(double4_32a) * h->np);
     zero(h, a->bdelta, sizeof(double) * h->np);
     adj_stage_reverse(h, a->set64, 0, v);
     zero(h, a->bc, sizeof(double) * h->np);
-    adjl::delta(h->L, v, a->P[0], a->bdelta, h->K.cfl, a->bc, a->bP);
+    adjl::delta(h->L, v, a->P[0], a->bdelta, h->K.cfl, a->cs, a->bc, a->bP);
     if ((st = check_launch(h, "residual_vjp"))) return st;
     return download_points(h, a->bP, bar_prim);
 }
@@ -3701,7 +3703,7 @@ qlskum_status qlskum_residual_forward_device(qlskum_handle *h, const double *pri
     wait_on(h, h->L.stream, cs);
     fp64::fill_prim(h->L, h->np, make_double4_32a(1.0, 0, 0, 1.0), a->P[0]);
     fp64::permute_in(h->L, h->n, h->d_perm, reinterpret_cast<const double4_32a *>(prim), a->P[0]);
-    fp64::func_delta(h->L, h->dc, a->P[0], a->set64.delta, h->K.cfl);
+    fp64::func_delta(h->L, h->dc, a->P[0], a->cs, a->set64.delta, h->K.cfl);
     adj_stage_forward(h, a->set64, 0);
     fp64::permute_out(h->L, h->n, h->d_perm, a->set64.flux[0], reinterpret_cast<double4_32a *>(flux_res));
     wait_on(h, cs, h->L.stream);
@@ -3722,14 +3724,14 @@ qlskum_status qlskum_residual_vjp_device(qlskum_handle *h, const double *prim, c
     fp64::permute_in(h->L, h->n, h->d_perm, reinterpret_cast<const double4_32a *>(prim), a->P[0]);
     zero(h, a->bF, sizeof(double4_32a) * h->np);
     fp64::permute_in(h->L, h->n, h->d_perm, reinterpret_cast<const double4_32a *>(bar_flux_res), a->bF);
-    fp64::func_delta(h->L, h->dc, a->P[0], a->set64.delta, h->K.cfl);
+    fp64::func_delta(h->L, h->dc, a->P[0], a->cs, a->set64.delta, h->K.cfl);
     adj_stage_forward(h, a->set64, 0);
     const AdjView v = adj_view(h, false);
     zero(h, a->bP, sizeof(double4_32a) * h->np);
     zero(h, a->bdelta, sizeof(double) * h->np);
     adj_stage_reverse(h, a->set64, 0, v);
     zero(h, a->bc, sizeof(double) * h->np);
-    adjl::delta(h->L, v, a->P[0], a->bdelta, h->K.cfl, a->bc, a->bP);
+    adjl::delta(h->L, v, a->P[0], a->bdelta, h->K.cfl, a->cs, a->bc, a->bP);
     fp64::permute_out(h->L, h->n, h->d_perm, a->bP, reinterpret_cast<double4_32a *>(bar_prim));
     wait_on(h, cs, h->L.stream);
     return check_launch(h, "residual_vjp_device");
@@ -3748,7 +3750,7 @@ qlskum_status qlskum_residual_vjp_full(qlskum_handle *h, const double *prim, con
     AdjBuf *a = h->adj;
     if ((st = upload_points(h, prim, a->P[0], 1.0))) return st;
     if ((st = upload_points(h, bar_flux_res, a->bF, 0.0))) return st;
-    fp64::func_delta(h->L, h->dc, a->P[0], a->set64.delta, h->K.cfl);
+    fp64::func_delta(h->L, h->dc, a->P[0], a->cs, a->set64.delta, h->K.cfl);
     adj_stage_forward(h, a->set64, 0);
     adj_zero_geometry(h);
     const AdjView v = adj_view(h, geo);
@@ -3756,7 +3758,7 @@ qlskum_status qlskum_residual_vjp_full(qlskum_handle *h, const double *prim, con
     zero(h, a->bdelta, sizeof(double) * h->np);
     adj_stage_reverse(h, a->set64, 0, v);
     zero(h, a->bc, sizeof(double) * h->np);
-    adjl::delta(h->L, v, a->P[0], a->bdelta, h->K.cfl, a->bc, a->bP);
+    adjl::delta(h->L, v, a->P[0], a->bdelta, h->K.cfl, a->cs, a->bc, a->bP);
     if ((st = check_launch(h, "residual_vjp_full"))) return st;
     if ((st = download_points(h, a->bP, bar_prim))) return st;
     // R(prim) is the flux residual of one stage and its time step: neither

@@ -215,13 +215,16 @@ void update(const Launch &L, const AdjView &a, const CaseConst &K, const double4
 void flux(const Launch &L, const AdjView &a, const double4_32a *q, const double4_32a *dq, const double4_32a *qm,
           const double *delta, const double4_32a *flux, const double *ends, long long ns,
           const double4_32a *bF, double4_32a *bq, double4_32a *bdq, double4_32a *bqm, double *bdelta);
-void inner(const Launch &L, const AdjView &a, const double4_32a *q, const double4_32a *dq_in,
-           const double4_32a *bdq_out, double4_32a *bq, double4_32a *bdq_in);
-void grad(const Launch &L, const AdjView &a, const double4_32a *q, const double4_32a *bdq, const double4_32a *bqm,
-          double4_32a *bq);
+// one inner step from dq_in: adds to bdq_in (zeroed by the caller), sets (first) or adds to bdq0
+void inner(const Launch &L, const AdjView &a, const double4_32a *dq_in, const double4_32a *bdq_out, double4_32a *bdq_in,
+           double4_32a *bdq0, bool first);
+// the gradient's bar is bdq + bdq0 (bdq0 NULL: bdq alone)
+void grad(const Launch &L, const AdjView &a, const double4_32a *q, const double4_32a *bdq, const double4_32a *bdq0,
+          const double4_32a *bqm, double4_32a *bq);
 void qvars(const Launch &L, int n, const double4_32a *P, const double4_32a *bq, double4_32a *bP);
-void delta(const Launch &L, const AdjView &a, const double4_32a *P, const double *bdelta, double cfl, double *bc,
-           double4_32a *bP);
+// cs: scratch [n], the wave speeds of P
+void delta(const Launch &L, const AdjView &a, const double4_32a *P, const double *bdelta, double cfl, double *cs,
+           double *bc, double4_32a *bP);
 void objective(const Launch &L, const AdjView &a, const int *wall_perm, const double4_32a *wall_geo, int n_wall,
                double cp_scale, double theta, int which, double4_32a *bP);
 // bP += dJ/dprim of the stagnation-pressure loss
@@ -291,7 +294,10 @@ void q_derivatives(const Launch &L, const DevCloud &c, const double4_32a *q, dou
 // one inner step from dq_in; dq0: the first-order gradient of q (q_derivatives'), or NULL (formed again from q)
 void q_inner(const Launch &L, const DevCloud &c, const double4_32a *q, const double4_32a *dq0, const double4_32a *dq_in,
              double4_32a *dq_out);
-void func_delta(const Launch &L, const DevCloud &c, const double4_32a *prim, double *delta, double cfl);
+// cs[i] = the wave speed of prim[i]
+void wave_speeds(const Launch &L, int n, const double4_32a *prim, double *cs);
+// the local time step of prim; cs: receives the wave speeds
+void func_delta(const Launch &L, const DevCloud &c, const double4_32a *prim, double *cs, double *delta, double cfl);
 // ends (or NULL): per edge slot of the ns slots, the owner's and the
 // neighbour's end's values of fast64::keep_end, as 12 planes of ns doubles
 // (read back by the flux reverse).
