@@ -1285,7 +1285,7 @@ namespace adjl {
 void update(const Launch &L, const AdjView &a, const CaseConst &K, const double4_32a *Pin, const double4_32a *Pold,
             const double4_32a *Pout, int rk, double4_32a *bP, double4_32a *bPold, double4_32a *bF, double *buinf)
 {
-    adjk::k_update<<<adjk::grid_for(a.c.n, 128), 128, 0, L.stream>>>(a, K, Pin, Pold, Pout, rk, bP, bPold, bF, buinf);
+    adjk::k_update<<<adjk::grid_for(a.c.n, kPointBlock), kPointBlock, 0, L.stream>>>(a, K, Pin, Pold, Pout, rk, bP, bPold, bF, buinf);
 }
 
 void flux(const Launch &L, const AdjView &a, const double4_32a *q, const double4_32a *dq, const double4_32a *qm,
@@ -1328,7 +1328,7 @@ void grad(const Launch &L, const AdjView &a, const double4_32a *q, const double4
 
 void qvars(const Launch &L, int n, const double4_32a *P, const double4_32a *bq, double4_32a *bP)
 {
-    adjk::k_q<<<adjk::grid_for(n, 256), 256, 0, L.stream>>>(n, P, bq, bP);
+    adjk::k_q<<<adjk::grid_for(n, kPointBlock), kPointBlock, 0, L.stream>>>(n, P, bq, bP);
 }
 
 void delta(const Launch &L, const AdjView &a, const double4_32a *P, const double *bdelta, double cfl, double *cs,
@@ -1338,7 +1338,7 @@ void delta(const Launch &L, const AdjView &a, const double4_32a *P, const double
     const int g = adjk::grid_for(4 * (long long)a.c.n, 128);
     if (a.bdist) adjk::k_delta<true><<<g, 128, 0, L.stream>>>(a, cs, bdelta, cfl, bc);
     else adjk::k_delta<false><<<g, 128, 0, L.stream>>>(a, cs, bdelta, cfl, bc);
-    adjk::k_wave<<<adjk::grid_for(a.c.n, 256), 256, 0, L.stream>>>(a.c.n, P, bc, bP);
+    adjk::k_wave<<<adjk::grid_for(a.c.n, kPointBlock), kPointBlock, 0, L.stream>>>(a.c.n, P, bc, bP);
 }
 
 void objective_J(const Launch &L, int n, const double4_32a *P, double gamma, double p0_inf, double4_32a *bP)

@@ -374,13 +374,13 @@ __device__ __forceinline__ void partial8(double v, int i, int n, double *__restr
 
 // state_update_mod.h:92-283 over all points, with the residual's partial sums
 // (prim_next may be prim).
-__global__ void __launch_bounds__(128) k_state_update(DevCloud c, CaseConst K, const double4_32a *prim,
+__global__ void __launch_bounds__(kPointBlock) k_state_update(DevCloud c, CaseConst K, const double4_32a *prim,
                                                       const double4_32a *__restrict__ prim_old,
                                                       const double4_32a *__restrict__ flux_res,
                                                       double4_32a *prim_next, int rk, double *__restrict__ psum,
                                                       double *__restrict__ pmax)
 {
-    const int i = blockIdx.x * 128 + threadIdx.x;
+    const int i = blockIdx.x * kPointBlock + threadIdx.x;
     double r2 = 0.0;
     if (i < c.n) {
         const double2 nn = c.nrm[i];
@@ -701,13 +701,13 @@ void fold_weights(const Launch &L, const DevCloud &c, double2 *e_w64, double2 *e
 
 void q_variables(const Launch &L, const DevCloud &c, const double4_32a *prim, double4_32a *q)
 {
-    k_q_variables<<<grid_for(c.n, 256), 256, 0, L.stream>>>(c.n, prim, q);
+    k_q_variables<<<grid_for(c.n, kPointBlock), kPointBlock, 0, L.stream>>>(c.n, prim, q);
     QLSKUM_LAUNCHED(L);
 }
 
 void derived(const Launch &L, const DevCloud &c, const double4_32a *prim, double4_32a *q, double *cspeed)
 {
-    k_derived<<<grid_for(c.n, 256), 256, 0, L.stream>>>(c.n, prim, q, cspeed);
+    k_derived<<<grid_for(c.n, kPointBlock), kPointBlock, 0, L.stream>>>(c.n, prim, q, cspeed);
     QLSKUM_LAUNCHED(L);
 }
 
@@ -736,7 +736,7 @@ void q_inner(const Launch &L, const DevCloud &c, const double4_32a *q, const dou
 
 void wave_speeds(const Launch &L, int n, const double4_32a *prim, double *cs)
 {
-    k_wave_speeds<<<grid_for(n, 64), 64, 0, L.stream>>>(n, prim, cs);
+    k_wave_speeds<<<grid_for(n, kPointBlock), kPointBlock, 0, L.stream>>>(n, prim, cs);
     QLSKUM_LAUNCHED(L);
 }
 
@@ -761,7 +761,7 @@ void state_update(const Launch &L, const DevCloud &c, const CaseConst &k, const 
                   const double4_32a *prim_old, const double4_32a *flux_res, double4_32a *prim_next, int rk,
                   const Reduce &R)
 {
-    k_state_update<<<grid_for(c.n, 128), 128, 0, L.stream>>>(c, k, prim, prim_old, flux_res, prim_next, rk,
+    k_state_update<<<grid_for(c.n, kPointBlock), kPointBlock, 0, L.stream>>>(c, k, prim, prim_old, flux_res, prim_next, rk,
                                                              R.partial_sum, R.partial_max);
     QLSKUM_LAUNCHED(L);
 }

@@ -23,6 +23,12 @@
 namespace qlskum {
 
 enum : int { kWall = 0, kInterior = 1, kOuter = 2 };
+// Threads per block of the FP64 kernels with one thread per point and no
+// neighbours (state update, q, wave speed, their reverses): the wall and outer
+// points, with the far field's exps, sit together in the point order, so small
+// blocks spread them over the SMs.  Reverse update of 20,480 points 32 us at 128
+// threads, 26 at 32; state update 16.5 and 14.4; q 7.9 (256 threads) and 6.4.
+constexpr int kPointBlock = 32;
 constexpr int kMaxNbhs = 20;                   // QLSKUM_MAX_NBHS
 constexpr int kGaussTab = 6145, kExpTab = 512;
 enum : unsigned { kXpos = 1u, kXneg = 2u, kYpos = 4u, kYneg = 8u };
