@@ -42,6 +42,65 @@ __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_grou
 
 template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
+// ------------------------------------------------------- bulk copies
+// Contiguous global memory -> shared memory by the copy engine of the SM
+// (cp.async.bulk, completion counted on an mbarrier); addresses and sizes are
+// multiples of 16 bytes.
+
+__device__ __forceinline__ void mbar_init(unsigned bar, unsigned count)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
+__device__ __forceinline__ void mbar_expect(unsigned bar, unsigned bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+
+__device__ __forceinline__ bool mbar_try(unsigned bar, unsigned phase)
+{
+    unsigned ok;
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+                 " selp.u32 %0, 1, 0, p;\n}\n"
+                 : "=r"(ok)
+                 : "r"(bar), "r"(phase)
+                 : "memory");
+    return ok != 0;
+}
+
+// Waits for the barrier's phase; false if it has not completed after a second
+// (a bound on the wait, not expected).
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned phase)
+{
+    for (int t = 0; t < 1024; t++)
+        if (mbar_try(bar, phase)) return true;
+    unsigned long long t0, t1;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
+    do {
+        if (mbar_try(bar, phase)) return true;
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t1));
+    } while (t1 - t0 < 1000000000ull);
+    return false;
+}
+
+// Evict-first in L2: data streamed once per launch.
+__device__ __forceinline__ unsigned long long stream_policy()
+{
+    unsigned long long p;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+
+__device__ __forceinline__ void bulk_load(unsigned dst, const void *src, unsigned bytes, unsigned bar,
+                                          unsigned long long policy)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;"
+                 ::"r"(dst), "l"(src), "r"(bytes), "r"(bar), "l"(policy)
+                 : "memory");
+}
+
 // One end of an edge in the mixed form (interior_fluxes_mod.h:50-89 with
 // limiters_mod.h:64-104, q_variables_mod.h:230-253, split_fluxes_mod.h:14-26):
 // the limited reconstruction q~ = q + phi dn, dn = -(delx dqx + dely dqy) / 2

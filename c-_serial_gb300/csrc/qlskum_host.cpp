@@ -627,6 +627,7 @@ qlskum_status check_status(qlskum_handle *h)
     int st = 0;
     CK(h, cudaMemcpyAsync(&st, h->R.status, sizeof(int), cudaMemcpyDeviceToHost, h->L.stream));
     CK(h, cudaStreamSynchronize(h->L.stream));
+    if (st == 2) return fail(h, QLSKUM_ERR_CUDA, "a bulk copy of the edge lists did not complete");
     if (st) return fail(h, QLSKUM_ERR_NONFINITE, "residual became non-finite (NaN/Inf in the state)");
     return QLSKUM_OK;
 }
@@ -1019,6 +1020,7 @@ qlskum_status qlskum_create(const qlskum_cloud *c, const qlskum_params *p, qlsku
     h->R.res_old = A.alloc<double>(1);
     h->R.iter = A.alloc<int>(1);
     h->R.status = A.alloc<int>(1);
+    h->dc.fault = h->R.status;
     h->d_obj = A.alloc<double>(8);
     h->d_obj_partial = A.alloc<double>(4 * (size_t)((std::max(n, sp) + 255) / 256));
     h->d_entropy = A.alloc<double>(h->np);
@@ -1844,6 +1846,7 @@ qlskum_status qlskum_batch_create(const qlskum_cloud *clouds, int n_clouds, cons
     b->pmax = A.alloc<double>(T / 64);
     b->d_iter = A.alloc<int>(1);
     b->d_status = A.alloc<int>(1);
+    b->sc.fault = b->d_status;
     b->res_old = A.alloc<double>(n_cases);
     b->res_new = A.alloc<double>(n_cases);
     b->d_obj = A.alloc<double>(4 * (size_t)n_cases);
@@ -1926,6 +1929,7 @@ qlskum_status qlskum_batch_run(qlskum_batch *b, int iters)
     int status = 0;
     BCK(b, cudaMemcpyAsync(&status, b->d_status, sizeof(int), cudaMemcpyDeviceToHost, b->L.stream));
     BCK(b, cudaStreamSynchronize(b->L.stream));
+    if (status == 2) return bfail(b, QLSKUM_ERR_CUDA, "a bulk copy of the edge lists did not complete");
     if (status) return bfail(b, QLSKUM_ERR_NONFINITE, "a case's residual became non-finite");
     return QLSKUM_OK;
 }
@@ -2543,6 +2547,7 @@ qlskum_status qlskum_partition_create(const qlskum_cloud *c, const qlskum_params
     P->R.res_old = P->A.alloc<double>(1);
     P->R.iter = P->A.alloc<int>(1);
     P->R.status = P->A.alloc<int>(1);
+    for (PartDev *d : P->parts) d->G.dc.fault = P->R.status;
     if (P->A.err != cudaSuccess) {
         part_free(P);
         return fail(nullptr, QLSKUM_ERR_CUDA, fmt("cudaMalloc: %s", cudaGetErrorString(P->A.err)));
@@ -2641,6 +2646,7 @@ qlskum_status qlskum_partition_q_lskum(qlskum_partition *P, int iters)
     if (st) return st;
     int bad = 0;
     PCK(P, cudaMemcpy(&bad, P->R.status, sizeof(int), cudaMemcpyDeviceToHost));
+    if (bad == 2) return pfail(P, QLSKUM_ERR_CUDA, "a bulk copy of the edge lists did not complete");
     if (bad) return pfail(P, QLSKUM_ERR_NONFINITE, "residual became non-finite (NaN/Inf in the state)");
     return QLSKUM_OK;
 }

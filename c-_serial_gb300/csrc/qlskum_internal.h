@@ -94,6 +94,9 @@ struct DevCloud {
     // NULL for a single case, whose constants come with the launch.
     const CaseConst *case_k = nullptr;
     const int *slice_case = nullptr;
+    // set to 2 by a kernel whose bulk copy did not arrive (the status word that
+    // also holds 1 for a non-finite residual)
+    int *fault = nullptr;
 };
 
 // Free-stream constants of one case (parameter_mod.h:4-30).

@@ -1,0 +1,43 @@
+"""The mixed gradient kernel whose edge list comes by bulk copies: the same bits
+at every block size, and the four-lanes form's values."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def run(c, block, lanes, power, inner=2):
+    import qlskum
+    s = qlskum.Solver(c, mach=0.63, aoa=2.0, cfl=0.2, vl_const=50.0, power=power, inner_iterations=inner,
+                      precision=qlskum.MIXED)
+    s.set_launch_config(10, block, 0, lanes)
+    rng = np.random.default_rng(2)
+    s.set_prim(s.prim * (1.0 + 1e-2 * rng.standard_normal((c.n, 4))))
+    s.q_lskum(1)
+    return s.prim, s.field(qlskum.FIELD_DQ), s.field(qlskum.FIELD_QM)
+
+
+# few slices, a remainder of a slice, more slices than resident warps
+# (152 x 24); lists of up to 20 edges (several chunks)
+@pytest.mark.parametrize("wall, layers", [(40, 12), (49, 21), (397, 331)])
+@pytest.mark.parametrize("power", [0.0, -2.0])
+def test_block_sizes_and_lanes(wall, layers, power):
+    """The gradients are sums of at most 20 products in FP32: split over four
+    lanes they move by at most 20 ulps of the terms' sum, whose weights sum to at
+    most 2.5 / min_dist (x and y half range: twice); two inner steps repeat that.
+    The extrema are the same."""
+    from conftest import small_cloud
+    from qlskum import cloudgen
+    c = small_cloud(wall, layers) if wall < 60 else cloudgen.make_cloud(n_wall=wall, n_layers=layers, seed=3,
+                                                                       te_spread=0.064)
+    ref = run(c, 128, 1, power)
+    for block in (64, 256, 512):
+        for a, b in zip(ref, run(c, block, 1, power)):
+            assert np.array_equal(a, b)
+    p4, dq4, qm4 = run(c, 128, 4, power)
+    scale = 2 * 2.5 * np.abs(ref[2]).max() / c.min_dist[:, None, None]
+    assert (np.abs(dq4 - ref[1]) <= 3 * 20 * 2.0 ** -24 * scale).all()
+    assert np.allclose(qm4, ref[2], rtol=0, atol=1e-5 * np.abs(ref[2]).max())
+    assert np.allclose(p4, ref[0], rtol=1e-5, atol=1e-6)
+
+
