@@ -440,6 +440,7 @@ __global__ void __launch_bounds__(RB) k_reduce_residual(int nblocks, const doubl
                                                        int *status, int latch)
 {
     __shared__ double ss[RB], sm[RB];
+    begin_dependent();
     double v[4] = {0.0, 0.0, 0.0, 0.0}, mm[4] = {0.0, 0.0, 0.0, 0.0};
     int b = threadIdx.x;
     for (; b + 3 * RB < nblocks; b += 4 * RB) {
@@ -781,8 +782,8 @@ void flux_update(const Launch &L, const DevCloud &c, const CaseConst &k, const d
 
 void reduce_residual(const Launch &L, const Reduce &R, int n, int it)
 {
-    k_reduce_residual<<<1, RB, 0, L.stream>>>(R.blocks, R.partial_sum, R.partial_max, n, it, R.hist, R.capacity,
-                                              R.res_old, R.iter, R.status, R.latch);
+    launch_after(L, k_reduce_residual, 1, RB, 0, R.blocks, R.partial_sum, R.partial_max, n, it, R.hist, R.capacity,
+                 R.res_old, R.iter, R.status, R.latch);
     QLSKUM_LAUNCHED(L);
 }
 

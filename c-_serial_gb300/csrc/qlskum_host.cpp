@@ -966,6 +966,7 @@ qlskum_status qlskum_create(const qlskum_cloud *c, const qlskum_params *p, qlsku
     }
     h->L.block = p->block_size ? p->block_size : 128;
     h->L.launches = &h->launches;
+    h->L.chain = p->precision == QLSKUM_MIXED;
     DeviceArena &A = h->arena;
     {
         st = build_geometry(c, p, sp, true, p->precision == QLSKUM_MIXED, A, h->L.stream, G);
@@ -1694,6 +1695,7 @@ qlskum_status qlskum_batch_create(const qlskum_cloud *clouds, int n_clouds, cons
         return bfail(nullptr, QLSKUM_ERR_CUDA, fmt("cudaStreamCreate: %s", cudaGetErrorString(ce)));
     }
     b->L.launches = &b->launches;
+    b->L.chain = true;
     DeviceArena &A = b->arena;
     auto cleanup = [&](qlskum_status st, const std::string &m) {
         A.release();

@@ -172,12 +172,13 @@ __device__ __forceinline__ void grad_point(const DevCloud &c, int i, const float
                                            int sub = 0)
 {
     float qi[4], qmax[4], qmin[4], dx[4] = {0, 0, 0, 0}, dy[4] = {0, 0, 0, 0};
+    const int nb = c.nbhs[i];
+    const long long base = c.slice_base[i >> 5] + (i & 31);
+    begin_dependent();
     ld4(q[i], qi);
 #pragma unroll
     for (int r = 0; r < 4; r++) { qmax[r] = qi[r]; qmin[r] = qi[r]; }
     float min_dt = 1.0f;
-    const int nb = c.nbhs[i];
-    const long long base = c.slice_base[i >> 5] + (i & 31);
     // two edges per trip: their index loads and gathers are issued together
 #pragma unroll 2
     for (int j = sub; j < nb; j += L) {
@@ -248,6 +249,7 @@ __device__ __forceinline__ void inner_point(const DevCloud &c, int i, const floa
     float dxi[4], dyi[4], ax[4] = {0, 0, 0, 0}, ay[4] = {0, 0, 0, 0};
     const int nb = c.nbhs[i];
     const long long base = c.slice_base[i >> 5] + (i & 31);
+    begin_dependent();
 #pragma unroll 2
     for (int j = sub; j < nb; j += L) {
         const long long e = base + 32LL * j;
@@ -339,6 +341,7 @@ __global__ void __launch_bounds__(B) k_q_inner_st(DevCloud c, const float4 *__re
     const int nb = c.nbhs[i];
     const long long base = c.slice_base[i >> 5] + (i & 31);
     stage_edges<B, UW>(c, base, nb, t, snbr, sgeo);
+    begin_dependent();
     float dxi[4], dyi[4], ax[4] = {0, 0, 0, 0}, ay[4] = {0, 0, 0, 0};
     ld4(dq_in[2 * i], dxi);
     ld4(dq_in[2 * i + 1], dyi);
@@ -398,6 +401,7 @@ __global__ void __launch_bounds__(B) k_q_derivatives_st(DevCloud c, const float4
         cp_async8(static_cast<float2 *>(sgeo) + j * B + t, c.e_gw32 + e);
     }
     cp_commit();
+    begin_dependent();
     float qi[4], qmax[4], qmin[4], dx[4] = {0, 0, 0, 0}, dy[4] = {0, 0, 0, 0};
     ld4(q[i], qi);
 #pragma unroll
@@ -711,6 +715,9 @@ __device__ __forceinline__ float flux_point(const DevCloud &c, const CaseConst &
     const int f = c.flag[i];
     const double2 nn = c.nrm[i];
     const float nx = d2f(nn.x), ny = d2f(nn.y);
+    const int nb = c.nbhs[i];
+    const long long base = c.slice_base[i >> 5] + (i & 31);
+    begin_dependent();
     float qi[4], dxi[4], dyi[4], mxi[4], mni[4];
     ld4(q[i], qi);
     ld4(dq[2 * i], dxi);
@@ -725,8 +732,6 @@ __device__ __forceinline__ float flux_point(const DevCloud &c, const CaseConst &
     }
     const float e2i = c.eps2_32[i];
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    const int nb = c.nbhs[i];
-    const long long base = c.slice_base[i >> 5] + (i & 31);
     for (int j = sub; j < nb; j += L) {
         const long long e = base + 32LL * j;
         const int k = c.e_nbr[e];
@@ -786,9 +791,13 @@ __device__ __forceinline__ float flux_point_st(const DevCloud &c, const CaseCons
     float2 wn = make_float2(0.f, 0.f);
     unsigned dn = 0;
     if (nb > 0) {
-        issue(0, c.e_nbr[base]);
+        const int k0 = c.e_nbr[base];
         edge_geo<UW>(c, base, gn, wn);
         dn = c.e_dir[base];
+        begin_dependent();
+        issue(0, k0);
+    } else {
+        begin_dependent();
     }
     cp_commit();
     if (nb > 1) kn = c.e_nbr[base + 32];
@@ -874,12 +883,15 @@ __device__ __forceinline__ float flux_point_rp(const DevCloud &c, const CaseCons
     float2 wn = make_float2(0.f, 0.f);
     unsigned dn = 0;
     int kn = 0;
+    int k0 = 0;
     if (nb > 0) {
-        load_nbr(c, c.e_nbr[base], q, dq, qm, nd);
+        k0 = c.e_nbr[base];
         edge_geo<UW>(c, base, gn, wn);
         dn = c.e_dir[base];
     }
     if (nb > 1) kn = c.e_nbr[base + 32];
+    begin_dependent();
+    if (nb > 0) load_nbr(c, k0, q, dq, qm, nd);
     NbrData me;
     load_nbr(c, i, q, dq, qm, me);
     float qi[4], dxi[4], dyi[4], mxi[4], mni[4];
@@ -956,11 +968,12 @@ __device__ __forceinline__ float flux_point_rps(const DevCloud &c, const CaseCon
     int kc = 0;
     if (nb > 0) {
         kc = c.e_nbr[base];
-        if (PF) load_nbr(c, kc, q, dq, qm, nd);
         edge_geo<UW>(c, base, gn, wn);
         dn = c.e_dir[base];
     }
     if (nb > 1) kn = c.e_nbr[base + 32];
+    begin_dependent();
+    if (PF && nb > 0) load_nbr(c, kc, q, dq, qm, nd);
     {
         NbrData me;
         load_nbr(c, i, q, dq, qm, me);
@@ -1168,6 +1181,7 @@ __global__ void k_q_derivatives_ring(DevCloud c, const float4 *__restrict__ q, f
     R.start(c, first, stride, pol);
     const int nslices = (c.n + 31) >> 5;
     int nb = 32 * first + lane < c.n ? c.nbhs[32 * first + lane] : 0;
+    begin_dependent();
     for (int s = first; s < nslices; s += stride) {
         const int i = 32 * s + lane;
         const bool has = i < c.n;
@@ -1336,6 +1350,7 @@ __global__ void kb_reduce(const BatchCase *__restrict__ cases, int ncases, int t
                           double *hist, int capacity, int *status)
 {
     __shared__ double ss[256];
+    begin_dependent();
     const int c = blockIdx.x;
     if (c >= ncases) return;
     const BatchCase &C = cases[c];
@@ -1438,29 +1453,27 @@ void q_derivatives(const Launch &L, const DevCloud &c, const float4 *q, float4 *
     if (L.staged > 0) {
         QLSKUM_STAGED_SWITCH(L.staged,
             if (c.unit_w)
-                k_q_derivatives_st<B_, D_, true><<<grid_for(c.n, B_), B_, staged_bytes(B_, D_, 2, c.max_nb, true),
-                                                   L.stream>>>(c, q, dq, qm, cspeed, delta, cfl);
+                launch_after(L, k_q_derivatives_st<B_, D_, true>, grid_for(c.n, B_), B_, staged_bytes(B_, D_, 2, c.max_nb, true), c, q, dq, qm, cspeed, delta, cfl);
             else
-                k_q_derivatives_st<B_, D_, false><<<grid_for(c.n, B_), B_, staged_bytes(B_, D_, 2, c.max_nb, true),
-                                                    L.stream>>>(c, q, dq, qm, cspeed, delta, cfl))
+                launch_after(L, k_q_derivatives_st<B_, D_, false>, grid_for(c.n, B_), B_, staged_bytes(B_, D_, 2, c.max_nb, true), c, q, dq, qm, cspeed, delta, cfl))
     } else if (L.lanes == 1) {
         const int g = ring_grid(c.n, L.block, 24);
         if (delta) {
             const size_t sm = ring_bytes(L.block, 16);
             allow_smem(k_q_derivatives_ring<true>, sm);
-            k_q_derivatives_ring<true><<<g, L.block, sm, L.stream>>>(c, q, dq, qm, cspeed, delta, cfl);
+            launch_after(L, k_q_derivatives_ring<true>, g, L.block, sm, c, q, dq, qm, cspeed, delta, cfl);
         } else {
             const size_t sm = ring_bytes(L.block, 12);
             allow_smem(k_q_derivatives_ring<false>, sm);
-            k_q_derivatives_ring<false><<<g, L.block, sm, L.stream>>>(c, q, dq, qm, nullptr, nullptr, cfl);
+            launch_after(L, k_q_derivatives_ring<false>, g, L.block, sm, c, q, dq, qm, nullptr, nullptr, cfl);
         }
     } else {
 #define QLSKUM_GRAD(LN)                                                                                         \
     if (delta)                                                                                                  \
-        k_q_derivatives<true, LN><<<grid_for(c.n * LN, L.block), L.block, 0, L.stream>>>(c, q, dq, qm, cspeed,  \
+        launch_after(L, k_q_derivatives<true, LN>, grid_for(c.n * LN, L.block), L.block, 0, c, q, dq, qm, cspeed,  \
                                                                                         delta, cfl);           \
     else                                                                                                        \
-        k_q_derivatives<false, LN><<<grid_for(c.n * LN, L.block), L.block, 0, L.stream>>>(c, q, dq, qm, cspeed, \
+        launch_after(L, k_q_derivatives<false, LN>, grid_for(c.n * LN, L.block), L.block, 0, c, q, dq, qm, cspeed, \
                                                                                          delta, cfl)
         if (L.lanes == 4) { QLSKUM_GRAD(4); }
         else { QLSKUM_GRAD(2); }
@@ -1474,17 +1487,15 @@ void q_inner(const Launch &L, const DevCloud &c, const float4 *dq0, const float4
     if (L.staged > 0) {
         QLSKUM_STAGED_SWITCH(L.staged,
             if (c.unit_w)
-                k_q_inner_st<B_, D_, true><<<grid_for(c.n, B_), B_, staged_bytes(B_, D_, 2, c.max_nb, true),
-                                             L.stream>>>(c, dq0, dq_in, dq_out);
+                launch_after(L, k_q_inner_st<B_, D_, true>, grid_for(c.n, B_), B_, staged_bytes(B_, D_, 2, c.max_nb, true), c, dq0, dq_in, dq_out);
             else
-                k_q_inner_st<B_, D_, false><<<grid_for(c.n, B_), B_, staged_bytes(B_, D_, 2, c.max_nb, false),
-                                              L.stream>>>(c, dq0, dq_in, dq_out))
+                launch_after(L, k_q_inner_st<B_, D_, false>, grid_for(c.n, B_), B_, staged_bytes(B_, D_, 2, c.max_nb, false), c, dq0, dq_in, dq_out))
     } else {
 #define QLSKUM_INNER(LN)                                                                                        \
     if (c.unit_w)                                                                                               \
-        k_q_inner<true, LN><<<grid_for(c.n * LN, L.block), L.block, 0, L.stream>>>(c, dq0, dq_in, dq_out);      \
+        launch_after(L, k_q_inner<true, LN>, grid_for(c.n * LN, L.block), L.block, 0, c, dq0, dq_in, dq_out);      \
     else                                                                                                        \
-        k_q_inner<false, LN><<<grid_for(c.n * LN, L.block), L.block, 0, L.stream>>>(c, dq0, dq_in, dq_out)
+        launch_after(L, k_q_inner<false, LN>, grid_for(c.n * LN, L.block), L.block, 0, c, dq0, dq_in, dq_out)
         if (L.lanes == 4) { QLSKUM_INNER(4); }
         else if (L.lanes == 2) { QLSKUM_INNER(2); }
         else { QLSKUM_INNER(1); }
@@ -1518,45 +1529,45 @@ void flux_update(const Launch &L, const DevCloud &c, const CaseConst &k, const f
 {
 #define QLSKUM_FLUX_L(B, MB, LN)                                                                            \
     if (c.unit_w)                                                                                           \
-        k_flux_update<B, MB, true, LN><<<grid_for(c.n * LN, B), B, 0, L.stream>>>(                          \
+        launch_after(L, k_flux_update<B, MB, true, LN>, grid_for(c.n * LN, B), B, 0,                           \
             c, k, q, dq, qm, delta, prim, prim_old, prim_next, q_next, cspeed_next, rk, R.partial_sum,      \
             R.partial_max, acc_out);                                                                        \
     else                                                                                                    \
-        k_flux_update<B, MB, false, LN><<<grid_for(c.n * LN, B), B, 0, L.stream>>>(                         \
+        launch_after(L, k_flux_update<B, MB, false, LN>, grid_for(c.n * LN, B), B, 0,                          \
             c, k, q, dq, qm, delta, prim, prim_old, prim_next, q_next, cspeed_next, rk, R.partial_sum,      \
             R.partial_max, acc_out)
 #define QLSKUM_FLUX(B, MB) QLSKUM_FLUX_L(B, MB, 1)
 #define QLSKUM_FLUX_ST(B, MB)                                                                               \
     if (c.unit_w)                                                                                           \
-        k_flux_update_st<B, MB, true><<<grid_for(c.n, B), B, 0, L.stream>>>(c, k, q, dq, qm, delta, prim,   \
+        launch_after(L, k_flux_update_st<B, MB, true>, grid_for(c.n, B), B, 0, c, k, q, dq, qm, delta, prim,   \
                                                                          prim_old, prim_next, q_next,      \
                                                                          cspeed_next, rk, R.partial_sum,   \
                                                                          R.partial_max, acc_out);          \
     else                                                                                                    \
-        k_flux_update_st<B, MB, false><<<grid_for(c.n, B), B, 0, L.stream>>>(c, k, q, dq, qm, delta, prim,  \
+        launch_after(L, k_flux_update_st<B, MB, false>, grid_for(c.n, B), B, 0, c, k, q, dq, qm, delta, prim,  \
                                                                           prim_old, prim_next, q_next,     \
                                                                           cspeed_next, rk, R.partial_sum,  \
                                                                           R.partial_max, acc_out)
 #define QLSKUM_FLUX_RP(B, MB)                                                                               \
     if (c.unit_w)                                                                                           \
-        k_flux_update_rp<B, MB, true><<<grid_for(c.n, B), B, 0, L.stream>>>(c, k, q, dq, qm, delta, prim,   \
+        launch_after(L, k_flux_update_rp<B, MB, true>, grid_for(c.n, B), B, 0, c, k, q, dq, qm, delta, prim,   \
                                                                          prim_old, prim_next, q_next,      \
                                                                          cspeed_next, rk, R.partial_sum,   \
                                                                          R.partial_max, acc_out);          \
     else                                                                                                    \
-        k_flux_update_rp<B, MB, false><<<grid_for(c.n, B), B, 0, L.stream>>>(c, k, q, dq, qm, delta, prim,  \
+        launch_after(L, k_flux_update_rp<B, MB, false>, grid_for(c.n, B), B, 0, c, k, q, dq, qm, delta, prim,  \
                                                                           prim_old, prim_next, q_next,     \
                                                                           cspeed_next, rk, R.partial_sum,  \
                                                                           R.partial_max, acc_out)
 #define QLSKUM_FLUX_RPS(B, MB, PF)                                                                          \
     if (c.unit_w)                                                                                           \
-        k_flux_update_rps<B, MB, true, PF><<<grid_for(c.n, B), B, 0, L.stream>>>(c, k, q, dq, qm, delta,     \
+        launch_after(L, k_flux_update_rps<B, MB, true, PF>, grid_for(c.n, B), B, 0, c, k, q, dq, qm, delta,     \
                                                                               prim, prim_old, prim_next,   \
                                                                               q_next, cspeed_next, rk,     \
                                                                               R.partial_sum, R.partial_max, \
                                                                               acc_out);                    \
     else                                                                                                    \
-        k_flux_update_rps<B, MB, false, PF><<<grid_for(c.n, B), B, 0, L.stream>>>(c, k, q, dq, qm, delta,    \
+        launch_after(L, k_flux_update_rps<B, MB, false, PF>, grid_for(c.n, B), B, 0, c, k, q, dq, qm, delta,    \
                                                                                prim, prim_old, prim_next,  \
                                                                                q_next, cspeed_next, rk,    \
                                                                                R.partial_sum,              \
@@ -1609,8 +1620,8 @@ void batch_fill_normals(const Launch &L, double2 *nrm, long long n)
 void batch_reduce(const Launch &L, const BatchView &B, int points, const double *psum, const double *pmax,
                   int *iter, double *res_old, double *res_new, double *hist, int capacity, int *status)
 {
-    kb_reduce<<<B.ncases, 256, 0, L.stream>>>(B.cases, B.ncases, block_index(points), psum, pmax, iter, res_old,
-                                              res_new, hist, capacity, status);
+    launch_after(L, kb_reduce, B.ncases, 256, 0, B.cases, B.ncases, block_index(points), psum, pmax, iter, res_old,
+                 res_new, hist, capacity, status);
     kb_count<<<1, 1, 0, L.stream>>>(iter);
     if (L.launches) *L.launches += 2;
 }
