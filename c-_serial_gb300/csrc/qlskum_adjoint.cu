@@ -297,7 +297,9 @@ __global__ void __launch_bounds__(kRevThreads, GEO ? 1 : 4) k_flux(AdjView a, co
             const long long e = base + 32LL * j;
             const double4_32a g = c.e_geo[e];
             const double hx = -0.5 * g.x, hy = -0.5 * g.y;
-            const double2 w = c.e_w64[e];
+            double2 w = c.e_w64[e];
+            w.x += w.x;
+            w.y += w.y;
             const unsigned dir = c.e_dir[e];
             double w2x = 0.0, w2y = 0.0;
             if ((dir & (kXpos | kXneg)) == (kXpos | kXneg)) w2x = fast64::flux_weight(c, i, f, 1, c.e_sn[e]);

@@ -13,8 +13,8 @@
 // as the CUDA functions it replaces; arguments outside the ranges below
 // (which a physical state does not reach, and every Inf / NaN) take those.
 //
-// FP64 instructions per call: gauss_erf 10 (exp and erf: about 50), exp32 6
-// (about 16), rsqrt64 5, ratio64 4.
+// FP64 instructions per call: gauss_erf 10 (exp and erf: about 50), exp32 5
+// (about 16), rsqrt_rcp 7 for both, ratio64 3.
 #pragma once
 #include "qlskum_math.cuh"
 
@@ -40,28 +40,47 @@ __device__ __forceinline__ bool seed_ok(float s) { return fabsf(s) > 1e-37f && f
 static __device__ __noinline__ double div_slow(double a, double b) { return a / b; }
 static __device__ __noinline__ double rsqrt_slow(double x) { return rsqrt(x); }
 static __device__ __noinline__ double exp32_slow(double x) { return 32.0 * exp(x); }
-static __device__ __noinline__ double2 gauss_erf_slow(double s) { return make_double2(0.5641895835477563 * exp(-s * s), erf(s)); }
+static __device__ __noinline__ double2 gauss_erf_slow(double s) { return make_double2(1.1283791670955126 * exp(-s * s), erf(s)); }
 
-// num / den: the FP32 quotient corrected twice by its FP64 remainder.
-__device__ __forceinline__ double ratio64(double num, double den)
+// The 29 low mantissa bits of x that d2f(x) cuts off, as a float (x normal
+// and within FP32's range; below about 1e-30 it may flush to zero).
+__device__ __forceinline__ float d2f_rest(double x)
 {
-    const float r = __fdividef(1.0f, d2f(den));
-    const float q = d2f(num) * r;
-    if (!seed_ok(r) || !(fabsf(q) < 1e37f)) return div_slow(num, den);
-    const double rd = f2d(r);
-    double v = f2d(q);
-    v = fma(fma(-den, v, num), rd, v);
-    return fma(fma(-den, v, num), rd, v);
+    const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x) & 0x1fffffffu;
+    // 2^(e - 52) = the float of exponent e, times 2^-52
+    const float ulp = __uint_as_float((((h >> 20) & 0x7ffu) - 896u) << 23) * 2.220446049250313e-16f;
+    return copysignf((float)l, __uint_as_float(h)) * ulp;
 }
 
-// 1 / sqrt(x): FP32 seed y, then y (1 + e/2 + 3 e^2 / 8), e = 1 - x y^2 (the next term is 2^-64).
-__device__ __forceinline__ double rsqrt64(double x)
+// num / den for finite num, den > 0: the quotient to 2^-44 from FP32 (hi and
+// rest of both), corrected once by its FP64 remainder.
+__device__ __forceinline__ double ratio64(double num, double den)
+{
+    const float dh = d2f(den), nh = d2f(num);
+    const float r = __fdividef(1.0f, dh);
+    const float q = nh * r;
+    if (!seed_ok(r) || !(fabsf(q) < 1e37f)) return div_slow(num, den);
+    const float res = fmaf(-dh, q, nh) + fmaf(-d2f_rest(den), q, d2f_rest(num));
+    const double v = f2d(q) + f2d(res * r);
+    return fma(fma(-den, v, num), f2d(r), v);
+}
+
+// r = 1 / sqrt(x) and h = 1 / x from the FP32 seed y of r, whose square is
+// exact in FP64: with e = 1 - x y^2, r = y (1 + e/2 + 3 e^2 / 8) and
+// h = y^2 (1 + e + e^2), the next terms below 2^-60.
+__device__ __forceinline__ void rsqrt_rcp(double x, double &r, double &h)
 {
     const float s = rsqrtf(d2f(x));
-    if (!seed_ok(s)) return rsqrt_slow(x);
+    if (!seed_ok(s)) {
+        r = rsqrt_slow(x);
+        h = div_slow(1.0, x);
+        return;
+    }
     const double y = f2d(s);
-    const double e = fma(-(x * y), y, 1.0);
-    return fma(y * e, fma(0.375, e, 0.5), y);
+    const double y2 = y * y;
+    const double e = fma(-x, y2, 1.0);
+    r = fma(__dmul_rn(y, e), fma(0.375, e, 0.5), y);
+    h = fma(y2, fma(e, e, e), y2);
 }
 
 // 32 exp(x) from tab[i] = 32 2^(i/512): x = k ln2/512 + r, |r| <= 2^-10.5,
@@ -72,18 +91,18 @@ __device__ __forceinline__ double exp32(double x, const double *__restrict__ tab
     const float kf = rintf(d2f(x) * 738.65986f);
     const double kd = f2d(kf);
     const int k = (int)kf;
-    double r = fma(-kd, 0.0013538030870311431, x);
-    r = fma(-kd, 4.529388308293554e-20, r);
+    const double r = fma(-kd, 0.0013538030870311431, x);
     const float rf = d2f(r);
     const double h = 0.5 + f2d(rf * fmaf(rf, 0.041666667f, 0.16666667f));
-    const double p = r * fma(r, h, 1.0);
+    // the reduction's low part, below 2^-50, added to exp(r) - 1
+    const double p = fma(r, fma(r, h, 1.0), f2d(kf * -4.5293883e-20f));
     const double t = __ldg(tab + (k & 511));
     const double ts = __hiloint2double(__double2hiint(t) + ((k >> 9) << 20), __double2loint(t));
     return fma(ts, p, ts);
 }
 
-// e = exp(-s^2) / sqrt(pi) and E = erf(s) together, from
-// tab[j] = {exp(-x^2) / sqrt(pi), erf(x)} at the nearest x = j / 1024 to |s|,
+// e = 2 exp(-s^2) / sqrt(pi) and E = erf(s) together, from
+// tab[j] = {2 exp(-x^2) / sqrt(pi), erf(x)} at the nearest x = j / 1024 to |s|,
 // d = |s| - x (exact, |d| <= 2^-11):
 //   exp(-s^2) = exp(-x^2) exp(-u), u = d (2 x + d), by its series, u^3 on in FP32;
 //   erf(s) = erf(x) + 2/sqrt(pi) d [(f0 + f1) / 2 + d (f0' - f1') / 12],
@@ -109,10 +128,10 @@ __device__ __forceinline__ void gauss_erf(double s, const double2 *__restrict__ 
     const double h = 0.5 - f2d(uf * fmaf(uf, fmaf(uf, 0.0083333333f, -0.041666667f), 0.16666667f));
     const double p = u * fma(u, h, -1.0);
     e = fma(t.x, p, t.x);
-    // 2 d/6 (s e - x e0)
+    // d/6 (s e - x e0)
     const float pf = d2f(p);
-    const float w = 0.33333334f * df * d2f(t.x) * fmaf(df, 1.0f + pf, xf * pf);
-    const double z = (t.x + e) + f2d(w);
+    const float w = 0.16666667f * df * d2f(t.x) * fmaf(df, 1.0f + pf, xf * pf);
+    const double z = fma(0.5, t.x + e, f2d(w));
     E = flip(fma(d, z, t.y), (unsigned)__double2hiint(s) & 0x80000000u);
 }
 
@@ -136,14 +155,12 @@ __device__ __forceinline__ double limited(double q, double dn, double dp, double
 // moments (split_fluxes_mod.h:14-26) from q~ turned into the owner's (t, n)
 // frame (interior points' frame is (x, y)).  With b = -2 q~4 = 4 beta,
 // r = 1 / sqrt(b) and h = 1 / b: p / rho = 2 h, u = 2 h q~, S = u sqrt(beta) = r q~,
-// beta |u|^2 = S1^2 + S2^2, rho = exp(q~1 + S1^2 + S2^2) 32 h^2 r, and
-// 1 / (2 sqrt(pi beta)) = r / sqrt(pi).  h is r^2 corrected by its remainder:
-// rho takes it to the power 2.5, and with it the residual's error against a
-// 128-bit run is 0.85-1 times the one of reciprocals and a square root taken
-// one by one (without it 1.2 times).
+// beta |u|^2 = S1^2 + S2^2, rho = exp(q~1 + S1^2 + S2^2) 32 h^2 r, and the
+// moments B = exp(-S^2) / (2 sqrt(pi beta)) = r e / 2.  h has its own expansion
+// (r^2 would carry r's rounding twice, and rho takes it to the power 2.5).
 struct End {
-    Kin<double> k;
-    double r, e1, e2;  // kept for the reverse: r, exp(-S1^2) and exp(-S2^2) over sqrt(pi)
+    double rho, ut, un, pbr, usq, E1, E2;
+    double r, e1, e2;  // e = 2 exp(-S^2) / sqrt(pi)
 };
 
 __device__ __forceinline__ void end(const DevCloud &c, int f, double nx, double ny, const double t[4], End &s)
@@ -153,49 +170,43 @@ __device__ __forceinline__ void end(const DevCloud &c, int f, double nx, double 
         qs = fma(t[1], ny, -__dmul_rn(t[2], nx));
         qn = fma(t[1], nx, __dmul_rn(t[2], ny));
     }
-    const double b = -2.0 * t[3];
-    const double r = rsqrt64(b);
-    double h = r * r;
-    h = fma(h, fma(-b, h, 1.0), h);
-    const double S1 = qs * r, S2 = qn * r;
-    s.k.pbr = h + h;
-    s.k.ut = qs * s.k.pbr;
-    s.k.un = qn * s.k.pbr;
-    s.k.usq = fma(s.k.ut, s.k.ut, __dmul_rn(s.k.un, s.k.un));
-    s.k.rho = exp32(fma(S1, S1, fma(S2, S2, t[0])), c.exp_tab) * (h * h * r);
-    gauss_erf(S1, c.gauss_tab, s.e1, s.k.E1);
-    gauss_erf(S2, c.gauss_tab, s.e2, s.k.E2);
-    s.k.B1 = r * s.e1;
-    s.k.B2 = r * s.e2;
-    s.r = r;
+    double h;
+    rsqrt_rcp(-2.0 * t[3], s.r, h);
+    const double S1 = qs * s.r, S2 = qn * s.r;
+    s.pbr = h + h;
+    s.ut = qs * s.pbr;
+    s.un = qn * s.pbr;
+    s.usq = fma(s.ut, s.ut, __dmul_rn(s.un, s.un));
+    s.rho = exp32(fma(S1, S1, fma(S2, S2, t[0])), c.exp_tab) * (h * h * s.r);
+    gauss_erf(S1, c.gauss_tab, s.e1, s.E1);
+    gauss_erf(S2, c.gauss_tab, s.e2, s.E2);
 }
 
 // What the reverse reads back instead of evaluating it again, as planes of ns
 // doubles: rho, r, exp(-S1^2) and exp(-S2^2) over sqrt(pi), erf(S1), erf(S2).
 __device__ __forceinline__ void keep_end(double *__restrict__ o, long long ns, const End &s)
 {
-    o[0] = s.k.rho;
+    o[0] = s.rho;
     o[ns] = s.r;
-    o[2 * ns] = s.e1;
-    o[3 * ns] = s.e2;
-    o[4 * ns] = s.k.E1;
-    o[5 * ns] = s.k.E2;
+    o[2 * ns] = 0.5 * s.e1;
+    o[3 * ns] = 0.5 * s.e2;
+    o[4 * ns] = s.E1;
+    o[5 * ns] = s.E2;
 }
 
-// Adds one end's weighted split-flux pair wx Gx(s1) + wy Gy(s2) to v.  With
-// A = (1 + s E) / 2, al = wx rho A1, ga = wy rho A2 and
-// be = wx rho s1 B1 + wy rho s2 B2, the pair (split_fluxes_mod.h:14-84 and
-// :86-164) is
+// Adds one end's weighted split-flux pair 2 (wx Gx(s1) + wy Gy(s2)) to v (wx,
+// wy half the weights).  With al = wx rho (1 + s1 E1), ga = wy rho (1 + s2 E2)
+// and be = 2 (wx rho s1 B1 + wy rho s2 B2), the pair (split_fluxes_mod.h:14-84
+// and :86-164) is
 //   v0 = al ut + ga un + be,  v1 = ut v0 + al p/rho,  v2 = un v0 + ga p/rho,
 //   v3 = (usq v0 + p/rho (7 v0 - be)) / 2;  twice v3 is added.
 // sx, sy: the sign bits of s1, s2 (0 for +1).  Every product is in an explicit
 // fma or alone, here and below, so that no kernel contracts it differently.
-__device__ __forceinline__ void split_pair(const Kin<double> &k, unsigned sx, unsigned sy, double wx, double wy,
-                                           double v[4])
+__device__ __forceinline__ void split_pair(const End &k, unsigned sx, unsigned sy, double wx, double wy, double v[4])
 {
     const double wr = wx * k.rho, yr = wy * k.rho;
-    const double al = wr * fma(0.5, flip(k.E1, sx), 0.5), ga = yr * fma(0.5, flip(k.E2, sy), 0.5);
-    const double be = fma(flip(wr, sx), k.B1, __dmul_rn(flip(yr, sy), k.B2));
+    const double al = fma(wr, flip(k.E1, sx), wr), ga = fma(yr, flip(k.E2, sy), yr);
+    const double be = k.r * fma(flip(wr, sx), k.e1, __dmul_rn(flip(yr, sy), k.e2));
     const double v0 = fma(al, k.ut, fma(ga, k.un, be));
     v[0] += v0;
     v[1] = fma(k.ut, v0, fma(al, k.pbr, v[1]));
@@ -203,16 +214,17 @@ __device__ __forceinline__ void split_pair(const Kin<double> &k, unsigned sx, un
     v[3] = fma(k.pbr, fma(7.0, v0, -be), fma(k.usq, v0, v[3]));
 }
 
-// Adds w times a boundary end's quadrant flux (quadrant_fluxes_mod.h:6-211),
+// Adds 2 w times a boundary end's quadrant flux (quadrant_fluxes_mod.h:6-211),
 // the t half range of sign bit sx times the n half range of sign bit sn:
 //   f = ut A1 + s1 B1,  m = un A2 + s2 B2,
 //   G0 = rho A2 f,  G1 = rho A2 (ut f + p/rho A1),  G2 = rho f m,
 //   G3 = rho (A2 (usq f + p/rho (7 f - s1 B1)) + s2 un B2 f) / 2; twice G3 is added.
-__device__ __forceinline__ void quad_x(const Kin<double> &k, unsigned sx, unsigned sn, double w, double v[4])
+__device__ __forceinline__ void quad_x(const End &k, unsigned sx, unsigned sn, double w, double v[4])
 {
     const double A1 = fma(0.5, flip(k.E1, sx), 0.5), A2 = fma(0.5, flip(k.E2, sn), 0.5);
-    const double B1 = flip(k.B1, sx), B2 = flip(k.B2, sn);
-    const double wr = w * k.rho, wa = wr * A2;
+    const double hr = 0.5 * k.r;
+    const double B1 = hr * flip(k.e1, sx), B2 = hr * flip(k.e2, sn);
+    const double wr = 2.0 * w * k.rho, wa = wr * A2;
     const double f = fma(k.ut, A1, B1);
     const double wf = wr * f;
     v[0] = fma(wa, f, v[0]);

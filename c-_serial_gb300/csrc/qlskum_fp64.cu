@@ -180,7 +180,7 @@ __global__ void k_wave_speeds(int n, const double4_32a *__restrict__ prim, doubl
 
 // ------------------------------------------------------------- flux
 
-// Once per cloud: per edge {weight of its x half-range (xpos if it lies there,
+// Once per cloud: per edge half of {weight of its x half-range (xpos if it lies there,
 // else xneg), weight of its y half-range (ypos, else yneg)}, and the gradient's
 // 2x2 solve (q_variables_mod.h:112-116) times the edge's weights.
 __global__ void k_fold_weights(DevCloud c, double2 *__restrict__ e_w64, double2 *__restrict__ e_gw64)
@@ -195,8 +195,8 @@ __global__ void k_fold_weights(DevCloud c, double2 *__restrict__ e_w64, double2 
         const unsigned dir = c.e_dir[e];
         const double2 sn = c.e_sn[e];
         const double4_32a g = c.e_geo[e];
-        e_w64[e] = make_double2(fast64::flux_weight(c, i, f, (dir & kXpos) ? 0 : 1, sn),
-                                fast64::flux_weight(c, i, f, (dir & kYpos) ? 2 : 3, sn));
+        e_w64[e] = make_double2(0.5 * fast64::flux_weight(c, i, f, (dir & kXpos) ? 0 : 1, sn),
+                                0.5 * fast64::flux_weight(c, i, f, (dir & kYpos) ? 2 : 3, sn));
         e_gw64[e] = make_double2(m.w * fast64::diff_of_products(m.y, g.z, m.z, g.w), m.w * fast64::diff_of_products(m.x, g.w, m.z, g.z));
     }
 }
@@ -273,26 +273,26 @@ __device__ __forceinline__ void edge_flux(const DevCloud &c, int i, int f, doubl
 #pragma unroll
     for (int r = 0; r < 4; r++) v[r] = 0.0;
     const double wx = inner ? w.x : 0.0;
-    fast64::split_pair(si.k, sx, sy, -wx, -w.y, v);
-    fast64::split_pair(sk.k, sx, sy, wx, w.y, v);
+    fast64::split_pair(si, sx, sy, -wx, -w.y, v);
+    fast64::split_pair(sk, sx, sy, wx, w.y, v);
     if (!inner) {
-        fast64::quad_x(si.k, sx, s2, -w.x, v);
-        fast64::quad_x(sk.k, sx, s2, w.x, v);
+        fast64::quad_x(si, sx, s2, -w.x, v);
+        fast64::quad_x(sk, sx, s2, w.x, v);
     }
     if ((dir & (kXpos | kXneg)) == (kXpos | kXneg)) {
-        const double w2 = fast64::flux_weight(c, i, f, 1, c.e_sn[e]);
+        const double w2 = 0.5 * fast64::flux_weight(c, i, f, 1, c.e_sn[e]);
         if (inner) {
-            fast64::split_pair(si.k, neg, 0u, -w2, 0.0, v);
-            fast64::split_pair(sk.k, neg, 0u, w2, 0.0, v);
+            fast64::split_pair(si, neg, 0u, -w2, 0.0, v);
+            fast64::split_pair(sk, neg, 0u, w2, 0.0, v);
         } else {
-            fast64::quad_x(si.k, neg, s2, -w2, v);
-            fast64::quad_x(sk.k, neg, s2, w2, v);
+            fast64::quad_x(si, neg, s2, -w2, v);
+            fast64::quad_x(sk, neg, s2, w2, v);
         }
     }
     if ((dir & (kYpos | kYneg)) == (kYpos | kYneg)) {
-        const double w2 = fast64::flux_weight(c, i, f, 3, c.e_sn[e]);
-        fast64::split_pair(si.k, 0u, neg, 0.0, -w2, v);
-        fast64::split_pair(sk.k, 0u, neg, 0.0, w2, v);
+        const double w2 = 0.5 * fast64::flux_weight(c, i, f, 3, c.e_sn[e]);
+        fast64::split_pair(si, 0u, neg, 0.0, -w2, v);
+        fast64::split_pair(sk, 0u, neg, 0.0, w2, v);
     }
 }
 
@@ -395,12 +395,14 @@ __global__ void __launch_bounds__(kPointBlock) k_state_update(DevCloud c, CaseCo
 
 // Fused stage: flux residual + SSPRK update of the block's points, then q and
 // (after the last stage) the wave speed of the new state for the next stage's
-// kernels.  Bound by the FP64 pipe, about 240 FP64 instructions per edge and
+// kernels.  Bound by the FP64 pipe, about 200 FP64 instructions per edge and
 // 110 per point.  Measured on 204,800 points (2.05 M edges, inner 3): 2908 us
 // per launch with CUDA's exp / erf / rsqrt, all four half-range fluxes at every
 // edge and 32 directional sums (about 630 per edge), 1066 us in this form with
-// a thread per point, 951 us with the edges spread (flux_shape).  Four blocks
-// of 128 registers a thread per SM: 5% over three blocks at 146.
+// a thread per point, 951 us with the edges spread (flux_shape), 898 us with
+// the quotient, the reciprocals and the half weights in their present forms
+// (220 -> 200 per edge, FP64 pipe 86% active).  Four blocks of 128 registers a
+// thread per SM: 5% over three blocks at 146.
 template <int P>
 __global__ void __launch_bounds__(kFluxThreads, 4) k_flux_update(DevCloud c, CaseConst K, const double4_32a *__restrict__ q,
                                                    const double4_32a *__restrict__ dq,

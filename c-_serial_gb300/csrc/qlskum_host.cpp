@@ -347,7 +347,7 @@ struct FastTables {
     std::vector<double> exp;
     FastTables() : gauss(kGaussTab), exp(kExpTab)
     {
-        const long double rpi = 0.564189583547756286948079451560772586L;  // 1 / sqrt(pi)
+        const long double rpi = 1.128379167095512573896158903121545172L;  // 2 / sqrt(pi)
         for (int j = 0; j < kGaussTab; j++) {
             const long double x = j / 1024.0L;
             gauss[j] = make_double2((double)(rpi * expl(-x * x)), (double)erfl(x));

@@ -50,7 +50,7 @@ struct DevCloud {
     const double *eps2 = nullptr;
     const double4_32a *ggeo = nullptr;           // [np]
     const double4_32a *fgeo = nullptr;           // [np][4]
-    // FP64 form: the folded weights of e_w32 and e_gw32 (below) in FP64, and the
+    // FP64 form: the folded weights of e_w32 (below; halved) and e_gw32 in FP64, and the
     // tables of the fast FP64 functions (qlskum_fast64.cuh)
     const double2 *e_w64 = nullptr;
     const double2 *e_gw64 = nullptr;
