@@ -962,6 +962,7 @@ __global__ void __launch_bounds__(128, 4) k_flux(DevCloud c, AdjT T, const float
     const int f = c.flag[i];
     const double2 nn = c.nrm[i];
     const float nx = d2f(nn.x), ny = d2f(nn.y);
+    begin_dependent();
     sown[t] = q[i];
     sown[B + t] = dq[2 * i];
     sown[2 * B + t] = dq[2 * i + 1];
@@ -1065,6 +1066,7 @@ __global__ void k_inner(DevCloud c, AdjT T, const float4 *__restrict__ bdq_out, 
     float ax[4] = {0, 0, 0, 0}, ay[4] = {0, 0, 0, 0};
     const int nb = T.nb[i];
     const long long base = T.sbase[i >> 5] + (i & 31);
+    begin_dependent();
     // the transposed list is streamed once (evict-first), the owners' bars
     // gathered as 32-byte pairs (the forward inner step's access pattern)
 #pragma unroll 2
@@ -1115,6 +1117,7 @@ __global__ void k_grad(DevCloud c, const float4 *__restrict__ q, const float4 *_
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.n) return;
+    begin_dependent();
     float bx[4], by[4], bmax[4], bmin[4], qi[4], b0x[4], b0y[4];
     ldf4(bdq[2 * i], bx);
     ldf4(bdq[2 * i + 1], by);
@@ -1171,6 +1174,7 @@ __global__ void k_q(int n, const double4_32a *__restrict__ P, const float4 *__re
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    begin_dependent();
     const double4_32a p = P[i];
     const float pf[4] = {d2f(p.x), d2f(p.y), d2f(p.z), d2f(p.w)};
     float b[4], g[4] = {0, 0, 0, 0};
@@ -1243,6 +1247,7 @@ __global__ void k_update(DevCloud c, CaseConst K, const double4_32a *__restrict_
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     float bu1 = 0.f, bu2 = 0.f;
+    begin_dependent();
     if (i < c.n) {
         const int f = c.flag[i];
         const double2 nn = c.nrm[i];
@@ -1376,34 +1381,33 @@ void flux(const Launch &L, const DevCloud &c, const AdjT &T, const float4 *q, co
           const float4 *acc, const float4 *bF, const float4 *bs, float4 *bq, float4 *bdq, float4 *bqm, float *bdelta)
 {
     const int g = grid_for(c.n, 128);
-    if (c.unit_w) adjm::k_flux<true><<<g, 128, 0, L.stream>>>(c, T, q, dq, qm, acc, bF, bs, bq, bdq, bqm, bdelta);
-    else adjm::k_flux<false><<<g, 128, 0, L.stream>>>(c, T, q, dq, qm, acc, bF, bs, bq, bdq, bqm, bdelta);
+    if (c.unit_w) launch_after(L, adjm::k_flux<true>, g, 128, 0, c, T, q, dq, qm, acc, bF, bs, bq, bdq, bqm, bdelta);
+    else launch_after(L, adjm::k_flux<false>, g, 128, 0, c, T, q, dq, qm, acc, bF, bs, bq, bdq, bqm, bdelta);
 }
 
 void inner(const Launch &L, const DevCloud &c, const AdjT &T, const float4 *bdq_out, float4 *bdq_in, float4 *bdq0,
            bool first)
 {
-    adjm::k_inner<<<grid_for(c.n, 128), 128, 0, L.stream>>>(c, T, bdq_out, bdq_in, bdq0, first);
+    launch_after(L, adjm::k_inner, grid_for(c.n, 128), 128, 0, c, T, bdq_out, bdq_in, bdq0, (int)first);
 }
 
 void grad(const Launch &L, const DevCloud &c, const float4 *q, const float4 *bdq, const float4 *bdq0,
           const float4 *bqm, float4 *bq)
 {
-    if (c.unit_w) adjm::k_grad<true><<<grid_for(c.n, 128), 128, 0, L.stream>>>(c, q, bdq, bdq0, bqm, bq);
-    else adjm::k_grad<false><<<grid_for(c.n, 128), 128, 0, L.stream>>>(c, q, bdq, bdq0, bqm, bq);
+    if (c.unit_w) launch_after(L, adjm::k_grad<true>, grid_for(c.n, 128), 128, 0, c, q, bdq, bdq0, bqm, bq);
+    else launch_after(L, adjm::k_grad<false>, grid_for(c.n, 128), 128, 0, c, q, bdq, bdq0, bqm, bq);
 }
 
 void update(const Launch &L, const DevCloud &c, const CaseConst &K, const double4_32a *Pin, const double4_32a *Pold,
             const double4_32a *Pout, int rk, const float *delta, double4_32a *bP, double4_32a *bPold, float4 *bF,
             float4 *bs, double *buinf)
 {
-    adjm::k_update<<<grid_for(c.n, 128), 128, 0, L.stream>>>(c, K, Pin, Pold, Pout, rk, delta, bP, bPold, bF, bs,
-                                                           buinf);
+    launch_after(L, adjm::k_update, grid_for(c.n, 128), 128, 0, c, K, Pin, Pold, Pout, rk, delta, bP, bPold, bF, bs, buinf);
 }
 
 void qvars(const Launch &L, int n, const double4_32a *P, const float4 *bq, double4_32a *bP)
 {
-    adjm::k_q<<<grid_for(n, 256), 256, 0, L.stream>>>(n, P, bq, bP);
+    launch_after(L, adjm::k_q, grid_for(n, 256), 256, 0, n, P, bq, bP);
 }
 
 void delta(const Launch &L, const DevCloud &c, const double4_32a *P, const float *cs, const float *bdelta, float cfl,
