@@ -2975,11 +2975,20 @@ struct AdjBuf {
     AdjT T;                            // the edge list transposed (mixed reverse)
     float4 *bq32 = nullptr, *bdqA32 = nullptr, *bdqB32 = nullptr, *bdq0_32 = nullptr, *bqm32 = nullptr;
     float *bdelta32 = nullptr, *bcs32 = nullptr;
+    // the kernels of a residual and of its VJP between the caller's buffers,
+    // captured on the second call (replay_core)
+    struct Core {
+        cudaGraphExec_t graph = nullptr;
+        long long launches = 0;
+        bool ran = false;
+    } core[2];
 };
 
 void adj_free(qlskum_handle *h)
 {
     if (!h->adj) return;
+    for (auto &g : h->adj->core)
+        if (g.graph) cudaGraphExecDestroy(g.graph);
     if (h->adj->ckpt) cudaFree(h->adj->ckpt);
     if (h->adj->seg) cudaFree(h->adj->seg);
     h->adj->set_arena.release();
@@ -3639,6 +3648,68 @@ qlskum_status adj_args(qlskum_handle *h, int objective, int count, const double 
 
 }  // namespace
 
+namespace {
+
+// flux[0] = R(P[0]) of one stage.
+void residual_core(qlskum_handle *h)
+{
+    AdjBuf *a = h->adj;
+    fp64::func_delta(h->L, h->dc, a->P[0], a->cs, a->set64.delta, h->K.cfl);
+    adj_stage_forward(h, a->set64, 0);
+}
+
+// bP = (dR/dP)^T bF at P[0].
+void vjp_core(qlskum_handle *h)
+{
+    AdjBuf *a = h->adj;
+    residual_core(h);
+    const AdjView v = adj_view(h, false);
+    zero(h, a->bP, sizeof(double4_32a) * h->np);
+    zero(h, a->bdelta, sizeof(double) * h->np);
+    adj_stage_reverse(h, a->set64, 0, v);
+    zero(h, a->bc, sizeof(double) * h->np);
+    adjl::delta(h->L, v, a->P[0], a->bdelta, h->K.cfl, a->cs, a->bc, a->bP);
+}
+
+// Runs residual_core (0) or vjp_core (1): their 10 to 30 launches and memsets
+// take the host longer than a small cloud takes the GPU (2,560 points: 400 us
+// per residual and VJP issued one by one, 340 us replayed).  The buffers are
+// the handle's own, so from the second call on the same graph is replayed; not
+// on a stream that is being captured, where the launches join the capture.
+qlskum_status replay_core(qlskum_handle *h, int which)
+{
+    AdjBuf::Core &g = h->adj->core[which];
+    void (*const run)(qlskum_handle *) = which ? vjp_core : residual_core;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CK(h, cudaStreamIsCapturing(h->L.stream, &cap));
+    if (!g.ran || cap != cudaStreamCaptureStatusNone) {
+        g.ran = true;
+        run(h);
+        return QLSKUM_OK;
+    }
+    if (!g.graph) {
+        cudaGraph_t graph = nullptr;
+        const long long before = h->launches;
+        CK(h, cudaStreamBeginCapture(h->L.stream, cudaStreamCaptureModeThreadLocal));
+        run(h);
+        cudaError_t e = cudaStreamEndCapture(h->L.stream, &graph);
+        g.launches = h->launches - before;
+        h->launches = before;
+        if (e != cudaSuccess) return cuda_fail(h, e, "cudaStreamEndCapture");
+        e = cudaGraphInstantiate(&g.graph, graph, 0);
+        cudaGraphDestroy(graph);
+        if (e != cudaSuccess) {
+            g.graph = nullptr;
+            return cuda_fail(h, e, "cudaGraphInstantiate");
+        }
+    }
+    CK(h, cudaGraphLaunch(g.graph, h->L.stream));
+    h->launches += g.launches;
+    return QLSKUM_OK;
+}
+
+}  // namespace
+
 extern "C" {
 
 qlskum_status qlskum_residual_forward(qlskum_handle *h, const double *prim, double *flux_res)
@@ -3649,8 +3720,7 @@ qlskum_status qlskum_residual_forward(qlskum_handle *h, const double *prim, doub
     if (st) return st;
     AdjBuf *a = h->adj;
     if ((st = upload_points(h, prim, a->P[0], 1.0))) return st;
-    fp64::func_delta(h->L, h->dc, a->P[0], a->cs, a->set64.delta, h->K.cfl);
-    adj_stage_forward(h, a->set64, 0);
+    if ((st = replay_core(h, 0))) return st;
     if ((st = check_launch(h, "residual_forward"))) return st;
     return download_points(h, a->set64.flux[0], flux_res);
 }
@@ -3664,14 +3734,7 @@ qlskum_status qlskum_residual_vjp(qlskum_handle *h, const double *prim, const do
     AdjBuf *a = h->adj;
     if ((st = upload_points(h, prim, a->P[0], 1.0))) return st;
     if ((st = upload_points(h, bar_flux_res, a->bF, 0.0))) return st;
-    fp64::func_delta(h->L, h->dc, a->P[0], a->cs, a->set64.delta, h->K.cfl);
-    adj_stage_forward(h, a->set64, 0);
-    const AdjView v = adj_view(h, false);
-    zero(h, a->bP, sizeof(double4_32a) * h->np);
-    zero(h, a->bdelta, sizeof(double) * h->np);
-    adj_stage_reverse(h, a->set64, 0, v);
-    zero(h, a->bc, sizeof(double) * h->np);
-    adjl::delta(h->L, v, a->P[0], a->bdelta, h->K.cfl, a->cs, a->bc, a->bP);
+    if ((st = replay_core(h, 1))) return st;
     if ((st = check_launch(h, "residual_vjp"))) return st;
     return download_points(h, a->bP, bar_prim);
 }
@@ -3711,8 +3774,7 @@ qlskum_status qlskum_residual_forward_device(qlskum_handle *h, const double *pri
     wait_on(h, h->L.stream, cs);
     fp64::fill_prim(h->L, h->np, make_double4_32a(1.0, 0, 0, 1.0), a->P[0]);
     fp64::permute_in(h->L, h->n, h->d_perm, reinterpret_cast<const double4_32a *>(prim), a->P[0]);
-    fp64::func_delta(h->L, h->dc, a->P[0], a->cs, a->set64.delta, h->K.cfl);
-    adj_stage_forward(h, a->set64, 0);
+    if ((st = replay_core(h, 0))) return st;
     fp64::permute_out(h->L, h->n, h->d_perm, a->set64.flux[0], reinterpret_cast<double4_32a *>(flux_res));
     wait_on(h, cs, h->L.stream);
     return check_launch(h, "residual_forward_device");
@@ -3732,14 +3794,7 @@ qlskum_status qlskum_residual_vjp_device(qlskum_handle *h, const double *prim, c
     fp64::permute_in(h->L, h->n, h->d_perm, reinterpret_cast<const double4_32a *>(prim), a->P[0]);
     zero(h, a->bF, sizeof(double4_32a) * h->np);
     fp64::permute_in(h->L, h->n, h->d_perm, reinterpret_cast<const double4_32a *>(bar_flux_res), a->bF);
-    fp64::func_delta(h->L, h->dc, a->P[0], a->cs, a->set64.delta, h->K.cfl);
-    adj_stage_forward(h, a->set64, 0);
-    const AdjView v = adj_view(h, false);
-    zero(h, a->bP, sizeof(double4_32a) * h->np);
-    zero(h, a->bdelta, sizeof(double) * h->np);
-    adj_stage_reverse(h, a->set64, 0, v);
-    zero(h, a->bc, sizeof(double) * h->np);
-    adjl::delta(h->L, v, a->P[0], a->bdelta, h->K.cfl, a->cs, a->bc, a->bP);
+    if ((st = replay_core(h, 1))) return st;
     fp64::permute_out(h->L, h->n, h->d_perm, a->bP, reinterpret_cast<double4_32a *>(bar_prim));
     wait_on(h, cs, h->L.stream);
     return check_launch(h, "residual_vjp_device");

@@ -31,3 +31,25 @@ def test_residual_vjp_launch_shapes(wall, layers, jitter):
         fd = float(np.sum(w * (s.residual(p + h * v) - s.residual(p - h * v))) / (2 * h))
         g = s.residual_vjp(p, w)
         assert abs(fd - float(np.sum(g * v))) <= 1e-8 * np.linalg.norm(g) * np.linalg.norm(v)
+
+
+def test_repeated_residual_and_vjp():
+    """The second and later calls replay a captured graph: the values of a first
+    call on another handle (the forward's bits; the VJP's neighbour bars are
+    added in no fixed order: 1e-13 of their norm), also after the wall gradient
+    has replaced the reverse's buffers."""
+    import qlskum
+    from qlskum import cloudgen
+    c = cloudgen.make_cloud(n_wall=49, n_layers=21, first_spacing=5e-3, radius=5.0, seed=4)
+    kw = dict(mach=0.63, aoa=2.0, cfl=0.2, vl_const=50.0, inner_iterations=1)
+    rng = np.random.default_rng(3)
+    s = qlskum.Solver(c, **kw)
+    for k in range(5):
+        P = np.tile([1.0, 0.6, 0.02, 1 / 1.4], (c.n, 1)) * (1.0 + 1e-2 * rng.standard_normal((c.n, 4)))
+        w = rng.standard_normal((c.n, 4))
+        if k == 3:
+            s.residual_vjp(P, w, wall=True)
+        o = qlskum.Solver(c, **kw)
+        assert np.array_equal(s.residual(P), o.residual(P))
+        a, b = s.residual_vjp(P, w), o.residual_vjp(P, w)
+        assert np.linalg.norm(a - b) <= 1e-13 * np.linalg.norm(b)
