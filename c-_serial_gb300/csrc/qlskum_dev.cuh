@@ -93,6 +93,14 @@ __device__ __forceinline__ unsigned long long stream_policy()
     return p;
 }
 
+// Data that the next launches read again.
+__device__ __forceinline__ unsigned long long normal_policy()
+{
+    unsigned long long p;
+    asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+
 __device__ __forceinline__ void bulk_load(unsigned dst, const void *src, unsigned bytes, unsigned bar,
                                           unsigned long long policy)
 {

@@ -879,6 +879,7 @@ qlskum_status build_geometry(const qlskum_cloud *c, const qlskum_params *p, int 
         dc.e_w64 = d_ew64;
         dc.e_gw64 = d_egw64;
     }
+    dc.stream_edges = stream_edges(ne, unit_w);
     dc.max_nb = 0;
     for (int pp = 0; pp < n; pp++) dc.max_nb = std::max(dc.max_nb, c->nbhs[G.iperm[pp]]);
 
@@ -1832,6 +1833,7 @@ qlskum_status qlskum_batch_create(const qlskum_cloud *clouds, int n_clouds, cons
         S.e_w32b = s_ewb;
         S.e_gw32 = s_egw;
         S.unit_w = unit_w ? 1 : 0;
+        S.stream_edges = stream_edges((size_t)ne_tot, unit_w);
         S.max_nb = max_nb;
         S.case_k = s_k;
         S.slice_case = s_case;

@@ -86,6 +86,8 @@ struct DevCloud {
     // per edge (FP32) and rotate it by the point normal themselves.
     int unit_w = 0;
     const float2 *e_xy32 = nullptr;
+    // the mixed gradient and inner step read their edge arrays evict-first (stream_edges())
+    int stream_edges = 0;
     // largest neighbour count of the cloud (sizes the staged kernels' shared memory)
     int max_nb = 0;
     // A batch's concatenated cloud (several cases, each its own flight
@@ -98,6 +100,16 @@ struct DevCloud {
     // also holds 1 for a non-finite residual)
     int *fault = nullptr;
 };
+
+// The bytes per launch up to which the mixed inner step's edge arrays (20 B per
+// slot with unit weights, 28 B with others) are left in L2 for the next launch:
+// half of the 129 MB, the rest for the per-point data of the launches between.
+// One lane per point, three inner iterations per stage, us per iteration,
+// evict-first / left in L2: 51,200 points (10 MB) 202 / 189, 101,617 (20 MB)
+// 259 / 250, 204,800 (41 MB) 391 / 362, 300,000 (60 MB) 553 / 520, 360,000
+// (72 MB) 586 / 583, 409,600 (82 MB) 635 / 650, 1,024,000 (205 MB) 1,358 / 1,390.
+constexpr size_t kL2EdgeBytes = 64u << 20;
+inline int stream_edges(size_t slots, bool unit_w) { return slots * (unit_w ? 20 : 28) > kL2EdgeBytes ? 1 : 0; }
 
 // Free-stream constants of one case (parameter_mod.h:4-30).
 struct CaseConst {

@@ -142,18 +142,24 @@ __global__ void k_derived(int n, const double4_32a *__restrict__ prim, float4 *_
 }
 
 // Edge vector and least-squares weights of edge e: {delx, dely, w delx, w dely}.
-// The gradient and inner-step kernels stream their edge arrays once per
-// launch: those loads are marked evict-first (__ldcs), so that L1 and L2
-// keep the gathered neighbour data instead (inner step 0.059 -> 0.055 ms on
-// the 1.02 M cloud).
-template <bool UW>
+// STREAM (DevCloud::stream_edges): the edge arrays are past what L2 keeps from
+// one launch to the next, and the gradient and inner-step kernels' edge loads
+// are marked evict-first (__ldcs) so that L2 keeps the gathered neighbour data
+// instead (inner step 0.059 -> 0.055 ms on the 1.02 M cloud).  Smaller clouds
+// read them as ordinary read-only data, so that the next launch finds them in L2.
+template <bool STREAM, typename T> __device__ __forceinline__ T edge_load(const T *p)
+{
+    return STREAM ? __ldcs(p) : __ldg(p);
+}
+
+template <bool UW, bool STREAM>
 __device__ __forceinline__ float4 edge_w(const DevCloud &c, long long e)
 {
     if (UW) {
-        const float2 d = __ldcs(c.e_xy32 + e);
+        const float2 d = edge_load<STREAM>(c.e_xy32 + e);
         return make_float4(d.x, d.y, d.x, d.y);
     }
-    return __ldcs(c.e_geo32 + e);
+    return edge_load<STREAM>(c.e_geo32 + e);
 }
 
 // ----------------------------------------------------------- point bodies
@@ -165,7 +171,7 @@ __device__ __forceinline__ float4 edge_w(const DevCloud &c, long long e)
 // q_variables_mod.h:36-118: FP32 differences, weighted by the FP64-folded
 // per-edge solve weights (DevCloud::e_gw32); with DT (the first stage) also
 // the local time step (state_update_mod.h:448-496) in FP32.
-template <bool DT, int L = 1>
+template <bool DT, int L, bool STREAM>
 __device__ __forceinline__ void grad_point(const DevCloud &c, int i, const float4 *__restrict__ q,
                                            float4 *__restrict__ dq, float4 *__restrict__ qm,
                                            const float *__restrict__ cs, float *__restrict__ delta, float cfl,
@@ -183,8 +189,8 @@ __device__ __forceinline__ void grad_point(const DevCloud &c, int i, const float
 #pragma unroll 2
     for (int j = sub; j < nb; j += L) {
         const long long e = base + 32LL * j;
-        const int k = __ldcs(c.e_nbr + e);
-        const float2 gw = __ldcs(c.e_gw32 + e);
+        const int k = edge_load<STREAM>(c.e_nbr + e);
+        const float2 gw = edge_load<STREAM>(c.e_gw32 + e);
         float qk[4];
         ld4(q[k], qk);
 #pragma unroll
@@ -195,7 +201,7 @@ __device__ __forceinline__ void grad_point(const DevCloud &c, int i, const float
             dx[r] = fmaf(gw.x, d, dx[r]);
             dy[r] = fmaf(gw.y, d, dy[r]);
         }
-        if (DT) min_dt = fminf(min_dt, cfl * __fdividef(__ldcs(c.e_dist32 + e), cs[k]));
+        if (DT) min_dt = fminf(min_dt, cfl * __fdividef(edge_load<STREAM>(c.e_dist32 + e), cs[k]));
     }
     if (L > 1) {
         const unsigned m = group_mask<L>();
@@ -241,7 +247,7 @@ __device__ __forceinline__ void inner_finish(const float ax[4], const float ay[4
     out[1] = mk4(ry);
 }
 
-template <bool UW, int L = 1>
+template <bool UW, int L, bool STREAM>
 __device__ __forceinline__ void inner_point(const DevCloud &c, int i, const float4 *__restrict__ dq0,
                                             const float4 *__restrict__ dq_in, float4 *__restrict__ dq_out,
                                             int sub = 0)
@@ -253,9 +259,9 @@ __device__ __forceinline__ void inner_point(const DevCloud &c, int i, const floa
 #pragma unroll 2
     for (int j = sub; j < nb; j += L) {
         const long long e = base + 32LL * j;
-        const int k = __ldcs(c.e_nbr + e);
-        const float4 g = edge_w<UW>(c, e);
-        const float2 gw = __ldcs(c.e_gw32 + e);
+        const int k = edge_load<STREAM>(c.e_nbr + e);
+        const float4 g = edge_w<UW, STREAM>(c, e);
+        const float2 gw = edge_load<STREAM>(c.e_gw32 + e);
         // the neighbour's gradient pair in one 32-byte load
         float4 gx, gy;
         ldg_2x4(dq_in + 2 * k, gx, gy);
@@ -1020,23 +1026,23 @@ __device__ __forceinline__ float flux_point_rps(const DevCloud &c, const CaseCon
 
 // ---------------------------------------------------- single-case kernels
 
-template <bool DT, int L>
+template <bool DT, int L, bool STREAM>
 __global__ void k_q_derivatives(DevCloud c, const float4 *__restrict__ q, float4 *__restrict__ dq,
                                 float4 *__restrict__ qm, const float *__restrict__ cs, float *__restrict__ delta,
                                 float cfl)
 {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = g / L;
-    if (i < c.n) grad_point<DT, L>(c, i, q, dq, qm, cs, delta, cfl, g % L);
+    if (i < c.n) grad_point<DT, L, STREAM>(c, i, q, dq, qm, cs, delta, cfl, g % L);
 }
 
-template <bool UW, int L>
+template <bool UW, int L, bool STREAM>
 __global__ void k_q_inner(DevCloud c, const float4 *__restrict__ dq0, const float4 *__restrict__ dq_in,
                           float4 *__restrict__ dq_out)
 {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = g / L;
-    if (i < c.n) inner_point<UW, L>(c, i, dq0, dq_in, dq_out, g % L);
+    if (i < c.n) inner_point<UW, L, STREAM>(c, i, dq0, dq_in, dq_out, g % L);
 }
 
 // ---------------------------------------------- edge lists by bulk copies
@@ -1165,7 +1171,7 @@ __global__ void k_q_derivatives_ring(DevCloud c, const float4 *__restrict__ q, f
     constexpr int NA = DT ? 3 : 2, PB = DT ? 16 : 12;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     unsigned char *buf = ring_smem + warp * (NS * CE * 32 * PB);
-    const unsigned long long pol = stream_policy();
+    const unsigned long long pol = c.stream_edges ? stream_policy() : normal_policy();
     EdgeRing<NA> R;
     R.src[0] = reinterpret_cast<const char *>(c.e_nbr);
     R.src[1] = reinterpret_cast<const char *>(c.e_gw32);
@@ -1468,15 +1474,20 @@ void q_derivatives(const Launch &L, const DevCloud &c, const float4 *q, float4 *
             launch_after(L, k_q_derivatives_ring<false>, g, L.block, sm, c, q, dq, qm, nullptr, nullptr, cfl);
         }
     } else {
-#define QLSKUM_GRAD(LN)                                                                                         \
+#define QLSKUM_GRAD(LN, ST)                                                                                     \
     if (delta)                                                                                                  \
-        launch_after(L, k_q_derivatives<true, LN>, grid_for(c.n * LN, L.block), L.block, 0, c, q, dq, qm, cspeed,  \
-                                                                                        delta, cfl);           \
+        launch_after(L, k_q_derivatives<true, LN, ST>, grid_for(c.n * LN, L.block), L.block, 0, c, q, dq, qm,   \
+                     cspeed, delta, cfl);                                                                       \
     else                                                                                                        \
-        launch_after(L, k_q_derivatives<false, LN>, grid_for(c.n * LN, L.block), L.block, 0, c, q, dq, qm, cspeed, \
-                                                                                         delta, cfl)
-        if (L.lanes == 4) { QLSKUM_GRAD(4); }
-        else { QLSKUM_GRAD(2); }
+        launch_after(L, k_q_derivatives<false, LN, ST>, grid_for(c.n * LN, L.block), L.block, 0, c, q, dq, qm,  \
+                     cspeed, delta, cfl)
+        if (c.stream_edges) {
+            if (L.lanes == 4) { QLSKUM_GRAD(4, true); }
+            else { QLSKUM_GRAD(2, true); }
+        } else {
+            if (L.lanes == 4) { QLSKUM_GRAD(4, false); }
+            else { QLSKUM_GRAD(2, false); }
+        }
 #undef QLSKUM_GRAD
     }
     QLSKUM_LAUNCHED(L);
@@ -1491,14 +1502,20 @@ void q_inner(const Launch &L, const DevCloud &c, const float4 *dq0, const float4
             else
                 launch_after(L, k_q_inner_st<B_, D_, false>, grid_for(c.n, B_), B_, staged_bytes(B_, D_, 2, c.max_nb, false), c, dq0, dq_in, dq_out))
     } else {
-#define QLSKUM_INNER(LN)                                                                                        \
+#define QLSKUM_INNER(LN, ST)                                                                                    \
     if (c.unit_w)                                                                                               \
-        launch_after(L, k_q_inner<true, LN>, grid_for(c.n * LN, L.block), L.block, 0, c, dq0, dq_in, dq_out);      \
+        launch_after(L, k_q_inner<true, LN, ST>, grid_for(c.n * LN, L.block), L.block, 0, c, dq0, dq_in, dq_out); \
     else                                                                                                        \
-        launch_after(L, k_q_inner<false, LN>, grid_for(c.n * LN, L.block), L.block, 0, c, dq0, dq_in, dq_out)
-        if (L.lanes == 4) { QLSKUM_INNER(4); }
-        else if (L.lanes == 2) { QLSKUM_INNER(2); }
-        else { QLSKUM_INNER(1); }
+        launch_after(L, k_q_inner<false, LN, ST>, grid_for(c.n * LN, L.block), L.block, 0, c, dq0, dq_in, dq_out)
+        if (c.stream_edges) {
+            if (L.lanes == 4) { QLSKUM_INNER(4, true); }
+            else if (L.lanes == 2) { QLSKUM_INNER(2, true); }
+            else { QLSKUM_INNER(1, true); }
+        } else {
+            if (L.lanes == 4) { QLSKUM_INNER(4, false); }
+            else if (L.lanes == 2) { QLSKUM_INNER(2, false); }
+            else { QLSKUM_INNER(1, false); }
+        }
 #undef QLSKUM_INNER
     }
     QLSKUM_LAUNCHED(L);

@@ -41,3 +41,20 @@ def test_block_sizes_and_lanes(wall, layers, power):
     assert np.allclose(p4, ref[0], rtol=1e-5, atol=1e-6)
 
 
+@pytest.mark.parametrize("lanes", [1, 2, 4])
+@pytest.mark.parametrize("power", [0.0, -2.0])
+def test_edge_lists_past_l2(lanes, power):
+    """Three cases of one cloud are past the size at which the edge lists are
+    read evict-first (26 or 37 MB each, 64 MB), one case is not: how they are read
+    changes no bit."""
+    import qlskum
+    from qlskum import cloudgen
+    c = cloudgen.make_cloud(n_wall=397, n_layers=331, seed=3, te_spread=0.064)
+    out = []
+    for cases in (1, 3):
+        b = qlskum.Batch([c], [(0, 0.63, 2.0)] * cases, cfl=0.2, vl_const=50.0, power=power, inner_iterations=2)
+        b.set_launch_config(128, lanes, 10)
+        b.run(3)
+        out += [b.prim(k) for k in range(cases)]
+    for p in out[1:]:
+        assert np.array_equal(out[0], p)
