@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(kPointBlock) k_state_update(DevCloud c, CaseCo
         double P[4], F[4];
         ld4(prim[i], P);
         ld4(flux_res[i], F);
-        r2 = fast64::stage(K, c.flag[i], nn.x, nn.y, P, prim_old + i, F, rk);
+        r2 = fast64::stage(K, c.gauss_tab, c.flag[i], nn.x, nn.y, P, prim_old + i, F, rk);
         prim_next[i] = mk4(P);
     }
     partial8(r2, i, c.n, psum, pmax);
@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(kFluxThreads, 4) k_flux_update(DevCloud c, Cas
         const double2 nn = c.nrm[i];
         double S[4], Q[4];
         ld4(prim[i], S);
-        r2 = fast64::stage(K, c.flag[i], nn.x, nn.y, S, prim_old + i, F, rk);
+        r2 = fast64::stage(K, c.gauss_tab, c.flag[i], nn.x, nn.y, S, prim_old + i, F, rk);
         prim_next[i] = mk4(S);
         fast64::q_of(S, Q);
         q_next[i] = mk4(Q);

@@ -856,13 +856,13 @@ qlskum_status build_geometry(const qlskum_cloud *c, const qlskum_params *p, int 
     up(d_exy32, e_xy32); up(d_egw32, e_gw32);
     double2 *d_ew64 = nullptr, *d_egw64 = nullptr, *d_gauss = nullptr;
     double *d_exp = nullptr;
+    const FastTables &T = fast_tables();
+    d_gauss = A.alloc<double2>(T.gauss.size());  // both forms: the outer points' state update is FP64
+    up(d_gauss, T.gauss);
     if (need_fp64) {
-        const FastTables &T = fast_tables();
         d_ew64 = A.alloc<double2>(ne);
         d_egw64 = A.alloc<double2>(ne);
-        d_gauss = A.alloc<double2>(T.gauss.size());
         d_exp = A.alloc<double>(T.exp.size());
-        up(d_gauss, T.gauss);
         up(d_exp, T.exp);
     }
     DevCloud &dc = G.dc;
@@ -1835,6 +1835,7 @@ qlskum_status qlskum_batch_create(const qlskum_cloud *clouds, int n_clouds, cons
         S.unit_w = unit_w ? 1 : 0;
         S.stream_edges = stream_edges((size_t)ne_tot, unit_w);
         S.max_nb = max_nb;
+        S.gauss_tab = b->geo[0].dc.gauss_tab;
         S.case_k = s_k;
         S.slice_case = s_case;
     }

@@ -22,6 +22,7 @@
 // the steady state).
 #include "qlskum_math.cuh"
 #include "qlskum_dev.cuh"
+#include "qlskum_fast64.cuh"
 #include <algorithm>
 
 namespace qlskum {
@@ -97,12 +98,17 @@ __device__ __forceinline__ void p2c_fast(const double P[4], double nx, double ny
 }
 
 // One SSPRK stage of one point (state_update_mod.h:111-282), FP64.
-__device__ __forceinline__ double stage_update_fast(const CaseConst &K, int f, double nx, double ny, double P[4],
+__device__ __forceinline__ double stage_update_fast(const CaseConst &K, const double2 *__restrict__ tab, int f,
+                                                    double nx, double ny, double P[4],
                                                     const double4_32a *prim_old_i, const double F[4], int rk)
 {
-    double U[4];
-    if (f == kOuter) conserved_vector_Ubar(K, P, nx, ny, U);
-    else p2c_fast(P, nx, ny, U);
+    double U[4], Uinf[4];
+    if (f == kOuter) {
+        fast64::half_range(-1.0, K.gamma - 1.0, K.rho_inf, K.u1_inf, K.u2_inf, K.pr_inf, nx, ny, tab, Uinf);
+        fast64::conserved(f, K.gamma - 1.0, nx, ny, P, Uinf, tab, U);
+    } else {
+        p2c_fast(P, nx, ny, U);
+    }
     const double rho0 = U[0];
     if (rk != 3) {
 #pragma unroll
@@ -110,7 +116,7 @@ __device__ __forceinline__ double stage_update_fast(const CaseConst &K, int f, d
     } else {
         double Po[4], Uo[4];
         ld4(*prim_old_i, Po);
-        if (f == kOuter) conserved_vector_Ubar(K, Po, nx, ny, Uo);
+        if (f == kOuter) fast64::conserved(f, K.gamma - 1.0, nx, ny, Po, Uinf, tab, Uo);
         else p2c_fast(Po, nx, ny, Uo);
 #pragma unroll
         for (int j = 0; j < 4; j++) U[j] = fma(2.0 / 3.0, Uo[j], (1.0 / 3.0) * fma(-0.5, F[j], U[j]));
@@ -658,8 +664,8 @@ __device__ __forceinline__ float flux_tail(const DevCloud &c, const CaseConst &K
         for (int r = 0; r < 4; r++) F[r] = dl * f2d(acc[r]);
         // (two calls, not a reference to either: a pointer to the launch's
         // constants would copy them to the stack)
-        if (c.case_k) r2 = d2f(stage_update_fast(c.case_k[c.slice_case[i >> 5]], f, nn.x, nn.y, P, prim_old + i, F, rk));
-        else r2 = d2f(stage_update_fast(K, f, nn.x, nn.y, P, prim_old + i, F, rk));
+        if (c.case_k) r2 = d2f(stage_update_fast(c.case_k[c.slice_case[i >> 5]], c.gauss_tab, f, nn.x, nn.y, P, prim_old + i, F, rk));
+        else r2 = d2f(stage_update_fast(K, c.gauss_tab, f, nn.x, nn.y, P, prim_old + i, F, rk));
         prim_next[i] = mk4(P);
         q_of(P, Q);
         cs = wave_speed32(P);

@@ -156,3 +156,35 @@ def test_inner_step_on_its_own(wall, power):
     md = c.min_dist[:, None, None]
     reach = 2.5 * 3.0 * np.abs(o.dq).max()  # gradient times an edge of up to 3 min_dist, over min_dist
     assert (np.abs(d - o.dq) <= EPS * (8 * 2.5 * 2 * np.abs(o.q).max() / md + 8 * reach)).all()
+
+
+@pytest.mark.parametrize("mach", [0.01, 0.85, 3.0, 9.0])
+@pytest.mark.parametrize("rk", [1, 3])
+def test_stage_over_the_mach_range(mach, rk):
+    """The SSPRK stage, with the outer points' half ranges (|S| past the table at
+    Mach 9).  A half range is at most 10 roundings and an S to 4 ulps, whose
+    dA / dS and S^2 exp(-S^2) are below 0.6: 20 ulps of rho (1, U, U, U^2); half
+    the residual's own bound comes with F.  u = m / rho and p = 0.4 (E - m^2 / (2 rho))
+    take an error dU to at most 4 times its size over rho (U for u, U^2 for p)."""
+    import qlskum
+    from qlskum import cloudgen
+    c = cloudgen.make_cloud(n_wall=48, n_layers=21, first_spacing=5e-3, radius=5.0, seed=3)
+    kw = dict(mach=mach, aoa=2.0, cfl=0.02, vl_const=50.0, inner_iterations=0)
+    P = disturbed(c, mach)
+    s, o = qlskum.Solver(c, **kw), qlskum_oracle.Oracle(c, **kw)
+    for h in (s, o):
+        h.set_prim(P)
+        h.snapshot_prim_old()
+        h.func_delta()
+        h.eval_q_variables()
+        h.eval_q_derivatives()
+        h.cal_flux_residual()
+        h.state_update(rk)
+    U = float((np.hypot(P[:, 1], P[:, 2]) + 3 * np.sqrt(P[:, 3] / P[:, 0])).max())
+    G = P[:, 0].max() * np.array([1.0, U, U, U * U])
+    # flux_bound()'s scale is U G
+    b = float((0.5 * flux_bound(c, P, o.delta) / G + 20 * EPS).max())
+    tol = 4 * b * np.array([1.0, U, U, U * U]) * P[:, 0].max() / o.prim[:, 0].min()
+    assert (np.abs(s.prim - o.prim).max(axis=0) <= tol).all()
+    outer = c.flag_1 == 2
+    assert outer.any() and np.abs(s.prim - P)[outer].max() > 1e-4
