@@ -714,15 +714,14 @@ __device__ __forceinline__ void block_sum_max32(float v, double *out_sum, double
 // Fused stage of one point: FP32 edge work with the FP64-folded solve
 // weights, then the stage update (flux_tail).
 // Returns the point's res_sqr.
-template <bool UW, int L = 1>
+template <bool UW>
 __device__ __forceinline__ float flux_point(const DevCloud &c, const CaseConst &K, int i,
                                              const float4 *__restrict__ q, const float4 *__restrict__ dq,
                                              const float4 *__restrict__ qm, const float *__restrict__ delta,
                                              const double4_32a *__restrict__ prim,
                                              const double4_32a *__restrict__ prim_old,
                                              double4_32a *__restrict__ prim_next, float4 *__restrict__ q_next,
-                                             float *__restrict__ cs_next, int rk, float4 *__restrict__ acc_out,
-                                             int sub = 0)
+                                             float *__restrict__ cs_next, int rk, float4 *__restrict__ acc_out)
 {
     const int f = c.flag[i];
     const double2 nn = c.nrm[i];
@@ -744,7 +743,7 @@ __device__ __forceinline__ float flux_point(const DevCloud &c, const CaseConst &
     }
     const float e2i = c.eps2_32[i];
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int j = sub; j < nb; j += L) {
+    for (int j = 0; j < nb; j++) {
         const long long e = base + 32LL * j;
         const int k = c.e_nbr[e];
         float4 g;
@@ -758,12 +757,6 @@ __device__ __forceinline__ float flux_point(const DevCloud &c, const CaseConst &
         ld4(qm[2 * k], mxk);
         ld4(qm[2 * k + 1], mnk);
         flux_edge(c, e, f, nx, ny, qi, dxi, dyi, mxi, mni, e2i, g, w, dir, qk, dxk, dyk, mxk, mnk, c.eps2_32[k], acc);
-    }
-    if (L > 1) {
-        const unsigned m = group_mask<L>();
-#pragma unroll
-        for (int r = 0; r < 4; r++) acc[r] = group_sum<L>(acc[r], m);
-        if (sub != 0) return 0.0f;
     }
     return flux_tail(c, K, i, f, nn, nx, ny, acc, delta, prim, prim_old, prim_next, q_next, cs_next, rk, acc_out);
 }
@@ -874,16 +867,22 @@ __device__ __forceinline__ void load_nbr(const DevCloud &c, int k, const float4 
 // pairs) and streamed edge data are loaded while edge j is evaluated, the
 // neighbour index one edge earlier still.  No shared memory: the L1 data
 // path carries only the gathers themselves.  Same arithmetic in the same
-// edge order as flux_point.  dq and qm must be 32-byte aligned per point
+// edge order as flux_point (L = 1).  With L lanes per point lane s takes edges
+// s, s + L, ...: below about 100,000 points the kernel waits for the longest
+// chain of edges, not for the chip, and halving it is worth more than the
+// second lane (us per launch, one lane / two: 9,600 points 15.8 / 14.5, 51,200
+// 18.9 / 18.4, 101,617 25.3 / 26.2, 204,800 40.5 / 52.2; without the prefetch two
+// lanes took 15.0, 19.5, 28.6, 59.9).  dq and qm must be 32-byte aligned per point
 // (two float4 per point from an aligned base).
-template <bool UW>
+template <bool UW, int L>
 __device__ __forceinline__ float flux_point_rp(const DevCloud &c, const CaseConst &K, int i,
                                                const float4 *__restrict__ q, const float4 *__restrict__ dq,
                                                const float4 *__restrict__ qm, const float *__restrict__ delta,
                                                const double4_32a *__restrict__ prim,
                                                const double4_32a *__restrict__ prim_old,
                                                double4_32a *__restrict__ prim_next, float4 *__restrict__ q_next,
-                                               float *__restrict__ cs_next, int rk, float4 *__restrict__ acc_out)
+                                               float *__restrict__ cs_next, int rk, float4 *__restrict__ acc_out,
+                                               int sub = 0)
 {
     const int f = c.flag[i];
     const double2 nn = c.nrm[i];
@@ -896,14 +895,15 @@ __device__ __forceinline__ float flux_point_rp(const DevCloud &c, const CaseCons
     unsigned dn = 0;
     int kn = 0;
     int k0 = 0;
-    if (nb > 0) {
-        k0 = c.e_nbr[base];
-        edge_geo<UW>(c, base, gn, wn);
-        dn = c.e_dir[base];
+    const long long e0 = base + 32 * sub;
+    if (sub < nb) {
+        k0 = c.e_nbr[e0];
+        edge_geo<UW>(c, e0, gn, wn);
+        dn = c.e_dir[e0];
     }
-    if (nb > 1) kn = c.e_nbr[base + 32];
+    if (sub + L < nb) kn = c.e_nbr[e0 + 32 * L];
     begin_dependent();
-    if (nb > 0) load_nbr(c, k0, q, dq, qm, nd);
+    if (sub < nb) load_nbr(c, k0, q, dq, qm, nd);
     NbrData me;
     load_nbr(c, i, q, dq, qm, me);
     float qi[4], dxi[4], dyi[4], mxi[4], mni[4];
@@ -920,18 +920,18 @@ __device__ __forceinline__ float flux_point_rp(const DevCloud &c, const CaseCons
     }
     const float e2i = me.e2;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    for (int j = 0; j < nb; j++) {
+    for (int j = sub; j < nb; j += L) {
         const long long e = base + 32LL * j;
         const NbrData cur = nd;
         const float4 g = gn;
         const float2 w = wn;
         const unsigned dir = dn;
-        if (j + 1 < nb) {
+        if (j + L < nb) {
             load_nbr(c, kn, q, dq, qm, nd);
-            edge_geo<UW>(c, e + 32, gn, wn);
-            dn = c.e_dir[e + 32];
+            edge_geo<UW>(c, e + 32 * L, gn, wn);
+            dn = c.e_dir[e + 32 * L];
         }
-        if (j + 2 < nb) kn = c.e_nbr[e + 64];
+        if (j + 2 * L < nb) kn = c.e_nbr[e + 64 * L];
         float qk[4], dxk[4], dyk[4], mxk[4], mnk[4];
         ld4(cur.q, qk);
         ld4(cur.dx, dxk);
@@ -939,6 +939,12 @@ __device__ __forceinline__ float flux_point_rp(const DevCloud &c, const CaseCons
         ld4(cur.mx, mxk);
         ld4(cur.mn, mnk);
         flux_edge(c, e, f, nx, ny, qi, dxi, dyi, mxi, mni, e2i, g, w, dir, qk, dxk, dyk, mxk, mnk, cur.e2, acc);
+    }
+    if (L > 1) {
+        const unsigned m = group_mask<L>();
+#pragma unroll
+        for (int r = 0; r < 4; r++) acc[r] = group_sum<L>(acc[r], m);
+        if (sub != 0) return 0.0f;
     }
     return flux_tail(c, K, i, f, nn, nx, ny, acc, delta, prim, prim_old, prim_next, q_next, cs_next, rk, acc_out);
 }
@@ -1250,8 +1256,7 @@ __global__ void k_q_derivatives_ring(DevCloud c, const float4 *__restrict__ q, f
     }
 }
 
-// L lanes per point: BLOCK threads hold BLOCK / L points.
-template <int BLOCK, int MINB, bool UW, int L = 1>
+template <int BLOCK, int MINB, bool UW>
 __global__ void __launch_bounds__(BLOCK, MINB) k_flux_update(DevCloud c, CaseConst K, const float4 *__restrict__ q,
                                                        const float4 *__restrict__ dq, const float4 *__restrict__ qm,
                                                        const float *__restrict__ delta,
@@ -1262,12 +1267,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_flux_update(DevCloud c, CaseCon
                                                        double *__restrict__ psum, double *__restrict__ pmax,
                                                        float4 *__restrict__ acc_out)
 {
-    const int g = blockIdx.x * BLOCK + threadIdx.x;
-    const int i = g / L;
+    const int i = blockIdx.x * BLOCK + threadIdx.x;
     float r2 = 0.0f;
     if (i < c.n)
-        r2 = flux_point<UW, L>(c, K, i, q, dq, qm, delta, prim, prim_old, prim_next, q_next, cs_next, rk, acc_out,
-                               g % L);
+        r2 = flux_point<UW>(c, K, i, q, dq, qm, delta, prim, prim_old, prim_next, q_next, cs_next, rk, acc_out);
     if (psum) block_sum_max32<BLOCK>(r2, psum + blockIdx.x, pmax + blockIdx.x);
 }
 
@@ -1295,8 +1298,9 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_flux_update_st(DevCloud c, Case
     if (psum) block_sum_max32<BLOCK>(r2, psum + blockIdx.x, pmax + blockIdx.x);
 }
 
-// Register-prefetch form of k_flux_update (flux_point_rp).
-template <int BLOCK, int MINB, bool UW>
+// Register-prefetch form of k_flux_update (flux_point_rp); L lanes per point:
+// BLOCK threads hold BLOCK / L points.
+template <int BLOCK, int MINB, bool UW, int L = 1>
 __global__ void __launch_bounds__(BLOCK, MINB) k_flux_update_rp(DevCloud c, CaseConst K, const float4 *__restrict__ q,
                                                           const float4 *__restrict__ dq,
                                                           const float4 *__restrict__ qm,
@@ -1308,10 +1312,12 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_flux_update_rp(DevCloud c, Case
                                                           int rk, double *__restrict__ psum,
                                                           double *__restrict__ pmax, float4 *__restrict__ acc_out)
 {
-    const int i = blockIdx.x * BLOCK + threadIdx.x;
+    const int g = blockIdx.x * BLOCK + threadIdx.x;
+    const int i = g / L;
     float r2 = 0.0f;
     if (i < c.n)
-        r2 = flux_point_rp<UW>(c, K, i, q, dq, qm, delta, prim, prim_old, prim_next, q_next, cs_next, rk, acc_out);
+        r2 = flux_point_rp<UW, L>(c, K, i, q, dq, qm, delta, prim, prim_old, prim_next, q_next, cs_next, rk, acc_out,
+                                  g % L);
     if (psum) block_sum_max32<BLOCK>(r2, psum + blockIdx.x, pmax + blockIdx.x);
 }
 
@@ -1529,10 +1535,9 @@ void q_inner(const Launch &L, const DevCloud &c, const float4 *dq0, const float4
 
 // Launch-shape variants of the fused kernel (threads per block, minimum
 // resident blocks per SM -> register cap; 4..7 the staged-gather form; 8, 9
-// the per-edge gather form with 2 / 4 lanes per point; 10..13 the
-// register-prefetch form; 14, 15 the same with the owner's data in shared
-// memory; 16..18 that form with only the edge index and data prefetched),
-// picked by the host's autotuner.
+// the register-prefetch form with 2 / 4 lanes per point, 10..13 with one;
+// 14, 15 the same with the owner's data in shared memory; 16..18 that form
+// with only the edge index and data prefetched), picked by the host's autotuner.
 const int kFluxVariants = 19;
 static const int kFluxBlock[kFluxVariants] = {128, 128, 64, 256, 128, 128, 64, 256, 128, 256,
                                               128, 128, 64, 256, 128, 128, 128, 128, 128};
@@ -1550,16 +1555,15 @@ void flux_update(const Launch &L, const DevCloud &c, const CaseConst &k, const f
                  double4_32a *prim_next, float4 *q_next, float *cspeed_next, int rk, const Reduce &R, int variant,
                  float4 *acc_out)
 {
-#define QLSKUM_FLUX_L(B, MB, LN)                                                                            \
+#define QLSKUM_FLUX(B, MB)                                                                                  \
     if (c.unit_w)                                                                                           \
-        launch_after(L, k_flux_update<B, MB, true, LN>, grid_for(c.n * LN, B), B, 0,                           \
+        launch_after(L, k_flux_update<B, MB, true>, grid_for(c.n, B), B, 0,                           \
             c, k, q, dq, qm, delta, prim, prim_old, prim_next, q_next, cspeed_next, rk, R.partial_sum,      \
             R.partial_max, acc_out);                                                                        \
     else                                                                                                    \
-        launch_after(L, k_flux_update<B, MB, false, LN>, grid_for(c.n * LN, B), B, 0,                          \
+        launch_after(L, k_flux_update<B, MB, false>, grid_for(c.n, B), B, 0,                          \
             c, k, q, dq, qm, delta, prim, prim_old, prim_next, q_next, cspeed_next, rk, R.partial_sum,      \
             R.partial_max, acc_out)
-#define QLSKUM_FLUX(B, MB) QLSKUM_FLUX_L(B, MB, 1)
 #define QLSKUM_FLUX_ST(B, MB)                                                                               \
     if (c.unit_w)                                                                                           \
         launch_after(L, k_flux_update_st<B, MB, true>, grid_for(c.n, B), B, 0, c, k, q, dq, qm, delta, prim,   \
@@ -1571,14 +1575,14 @@ void flux_update(const Launch &L, const DevCloud &c, const CaseConst &k, const f
                                                                           prim_old, prim_next, q_next,     \
                                                                           cspeed_next, rk, R.partial_sum,  \
                                                                           R.partial_max, acc_out)
-#define QLSKUM_FLUX_RP(B, MB)                                                                               \
+#define QLSKUM_FLUX_RP(B, MB, LN)                                                                           \
     if (c.unit_w)                                                                                           \
-        launch_after(L, k_flux_update_rp<B, MB, true>, grid_for(c.n, B), B, 0, c, k, q, dq, qm, delta, prim,   \
+        launch_after(L, k_flux_update_rp<B, MB, true, LN>, grid_for(c.n * LN, B), B, 0, c, k, q, dq, qm, delta, prim,   \
                                                                          prim_old, prim_next, q_next,      \
                                                                          cspeed_next, rk, R.partial_sum,   \
                                                                          R.partial_max, acc_out);          \
     else                                                                                                    \
-        launch_after(L, k_flux_update_rp<B, MB, false>, grid_for(c.n, B), B, 0, c, k, q, dq, qm, delta, prim,  \
+        launch_after(L, k_flux_update_rp<B, MB, false, LN>, grid_for(c.n * LN, B), B, 0, c, k, q, dq, qm, delta, prim,  \
                                                                           prim_old, prim_next, q_next,     \
                                                                           cspeed_next, rk, R.partial_sum,  \
                                                                           R.partial_max, acc_out)
@@ -1603,12 +1607,12 @@ void flux_update(const Launch &L, const DevCloud &c, const CaseConst &k, const f
     case 5: QLSKUM_FLUX_ST(128, 5); break;
     case 6: QLSKUM_FLUX_ST(64, 8); break;
     case 7: QLSKUM_FLUX_ST(256, 2); break;
-    case 8: QLSKUM_FLUX_L(128, 4, 2); break;
-    case 9: QLSKUM_FLUX_L(256, 2, 4); break;
-    case 10: QLSKUM_FLUX_RP(128, 4); break;
-    case 11: QLSKUM_FLUX_RP(128, 5); break;
-    case 12: QLSKUM_FLUX_RP(64, 6); break;
-    case 13: QLSKUM_FLUX_RP(256, 2); break;
+    case 8: QLSKUM_FLUX_RP(128, 4, 2); break;
+    case 9: QLSKUM_FLUX_RP(256, 2, 4); break;
+    case 10: QLSKUM_FLUX_RP(128, 4, 1); break;
+    case 11: QLSKUM_FLUX_RP(128, 5, 1); break;
+    case 12: QLSKUM_FLUX_RP(64, 6, 1); break;
+    case 13: QLSKUM_FLUX_RP(256, 2, 1); break;
     case 14: QLSKUM_FLUX_RPS(128, 5, true); break;
     case 15: QLSKUM_FLUX_RPS(128, 6, true); break;
     case 16: QLSKUM_FLUX_RPS(128, 6, false); break;
@@ -1617,7 +1621,6 @@ void flux_update(const Launch &L, const DevCloud &c, const CaseConst &k, const f
     default: QLSKUM_FLUX(128, 4); break;
     }
 #undef QLSKUM_FLUX
-#undef QLSKUM_FLUX_L
 #undef QLSKUM_FLUX_ST
 #undef QLSKUM_FLUX_RP
 #undef QLSKUM_FLUX_RPS
