@@ -271,17 +271,21 @@ __device__ __forceinline__ double edge_dt(double dist, double speed, double cfl)
 // that the module, fused and recording kernels, whatever the compiler inlines
 // around them, give the same bits.
 
-// q_variables_mod.h:19-33
-__device__ __forceinline__ void q_of(const double P[4], double Q[4])
+__device__ __forceinline__ double beta_of(const double P[4]) { return ratio64(0.5 * P[0], P[3]); }
+
+// q_variables_mod.h:19-33, with log(rho) and log(beta) given
+__device__ __forceinline__ void q_of(const double P[4], double log_rho, double log_beta, double Q[4])
 {
-    const double beta = ratio64(0.5 * P[0], P[3]);
+    const double beta = beta_of(P);
     const double usq = fma(P[1], P[1], __dmul_rn(P[2], P[2]));
-    Q[0] = fma(-beta, usq, fma(2.5, log(beta), log(P[0])));
+    Q[0] = fma(-beta, usq, fma(2.5, log_beta, log_rho));
     const double b2 = 2.0 * beta;
     Q[1] = b2 * P[1];
     Q[2] = b2 * P[2];
     Q[3] = -b2;
 }
+
+__device__ __forceinline__ void q_of(const double P[4], double Q[4]) { q_of(P, log(P[0]), log(beta_of(P)), Q); }
 
 // |u| + 3 sqrt(p / rho) of state_update_mod.h:483-485
 __device__ __forceinline__ double wave_speed(const double P[4])
