@@ -239,11 +239,12 @@ def measured_profile(workload, precision, kernel, key="traffic"):
 
 def flux_kernel_form(variant: int) -> str:
     """Kernel name of a mixed flux_variant (as qlskum_set_launch_config numbers
-    them): 4..7 staged gathers, 10..13 register prefetch, 14..18 register
-    prefetch with the owner's data in shared memory, else per-edge gathers."""
+    them): 4..7 staged gathers, 8..13 register prefetch (8, 9 with 2 / 4 lanes
+    per point), 14..18 register prefetch with the owner's data in shared
+    memory, else per-edge gathers."""
     if 4 <= variant <= 7:
         return "k_flux_update_st"
-    if 10 <= variant <= 13:
+    if 8 <= variant <= 13:
         return "k_flux_update_rp"
     if 14 <= variant <= 18:
         return "k_flux_update_rps"
@@ -782,11 +783,12 @@ def main():
     achieved = nbytes / (fl_ms / fl_n / 1e3) / 1e9
     lc = solver.launch_config()
     kname = (f"{flux_kernel_form(lc['flux_variant'])}<{lc['flux_block']},{lc['flux_min_blocks']}>"
-             if prec == qlskum.MIXED else "k_flux_update<128>")
+             if prec == qlskum.MIXED else "fp64::k_flux_update")
     traffic, traffic_kernel = measured_traffic(args.workload, args.precision, kname)
     # every per-stage kernel against HBM (event-timed launches, compulsory
     # bytes), with its ncu DRAM traffic per launch where a committed summary has it
-    names = {"gradient": "k_q_derivatives", "inner": "k_q_inner", "flux_update": kname}
+    ring = prec == qlskum.MIXED and lc["point_lanes"] == 1 and lc["gather_depth"] == 0
+    names = {"gradient": "k_q_derivatives_ring" if ring else "k_q_derivatives", "inner": "k_q_inner", "flux_update": kname}
     kernels = {}
     for kk in ("gradient", "inner", "flux_update"):
         ms, nl = kt[kk]

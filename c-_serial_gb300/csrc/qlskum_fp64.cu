@@ -8,10 +8,12 @@
 // results differ from the serial reference by those roundings: 1e-10 relative
 // after 1000 iterations (the parity tests).
 //
-// One thread per point, or in the flux kernels several (flux_shape); a point's
+// Four lanes per point (one per component) in the gradient kernels, several
+// threads per point in the flux kernels (flux_shape), one elsewhere; a point's
 // edges are summed in the reference's neighbour order, read from the
-// sliced-ELL edge arrays (coalesced across the warp); neighbour state is gathered through L1/L2 (points are Morton ordered, so
-// most neighbours of a block's points are cache-resident).  All geometry that
+// sliced-ELL edge arrays (coalesced across the warp); neighbour state is
+// gathered through L1/L2 (points are Morton ordered, so most neighbours of a
+// block's points are cache-resident).  All geometry that
 // does not change between iterations (edge vectors, least-squares moments,
 // 1/det, limiter epsilon) is precomputed on the host in the reference's
 // operation order, which on this chip trades a few bytes per edge for FP64
@@ -696,9 +698,10 @@ __global__ void __launch_bounds__(256) k_stagnation(int n, const double4_32a *__
 // Measured per launch (us, inner 0):
 //   points                       960  9,600  30,720  51,200  102,400  204,800
 //   a thread per point           228    217     281     329      649     1061
-//   8 per block, 128 threads      34     81     210     331      645     1260
-//   16                            45     86     182     277      524     1012
-//   32                            68     90     209     281      507      951
+//   8 per block, 128 threads      32     75     193     305      596     1163
+//   16                            42     79     169     261      493      946
+//   32                            64     85     196     262      479      898
+// (the first row before the shorter quotient and reciprocals, 6% on the others).
 template <typename F> void flux_shape(int n, F &&launch)
 {
     using std::integral_constant;
