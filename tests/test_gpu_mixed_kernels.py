@@ -58,3 +58,24 @@ def test_edge_lists_past_l2(lanes, power):
         out += [b.prim(k) for k in range(cases)]
     for p in out[1:]:
         assert np.array_equal(out[0], p)
+
+
+@pytest.mark.parametrize("wall, layers", [(40, 12), (49, 21), (64, 40), (257, 259)])
+def test_residual_of_few_and_many_partials(wall, layers):
+    """2 to 1,041 block partials (64, 128 and 256 points per block) of the same
+    state: the sum in FP64 moves by at most 1,041 roundings of 2^-53 and the maximum not at all."""
+    import qlskum
+    from conftest import small_cloud
+    from qlskum import cloudgen
+    c = small_cloud(wall, layers) if wall < 60 else cloudgen.make_cloud(n_wall=wall, n_layers=layers, seed=3)
+    out = []
+    for variant in (2, 0, 3):
+        s = qlskum.Solver(c, mach=0.63, aoa=2.0, cfl=0.2, vl_const=50.0, inner_iterations=0, precision=qlskum.MIXED)
+        s.set_launch_config(variant, 128, 0)
+        rng = np.random.default_rng(2)
+        s.set_prim(s.prim * (1.0 + 1e-2 * rng.standard_normal((c.n, 4))))
+        s.q_lskum(1)
+        out.append((s.prim, s.residual_history()[0]))
+    for prim, h in out[1:]:
+        assert np.array_equal(prim, out[0][0])
+        assert abs(h[0] / out[0][1][0] - 1.0) <= 1041 * 2.0 ** -53 and h[2] == out[0][1][2]
