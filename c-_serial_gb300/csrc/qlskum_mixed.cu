@@ -1073,6 +1073,9 @@ __global__ void k_q_inner(DevCloud c, const float4 *__restrict__ dq0, const floa
 // twice the bytes and streams 20 instead of 12 per edge, gains nothing there
 // (55.7 and 55.5: 275 MB with the write-back, 5 TB/s) and keeps its form.
 constexpr int kRingEdges = 5, kRingChunks = 2;
+// Most warps of a block, whose barriers have their place in static shared
+// memory; a launch of larger blocks (block_size up to 1,024) takes blocks of this many.
+constexpr int kRingWarps = 16;
 
 template <int NA> struct EdgeRing {
     static constexpr int CE = kRingEdges, NS = kRingChunks;
@@ -1156,6 +1159,7 @@ template <int NA> struct EdgeRing {
     {
         if (mbar_wait(bar + 8 * stage, phase)) return true;
         if (c.fault) *c.fault = 2;
+        static_assert(NS == 2, "the other chunk in flight is named by stage ^ 1");
         mbar_wait(bar + 8 * (stage ^ 1), stage ? phase ^ 1 : phase);
         return false;
     }
@@ -1179,7 +1183,7 @@ __global__ void k_q_derivatives_ring(DevCloud c, const float4 *__restrict__ q, f
 {
     constexpr int CE = kRingEdges, NS = kRingChunks;
     extern __shared__ __align__(128) unsigned char ring_smem[];
-    __shared__ unsigned long long bars[16 * NS];
+    __shared__ unsigned long long bars[kRingWarps * NS];
     constexpr int NA = DT ? 3 : 2, PB = DT ? 16 : 12;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     unsigned char *buf = ring_smem + warp * (NS * CE * 32 * PB);
@@ -1475,15 +1479,15 @@ void q_derivatives(const Launch &L, const DevCloud &c, const float4 *q, float4 *
             else
                 launch_after(L, k_q_derivatives_st<B_, D_, false>, grid_for(c.n, B_), B_, staged_bytes(B_, D_, 2, c.max_nb, true), c, q, dq, qm, cspeed, delta, cfl))
     } else if (L.lanes == 1) {
-        const int g = ring_grid(c.n, L.block, 24);
+        const int block = std::min(L.block, 32 * kRingWarps), g = ring_grid(c.n, block, 24);
         if (delta) {
-            const size_t sm = ring_bytes(L.block, 16);
+            const size_t sm = ring_bytes(block, 16);
             allow_smem(k_q_derivatives_ring<true>, sm);
-            launch_after(L, k_q_derivatives_ring<true>, g, L.block, sm, c, q, dq, qm, cspeed, delta, cfl);
+            launch_after(L, k_q_derivatives_ring<true>, g, block, sm, c, q, dq, qm, cspeed, delta, cfl);
         } else {
-            const size_t sm = ring_bytes(L.block, 12);
+            const size_t sm = ring_bytes(block, 12);
             allow_smem(k_q_derivatives_ring<false>, sm);
-            launch_after(L, k_q_derivatives_ring<false>, g, L.block, sm, c, q, dq, qm, nullptr, nullptr, cfl);
+            launch_after(L, k_q_derivatives_ring<false>, g, block, sm, c, q, dq, qm, nullptr, nullptr, cfl);
         }
     } else {
 #define QLSKUM_GRAD(LN, ST)                                                                                     \
