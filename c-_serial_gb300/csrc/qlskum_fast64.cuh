@@ -35,32 +35,40 @@ __device__ __forceinline__ bool within_cut(double x)
     return (__double_as_longlong(x) & 0x7fffffffffffffffLL) <= __double_as_longlong(10e-6);
 }
 
-// A finite seed that FP32 holds as a normal number.
-__device__ __forceinline__ bool seed_ok(float s) { return fabsf(s) > 1e-37f && fabsf(s) < 1e37f; }
+// Not so small that its low parts, 2^-46 of it, leave FP32's normal range.
+__device__ __forceinline__ bool large_enough(float x) { return fabsf(x) > 1e-24f; }
 
-static __device__ __noinline__ double div_slow(double a, double b) { return a / b; }
+// a / b; a zero numerator, which the limiter has at every extremum where eps^2 = 0, off the FP64 pipe.
+static __device__ __noinline__ double div_slow(double a, double b)
+{
+    if ((__double_as_longlong(a) << 1) == 0 && abs_hi(b) - 0x00100000u < 0x7fe00000u)  // b normal
+        return flip(a, (unsigned)__double2hiint(b) & 0x80000000u);
+    return a / b;
+}
 static __device__ __noinline__ double rsqrt_slow(double x) { return rsqrt(x); }
 static __device__ __noinline__ double exp32_slow(double x) { return 32.0 * exp(x); }
 static __device__ __noinline__ double2 gauss_erf_slow(double s) { return make_double2(1.1283791670955126 * exp(-s * s), erf(s)); }
 
-// The 29 low mantissa bits of x that d2f(x) cuts off, as a float (x normal
-// and within FP32's range; below about 1e-30 it may flush to zero).
+// The 29 low mantissa bits of x that d2f(x) cuts off, as a float (d2f(x)
+// normal; a rest below FP32's normal range may flush to zero).
 __device__ __forceinline__ float d2f_rest(double x)
 {
     const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x) & 0x1fffffffu;
-    // 2^(e - 52) = the float of exponent e, times 2^-52
-    const float ulp = __uint_as_float((((h >> 20) & 0x7ffu) - 896u) << 23) * 2.220446049250313e-16f;
-    return copysignf((float)l, __uint_as_float(h)) * ulp;
+    // 2^-52 first: the product with 2^e, the float of x's exponent, is then exact wherever it is normal
+    return copysignf((float)l, __uint_as_float(h)) * 2.220446049250313e-16f * __uint_as_float((((h >> 20) & 0x7ffu) - 896u) << 23);
 }
 
 // num / den for finite num, den > 0: the quotient to 2^-44 from FP32 (hi and
-// rest of both), corrected once by its FP64 remainder.
+// rest of both), corrected once by its FP64 remainder.  A numerator (the
+// limiter's is eps^2 alone at an extremum), denominator or quotient whose rests
+// FP32 cannot hold takes the division; so do zero, overflow, Inf and NaN.
 __device__ __forceinline__ double ratio64(double num, double den)
 {
     const float dh = d2f(den), nh = d2f(num);
     const float r = __fdividef(1.0f, dh);
     const float q = nh * r;
-    if (!seed_ok(r) || !(fabsf(q) < 1e37f)) return div_slow(num, den);
+    if (!(fabsf(r) > 1e-37f && fabsf(r) < 1e24f && large_enough(nh) && large_enough(q) && fabsf(q) < 1e37f))
+        return div_slow(num, den);
     const float res = fmaf(-dh, q, nh) + fmaf(-d2f_rest(den), q, d2f_rest(num));
     const double v = f2d(q) + f2d(res * r);
     return fma(fma(-den, v, num), f2d(r), v);
@@ -72,7 +80,7 @@ __device__ __forceinline__ double ratio64(double num, double den)
 __device__ __forceinline__ void rsqrt_rcp(double x, double &r, double &h)
 {
     const float s = rsqrtf(d2f(x));
-    if (!seed_ok(s)) {
+    if (!(s > 1e-18f && s < 1e18f)) {  // x, whose root this is, is a normal float
         r = rsqrt_slow(x);
         h = div_slow(1.0, x);
         return;

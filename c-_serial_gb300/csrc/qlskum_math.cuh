@@ -25,7 +25,8 @@
 
 namespace qlskum {
 
-#ifdef __CUDACC__
+// (QLSKUM_HOST_INTRINSICS: a host build that has defined the intrinsics used here.)
+#if defined(__CUDACC__) || defined(QLSKUM_HOST_INTRINSICS)
 // Conversions between FP32 and FP64 on the integer pipe (the hardware
 // conversion issues on the FP64 pipe, which on this chip is the scarce one).
 // float -> double: exact for normal numbers and zero, flushes subnormals to

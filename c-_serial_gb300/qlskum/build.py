@@ -17,10 +17,11 @@ library with a C ABI (include/qlskum.h):
 * csrc/qlskum_io.cpp -- partGrid file I/O and the sub-stencil quality check
   (host only, no GPU needed).
 
-`build_vjp_host()` compiles a separate, test-only library
-(tests/vjp_host/qlskum_vjp_host.cpp -> tests/_build/libqlskum_vjp_host.so):
-the per-point arithmetic and its reverse mode compiled for the host, for
-derivative checks without a GPU.  It is not part of libqlskum.so.
+`build_vjp_host()` and `build_fast64_host()` compile separate, test-only
+libraries (tests/vjp_host/qlskum_vjp_host.cpp and
+tests/fast64_host/qlskum_fast64_host.cpp -> tests/_build/): the per-point
+arithmetic, its reverse mode and the FP64 form's fast functions compiled for
+the host, for checks without a GPU.  They are not part of libqlskum.so.
 
 Output: c-_serial_gb300/_build/libqlskum.so (git-ignored; rebuilt on the GPU
 machine because binaries do not travel between architectures).
@@ -121,25 +122,33 @@ def build(force: bool = False, verbose: bool = False, ptxas_info: bool = False) 
     return LIB
 
 
-VJP_SRC = os.path.join(REPO, "tests", "vjp_host", "qlskum_vjp_host.cpp")
-VJP_LIB = os.path.join(REPO, "tests", "_build", "libqlskum_vjp_host.so")
+def _build_host_test(name: str) -> str:
+    """Compile the test-only host library tests/<name>/qlskum_<name>.cpp (g++,
+    no GPU needed) if missing or stale; return its path."""
+    src = os.path.join(REPO, "tests", name, f"qlskum_{name}.cpp")
+    lib = os.path.join(REPO, "tests", "_build", f"libqlskum_{name}.so")
+    deps = [src] + [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
+    if os.path.exists(lib) and all(os.path.getmtime(p) <= os.path.getmtime(lib) for p in deps):
+        return lib
+    os.makedirs(os.path.dirname(lib), exist_ok=True)
+    tmp = lib + f".tmp{os.getpid()}"
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-ffp-contract=off", "-Wall", "-Wno-unused-function",
+           "-I", INCLUDE, "-I", CSRC, "-I", _cuda_include(_nvcc()), src, "-o", tmp]
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"building the host test library {name} failed:\n" + " ".join(cmd) + "\n" + r.stdout)
+    os.replace(tmp, lib)
+    return lib
 
 
 def build_vjp_host() -> str:
-    """Compile the test-only host build of the per-point reverse arithmetic
-    (g++, no GPU needed) if missing or stale; return its path."""
-    deps = [VJP_SRC] + [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))]
-    if os.path.exists(VJP_LIB) and all(os.path.getmtime(p) <= os.path.getmtime(VJP_LIB) for p in deps):
-        return VJP_LIB
-    os.makedirs(os.path.dirname(VJP_LIB), exist_ok=True)
-    tmp = VJP_LIB + f".tmp{os.getpid()}"
-    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-ffp-contract=off", "-Wall", "-Wno-unused-function",
-           "-I", INCLUDE, "-I", CSRC, "-I", _cuda_include(_nvcc()), VJP_SRC, "-o", tmp]
-    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
-    if r.returncode != 0:
-        raise RuntimeError("building the host VJP test library failed:\n" + " ".join(cmd) + "\n" + r.stdout)
-    os.replace(tmp, VJP_LIB)
-    return VJP_LIB
+    """The host build of the per-point reverse arithmetic."""
+    return _build_host_test("vjp_host")
+
+
+def build_fast64_host() -> str:
+    """The host build of the FP64 form's fast functions."""
+    return _build_host_test("fast64_host")
 
 
 if __name__ == "__main__":
