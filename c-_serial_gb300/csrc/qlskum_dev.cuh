@@ -71,7 +71,8 @@ __device__ __forceinline__ bool mbar_try(unsigned bar, unsigned phase)
 }
 
 // Waits for the barrier's phase; false if it has not completed after a second
-// (a bound on the wait, not expected).
+// (a bound on the wait, not expected).  The first tries are without a look at
+// the clock (with one the mixed gradient takes 42.9 instead of 41.4 us on 1.02 M points).
 __device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned phase)
 {
     for (int t = 0; t < 1024; t++)

@@ -87,12 +87,36 @@ struct DeviceArena {
         ptrs.push_back(p);
         return static_cast<T *>(p);
     }
+    // The word of DevCloud::fault, in pinned host memory: the host reads it after
+    // any wait for the kernels without a copy.
+    int *fault = nullptr;
+    int *alloc_fault()
+    {
+        void *p = nullptr, *d = nullptr;
+        cudaError_t e = cudaHostAlloc(&p, sizeof(int), cudaHostAllocMapped);
+        if (e == cudaSuccess) {
+            fault = static_cast<int *>(p);
+            *fault = 0;
+            e = cudaHostGetDevicePointer(&d, p, 0);
+        }
+        if (e != cudaSuccess) err = e;
+        return static_cast<int *>(d);
+    }
+    bool faulted() const { return fault && *static_cast<volatile int *>(fault) != 0; }
+    void clear_fault()
+    {
+        if (fault) *static_cast<volatile int *>(fault) = 0;
+    }
     void release()
     {
         for (void *p : ptrs) cudaFree(p);
         ptrs.clear();
+        if (fault) cudaFreeHost(fault);
+        fault = nullptr;
     }
 };
+
+const char kLostCopy[] = "a bulk copy of the edge lists did not complete";
 
 struct qlskum_handle {
     qlskum_params prm{};
@@ -164,6 +188,20 @@ qlskum_status cuda_fail(qlskum_handle *h, cudaError_t e, const char *where)
     do {                                                     \
         cudaError_t e_ = (call);                             \
         if (e_ != cudaSuccess) return cuda_fail(h, e_, #call); \
+    } while (0)
+
+// Waits for the handle's kernels.  Every call that hands results to the caller
+// does so, and fails if one of those kernels gave up on a bulk copy.
+qlskum_status wait_kernels(qlskum_handle *h)
+{
+    CK(h, cudaStreamSynchronize(h->L.stream));
+    if (h->arena.faulted()) return fail(h, QLSKUM_ERR_CUDA, kLostCopy);
+    return QLSKUM_OK;
+}
+
+#define WAIT(h)                                       \
+    do {                                              \
+        if (qlskum_status s_ = wait_kernels(h)) return s_; \
     } while (0)
 
 qlskum_status check_launch(qlskum_handle *h, const char *where)
@@ -616,7 +654,7 @@ qlskum_status print_iters(qlskum_handle *h, int from, int to)
     std::vector<double> hist((size_t)3 * (size_t)(to - from));
     CK(h, cudaMemcpyAsync(hist.data(), h->R.hist + 3 * (size_t)from, sizeof(double) * hist.size(),
                           cudaMemcpyDeviceToHost, h->L.stream));
-    CK(h, cudaStreamSynchronize(h->L.stream));
+    WAIT(h);
     for (int t = from; t < to; t++) printf("iterations %d residue : %.13e\n", t + 1, hist[3 * (size_t)(t - from) + 1]);
     fflush(stdout);
     return QLSKUM_OK;
@@ -626,8 +664,7 @@ qlskum_status check_status(qlskum_handle *h)
 {
     int st = 0;
     CK(h, cudaMemcpyAsync(&st, h->R.status, sizeof(int), cudaMemcpyDeviceToHost, h->L.stream));
-    CK(h, cudaStreamSynchronize(h->L.stream));
-    if (st == 2) return fail(h, QLSKUM_ERR_CUDA, "a bulk copy of the edge lists did not complete");
+    WAIT(h);
     if (st) return fail(h, QLSKUM_ERR_NONFINITE, "residual became non-finite (NaN/Inf in the state)");
     return QLSKUM_OK;
 }
@@ -1022,7 +1059,7 @@ qlskum_status qlskum_create(const qlskum_cloud *c, const qlskum_params *p, qlsku
     h->R.res_old = A.alloc<double>(1);
     h->R.iter = A.alloc<int>(1);
     h->R.status = A.alloc<int>(1);
-    h->dc.fault = h->R.status;
+    if (p->precision == QLSKUM_MIXED) h->dc.fault = A.alloc_fault();
     h->d_obj = A.alloc<double>(8);
     h->d_obj_partial = A.alloc<double>(4 * (size_t)((std::max(n, sp) + 255) / 256));
     h->d_entropy = A.alloc<double>(h->np);
@@ -1226,7 +1263,7 @@ qlskum_status qlskum_q_lskum(qlskum_handle *h, int iters)
     if (st) return st;
     // the device counter continues from the host's
     CK(h, cudaMemcpyAsync(h->R.iter, &h->it, sizeof(int), cudaMemcpyHostToDevice, h->L.stream));
-    CK(h, cudaStreamSynchronize(h->L.stream));
+    WAIT(h);
     if (!h->timing && iters > 0 && (st = ensure_graphs(h))) return st;
     for (int t = 0; t < iters; t++) {
         const int o = h->pcur;
@@ -1262,7 +1299,7 @@ qlskum_status qlskum_objective(qlskum_handle *h, double *cl, double *cd, double 
     if (st) return st;
     double o[4];
     CK(h, cudaMemcpyAsync(o, h->d_obj, sizeof o, cudaMemcpyDeviceToHost, h->L.stream));
-    CK(h, cudaStreamSynchronize(h->L.stream));
+    WAIT(h);
     const double H = o[0], V = o[1];
     if (cl) *cl = V * std::cos(h->K.theta) - H * std::sin(h->K.theta);
     if (cd) *cd = H * std::cos(h->K.theta) + V * std::sin(h->K.theta);
@@ -1315,11 +1352,11 @@ qlskum_status qlskum_get_field(qlskum_handle *h, int field, double *out)
     if (f32) {
         std::vector<float> d32((size_t)n * width);
         CK(h, cudaMemcpyAsync(d32.data(), src, sizeof(float) * d32.size(), cudaMemcpyDeviceToHost, h->L.stream));
-        CK(h, cudaStreamSynchronize(h->L.stream));
+        WAIT(h);
         for (size_t t = 0; t < d32.size(); t++) dev[t] = d32[t];
     } else {
         CK(h, cudaMemcpyAsync(dev.data(), src, sizeof(double) * dev.size(), cudaMemcpyDeviceToHost, h->L.stream));
-        CK(h, cudaStreamSynchronize(h->L.stream));
+        WAIT(h);
     }
     unpermute(h, dev, out, width);
     return QLSKUM_OK;
@@ -1357,7 +1394,7 @@ qlskum_status qlskum_get_prim(qlskum_handle *h, double *out)
     if (st) return st;
     fp64::permute_out(h->L, h->n, h->d_perm, h->s64.prim[h->pcur], h->d_stage);
     CK(h, cudaMemcpyAsync(out, h->d_stage, sizeof(double4_32a) * (size_t)h->n, cudaMemcpyDeviceToHost, h->L.stream));
-    CK(h, cudaStreamSynchronize(h->L.stream));
+    WAIT(h);
     return QLSKUM_OK;
 }
 
@@ -1370,9 +1407,10 @@ qlskum_status qlskum_set_prim(qlskum_handle *h, const double *prim)
     CK(h, cudaMemcpyAsync(h->d_stage, prim, sizeof(double4_32a) * (size_t)h->n, cudaMemcpyHostToDevice, h->L.stream));
     // padding rows of the state keep the finite values they were created with
     fp64::permute_in(h->L, h->n, h->d_perm, h->d_stage, h->s64.prim[h->pcur]);
-    // a new state clears a non-finite flag raised by the old one
+    // a new state clears a non-finite flag or a fault raised by the old one
     CK(h, cudaMemsetAsync(h->R.status, 0, sizeof(int), h->L.stream));
     CK(h, cudaStreamSynchronize(h->L.stream));
+    h->arena.clear_fault();
     h->derived_valid = false;
     return QLSKUM_OK;
 }
@@ -1393,7 +1431,7 @@ qlskum_status qlskum_get_residual_history(qlskum_handle *h, double *out, int max
     int m = std::min(cnt, std::max(max_rows, 0));
     if (out && m > 0) {
         CK(h, cudaMemcpyAsync(out, h->R.hist, sizeof(double) * 3 * (size_t)m, cudaMemcpyDeviceToHost, h->L.stream));
-        CK(h, cudaStreamSynchronize(h->L.stream));
+        WAIT(h);
     }
     return QLSKUM_OK;
 }
@@ -1408,7 +1446,7 @@ qlskum_status qlskum_get_iteration(qlskum_handle *h, int *it)
 qlskum_status qlskum_synchronize(qlskum_handle *h)
 {
     NEED(h);
-    CK(h, cudaStreamSynchronize(h->L.stream));
+    WAIT(h);
     return QLSKUM_OK;
 }
 
@@ -1551,6 +1589,14 @@ qlskum_status bfail(qlskum_batch *b, qlskum_status s, const std::string &msg)
         cudaError_t e_ = (call);                                                                        \
         if (e_ != cudaSuccess) return bfail(b, QLSKUM_ERR_CUDA, fmt("%s: %s", #call, cudaGetErrorString(e_))); \
     } while (0)
+
+// As wait_kernels().
+qlskum_status batch_wait(qlskum_batch *b)
+{
+    BCK(b, cudaStreamSynchronize(b->L.stream));
+    if (b->arena.faulted()) return bfail(b, QLSKUM_ERR_CUDA, kLostCopy);
+    return QLSKUM_OK;
+}
 
 
 // Points of each flux block of a variant (its threads over its lanes per point).
@@ -1851,7 +1897,7 @@ qlskum_status qlskum_batch_create(const qlskum_cloud *clouds, int n_clouds, cons
     b->pmax = A.alloc<double>(T / 64);
     b->d_iter = A.alloc<int>(1);
     b->d_status = A.alloc<int>(1);
-    b->sc.fault = b->d_status;
+    b->sc.fault = A.alloc_fault();
     b->res_old = A.alloc<double>(n_cases);
     b->res_new = A.alloc<double>(n_cases);
     b->d_obj = A.alloc<double>(4 * (size_t)n_cases);
@@ -1933,8 +1979,7 @@ qlskum_status qlskum_batch_run(qlskum_batch *b, int iters)
     }
     int status = 0;
     BCK(b, cudaMemcpyAsync(&status, b->d_status, sizeof(int), cudaMemcpyDeviceToHost, b->L.stream));
-    BCK(b, cudaStreamSynchronize(b->L.stream));
-    if (status == 2) return bfail(b, QLSKUM_ERR_CUDA, "a bulk copy of the edge lists did not complete");
+    if (qlskum_status s_ = batch_wait(b)) return s_;
     if (status) return bfail(b, QLSKUM_ERR_NONFINITE, "a case's residual became non-finite");
     return QLSKUM_OK;
 }
@@ -1952,7 +1997,7 @@ qlskum_status qlskum_batch_objective(qlskum_batch *b, double *cl, double *cd, do
     }
     std::vector<double> o(4 * (size_t)nc);
     BCK(b, cudaMemcpyAsync(o.data(), b->d_obj, sizeof(double) * o.size(), cudaMemcpyDeviceToHost, b->L.stream));
-    BCK(b, cudaStreamSynchronize(b->L.stream));
+    if (qlskum_status s_ = batch_wait(b)) return s_;
     for (int c = 0; c < nc; c++) {
         const double H = o[4 * c], V = o[4 * c + 1], th = b->cases[c].K.theta;
         if (cl) cl[c] = V * std::cos(th) - H * std::sin(th);
@@ -1973,7 +2018,7 @@ qlskum_status qlskum_batch_get_prim(qlskum_batch *b, int case_index, double *out
     std::vector<double> dev(4 * (size_t)C.n);
     BCK(b, cudaMemcpyAsync(dev.data(), b->prim[b->pcur] + C.off, sizeof(double) * dev.size(), cudaMemcpyDeviceToHost,
                            b->L.stream));
-    BCK(b, cudaStreamSynchronize(b->L.stream));
+    if (qlskum_status s_ = batch_wait(b)) return s_;
     for (int p = 0; p < C.n; p++) std::memcpy(out + 4 * (size_t)G.iperm[p], dev.data() + 4 * (size_t)p, 32);
     return QLSKUM_OK;
 }
@@ -1987,7 +2032,7 @@ qlskum_status qlskum_batch_residual_history(qlskum_batch *b, double *out, int ma
     if (out && m > 0) {
         BCK(b, cudaMemcpyAsync(out, b->hist, sizeof(double) * b->cases.size() * (size_t)m, cudaMemcpyDeviceToHost,
                                b->L.stream));
-        BCK(b, cudaStreamSynchronize(b->L.stream));
+        if (qlskum_status s_ = batch_wait(b)) return s_;
     }
     return QLSKUM_OK;
 }
@@ -2335,9 +2380,12 @@ qlskum_status part_derived(qlskum_partition *P)
     return QLSKUM_OK;
 }
 
-qlskum_status part_sync(qlskum_partition *P)
+qlskum_status part_sync(qlskum_partition *P, bool new_state = false)
 {
     for (PartDev *d : P->parts) PCK(P, cudaStreamSynchronize(d->L.stream));
+    // a new state clears a fault raised by the old one
+    if (new_state) P->A.clear_fault();
+    if (P->A.faulted()) return pfail(P, QLSKUM_ERR_CUDA, kLostCopy);
     return QLSKUM_OK;
 }
 
@@ -2552,7 +2600,10 @@ qlskum_status qlskum_partition_create(const qlskum_cloud *c, const qlskum_params
     P->R.res_old = P->A.alloc<double>(1);
     P->R.iter = P->A.alloc<int>(1);
     P->R.status = P->A.alloc<int>(1);
-    for (PartDev *d : P->parts) d->G.dc.fault = P->R.status;
+    if (mx) {
+        int *fault = P->A.alloc_fault();
+        for (PartDev *d : P->parts) d->G.dc.fault = fault;
+    }
     if (P->A.err != cudaSuccess) {
         part_free(P);
         return fail(nullptr, QLSKUM_ERR_CUDA, fmt("cudaMalloc: %s", cudaGetErrorString(P->A.err)));
@@ -2651,7 +2702,6 @@ qlskum_status qlskum_partition_q_lskum(qlskum_partition *P, int iters)
     if (st) return st;
     int bad = 0;
     PCK(P, cudaMemcpy(&bad, P->R.status, sizeof(int), cudaMemcpyDeviceToHost));
-    if (bad == 2) return pfail(P, QLSKUM_ERR_CUDA, "a bulk copy of the edge lists did not complete");
     if (bad) return pfail(P, QLSKUM_ERR_NONFINITE, "residual became non-finite (NaN/Inf in the state)");
     return QLSKUM_OK;
 }
@@ -2676,7 +2726,7 @@ qlskum_status qlskum_partition_get_prim(qlskum_partition *P, double *out)
 qlskum_status qlskum_partition_set_prim(qlskum_partition *P, const double *prim)
 {
     if (!P || !prim) return QLSKUM_ERR_INVALID;
-    qlskum_status st = part_sync(P);
+    qlskum_status st = part_sync(P, true);
     if (st) return st;
     for (PartDev *d : P->parts) {
         const size_t ns = d->spec.local.size() + d->spec.ghost.size();
@@ -2719,6 +2769,7 @@ qlskum_status qlskum_partition_objective(qlskum_partition *P, double *cl, double
         PCK(P, cudaStreamSynchronize(d->L.stream));
         for (int j = 0; j < 4; j++) sum[j] += o[j];
     }
+    if (P->A.faulted()) return pfail(P, QLSKUM_ERR_CUDA, kLostCopy);
     const double H = sum[0], V = sum[1];
     if (cl) *cl = V * std::cos(P->K.theta) - H * std::sin(P->K.theta);
     if (cd) *cd = H * std::cos(P->K.theta) + V * std::sin(P->K.theta);
@@ -2755,7 +2806,7 @@ qlskum_status stagnation_values(qlskum_handle *h, const double4_32a *prim, Stagn
     const int blocks = (h->n + 255) / 256;
     std::vector<double> part(6 * (size_t)blocks);
     CK(h, cudaMemcpyAsync(part.data(), h->d_diag, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, h->L.stream));
-    CK(h, cudaStreamSynchronize(h->L.stream));
+    WAIT(h);
     sv.p0_min = part[0];
     sv.p0_max = part[2];
     sv.i_min = (long long)part[1];
@@ -2777,7 +2828,7 @@ qlskum_status download_prim(qlskum_handle *h, std::vector<double4_32a> &dev)
     dev.resize(h->np);
     CK(h, cudaMemcpyAsync(dev.data(), h->s64.prim[h->pcur], sizeof(double4_32a) * h->np, cudaMemcpyDeviceToHost,
                           h->L.stream));
-    CK(h, cudaStreamSynchronize(h->L.stream));
+    WAIT(h);
     return QLSKUM_OK;
 }
 
@@ -2794,7 +2845,7 @@ qlskum_status write_state(qlskum_handle *h, const char *path, bool restart_order
     double res_old = 0.0;
     CK(h, cudaMemcpyAsync(ent.data(), h->d_entropy, sizeof(double) * h->np, cudaMemcpyDeviceToHost, h->L.stream));
     CK(h, cudaMemcpyAsync(&res_old, h->R.res_old, sizeof(double), cudaMemcpyDeviceToHost, h->L.stream));
-    CK(h, cudaStreamSynchronize(h->L.stream));
+    WAIT(h);
     FILE *f = std::fopen(path, "w");
     if (!f) return fail(h, QLSKUM_ERR_INVALID, fmt("cannot open %s", path));
     std::fprintf(f, "%d %d %.17g\n", h->n, h->it, res_old);
@@ -2833,7 +2884,7 @@ qlskum_status qlskum_enstrophy(qlskum_handle *h, double *total, double *vorticit
         vort.resize(h->np);
         CK(h, cudaMemcpyAsync(vort.data(), h->d_vort, sizeof(double) * h->np, cudaMemcpyDeviceToHost, h->L.stream));
     }
-    CK(h, cudaStreamSynchronize(h->L.stream));
+    WAIT(h);
     double t = 0.0;
     for (double v : part) t += v;
     if (total) *total = t;
@@ -2895,7 +2946,7 @@ qlskum_status qlskum_read_restart(qlskum_handle *h, const char *path)
     if (st) return st;
     h->it = (int)itr;
     CK(h, cudaMemcpyAsync(h->R.res_old, &res_old, sizeof(double), cudaMemcpyHostToDevice, h->L.stream));
-    CK(h, cudaStreamSynchronize(h->L.stream));
+    WAIT(h);
     // fpi_solver_mod.h:139: a restarted run keeps the file's res_old
     h->R.latch = 0;
     h->restarted = true;
@@ -3021,10 +3072,19 @@ std::vector<long long> slice_bases(const qlskum_handle *h, size_t *ne)
     return sb;
 }
 
+// A read of the cloud's constants.
 qlskum_status d2h(qlskum_handle *h, void *dst, const void *src, size_t bytes)
 {
     CK(h, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, h->L.stream));
     CK(h, cudaStreamSynchronize(h->L.stream));
+    return QLSKUM_OK;
+}
+
+// A read of what the kernels computed.
+qlskum_status read_result(qlskum_handle *h, void *dst, const void *src, size_t bytes)
+{
+    CK(h, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, h->L.stream));
+    WAIT(h);
     return QLSKUM_OK;
 }
 
@@ -3517,7 +3577,7 @@ qlskum_status adj_seed(qlskum_handle *h, int which, const double4_32a *prim, dou
                     which, bP);
     if ((st = check_launch(h, "adjoint seed"))) return st;
     double v[4];
-    if ((st = d2h(h, v, h->d_obj, sizeof v))) return st;
+    if ((st = read_result(h, v, h->d_obj, sizeof v))) return st;
     const double cl = v[1] * std::cos(h->K.theta) - v[0] * std::sin(h->K.theta);
     const double cd = v[0] * std::cos(h->K.theta) + v[1] * std::sin(h->K.theta);
     o.J = which == QLSKUM_OBJECTIVE_CL ? cl : cd;
@@ -3563,10 +3623,10 @@ qlskum_status adj_geometry(qlskum_handle *h, int which, const double4_32a *prim_
     std::vector<double> gx(np), gy(np);
     std::vector<double2> gn(np);
     std::vector<double4_32a> prim(np);
-    if ((st = d2h(h, gx.data(), a->gbx, sizeof(double) * np))) return st;
-    if ((st = d2h(h, gy.data(), a->gby, sizeof(double) * np))) return st;
-    if ((st = d2h(h, gn.data(), a->gbn, sizeof(double2) * np))) return st;
-    if ((st = d2h(h, prim.data(), prim_dev, sizeof(double4_32a) * np))) return st;
+    if ((st = read_result(h, gx.data(), a->gbx, sizeof(double) * np))) return st;
+    if ((st = read_result(h, gy.data(), a->gby, sizeof(double) * np))) return st;
+    if ((st = read_result(h, gn.data(), a->gbn, sizeof(double2) * np))) return st;
+    if ((st = read_result(h, prim.data(), prim_dev, sizeof(double4_32a) * np))) return st;
     // in the cloud's order
     std::vector<double> bx(n), by(n), bnx(n), bny(n);
     for (int i = 0; i < n; i++) {
@@ -3625,14 +3685,14 @@ qlskum_status upload_points(qlskum_handle *h, const double *src, double4_32a *ds
         dev[h->perm[i]] = make_double4_32a(src[4 * (size_t)i], src[4 * (size_t)i + 1], src[4 * (size_t)i + 2],
                                            src[4 * (size_t)i + 3]);
     CK(h, cudaMemcpyAsync(dst, dev.data(), sizeof(double4_32a) * h->np, cudaMemcpyHostToDevice, h->L.stream));
-    CK(h, cudaStreamSynchronize(h->L.stream));
+    WAIT(h);
     return QLSKUM_OK;
 }
 
 qlskum_status download_points(qlskum_handle *h, const double4_32a *src, double *dst)
 {
     std::vector<double4_32a> dev(h->np);
-    qlskum_status st = d2h(h, dev.data(), src, sizeof(double4_32a) * h->np);
+    qlskum_status st = read_result(h, dev.data(), src, sizeof(double4_32a) * h->np);
     if (st) return st;
     for (int i = 0; i < h->n; i++) std::memcpy(dst + 4 * (size_t)i, &dev[h->perm[i]], sizeof(double4_32a));
     return QLSKUM_OK;
@@ -3969,9 +4029,9 @@ qlskum_status qlskum_adjoint_gradient(qlskum_handle *h, int objective, int iters
         double *d_init = a->buinf + 2;
         zero(h, d_init, 2 * sizeof(double));
         fp64::sum_yz(h->L, h->n, a->bP, d_init);
-        if ((st = d2h(h, binit, d_init, sizeof binit))) return st;
+        if ((st = read_result(h, binit, d_init, sizeof binit))) return st;
     }
-    if ((st = d2h(h, bu, a->buinf, sizeof bu))) return st;
+    if ((st = read_result(h, bu, a->buinf, sizeof bu))) return st;
     if (dJ_dprim0 && (st = download_points(h, a->bP, dJ_dprim0))) return st;
     if (J) *J = os.J;
     adj_params(h, os, bu, binit, dJ_dmach, dJ_daoa);
@@ -4021,14 +4081,14 @@ qlskum_status qlskum_adjoint_fixed_point(qlskum_handle *h, int objective, int ad
     adj_iteration_reverse(h, adj_view(h, dJ_dwall != nullptr), m32);
     if ((st = check_launch(h, "fixed-point adjoint"))) return st;
     double bu[2];
-    if ((st = d2h(h, bu, a->buinf, sizeof bu))) return st;
+    if ((st = read_result(h, bu, a->buinf, sizeof bu))) return st;
     if (adj_change) {
         // relative change of the last adjoint iteration, reduced on the device
         unsigned long long *d_mx = reinterpret_cast<unsigned long long *>(a->buinf + 2);
         zero(h, d_mx, 2 * sizeof(unsigned long long));
         fp64::max_change(h->L, h->n, a->lam, a->lam_prev, d_mx);
         unsigned long long mx[2];
-        if ((st = d2h(h, mx, d_mx, sizeof mx))) return st;
+        if ((st = read_result(h, mx, d_mx, sizeof mx))) return st;
         double dmax, lmax;
         std::memcpy(&dmax, &mx[0], sizeof dmax);
         std::memcpy(&lmax, &mx[1], sizeof lmax);

@@ -96,8 +96,9 @@ struct DevCloud {
     // NULL for a single case, whose constants come with the launch.
     const CaseConst *case_k = nullptr;
     const int *slice_case = nullptr;
-    // set to 2 by a kernel whose bulk copy did not arrive (the status word that
-    // also holds 1 for a non-finite residual)
+    // pinned host memory, set to 1 by a kernel whose bulk copy did not arrive, read
+    // by the host whenever it has waited for the kernels (NULL in the FP64 form,
+    // which makes no bulk copies)
     int *fault = nullptr;
 };
 

@@ -151,5 +151,26 @@ def build_fast64_host() -> str:
     return _build_host_test("fast64_host")
 
 
+def build_lost_copy() -> str:
+    """The library with its host layer rebuilt beside a test kernel
+    (tests/lost_copy/qlskum_lost_copy.cu), the other units as they are."""
+    build()
+    src = os.path.join(REPO, "tests", "lost_copy", "qlskum_lost_copy.cu")
+    lib = os.path.join(REPO, "tests", "_build", "libqlskum_lost_copy.so")
+    if os.path.exists(lib) and all(os.path.getmtime(p) <= os.path.getmtime(lib) for p in [src, LIB]):
+        return lib
+    nvcc = _nvcc()
+    os.makedirs(os.path.dirname(lib), exist_ok=True)
+    tmp = lib + f".tmp{os.getpid()}"
+    objs = [os.path.join(BUILD, f + ".o") for f in sources() if f != "qlskum_host.cpp"]
+    cmd = [nvcc, *ARCH, "-O1", "-std=c++17", "-Xcompiler", "-fPIC,-ffp-contract=off", "-I", INCLUDE, "-I", CSRC, "-shared", "-o", tmp,
+           src, *objs, "-lcudart_static", "-ldl", "-lrt", "-lpthread"]
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("building the lost-copy test library failed:\n" + " ".join(cmd) + "\n" + r.stdout)
+    os.replace(tmp, lib)
+    return lib
+
+
 if __name__ == "__main__":
     print(build(force="--force" in sys.argv, verbose=True, ptxas_info="--ptxas" in sys.argv))
