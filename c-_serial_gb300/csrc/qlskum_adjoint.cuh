@@ -212,30 +212,23 @@ template <typename R> QLSKUM_HD void edge_end_vjp(R delx, R dely, const R q[4], 
     }
 }
 
-// One edge end and its reverse in one piece, checked on the CPU against the
-// functions above; the device's flux reverse (adjk::k_flux) takes the same
-// steps in the forms of qlskum_fast64.cuh.  The limited reconstruction (interior_fluxes_mod.h:72-83, limiters_mod.h:64-104),
-// q~ -> prim (q_variables_mod.h:230-253) and the half-range moments
-// (split_fluxes_mod.h:14-26), keeping what end64_vjp reads.  The functions
-// above recompute each quantity they need (an edge end then costs 33 FP64
-// divisions, 6 exps and 2 logs); here one end costs 7 reciprocals (rcp64 on
-// the device: an FP32 seed and two Newton steps, no FP64 division), 3 exps
-// and 1 log.  The forward values are those of edge_states / kin_prep up to
-// last-bit roundings: the limiter's ratio is num * (1 / den), whose
-// reciprocal the VJP reads too; kin_prep's beta = rho / (2 p) and
-// p / rho are the q~ -> prim step's beta and 1 / (2 beta); 1 / (gamma - 1)
-// and 1 / sqrt(pi beta) are multiplications.  The reverse is the derivative
-// at that state, along the branches it took.
+// One edge end and its reverse in one piece from the formulas of the functions
+// above, for the CPU tests alone: the GPU's flux reverse (adjk::k_flux) has its
+// end in qlskum_reverse64.cuh, which is checked against this one, as this one is
+// against the functions above.  The limited reconstruction
+// (interior_fluxes_mod.h:72-83, limiters_mod.h:64-104), q~ -> prim
+// (q_variables_mod.h:230-253) and the half-range moments
+// (split_fluxes_mod.h:14-26), keeping what end64_vjp reads: the forward values
+// are those of edge_states / kin_prep up to last-bit roundings, the reverse is
+// the derivative at that state, along the branches it took.
 struct End64 {
     double g[4], dn[4], dp[4], rden[4], t[4];  // per component: g, q~u - q, qmax|qmin - q, 1 / den, num / den
     double eps2, qt1, qt2, beta, tm, u1, u2, rho, sb, rsb, e1, e2;
     Kin<double> k;
 };
 
-// kept (or NULL): the forward flux kernel's {rho, sqrt(beta), exp(-S1^2),
-// exp(-S2^2), erf(S1), erf(S2)} of this end (fp64::flux_residual's ends),
-// taken instead of recomputing the log, the exps, the square root and the
-// erfs.
+// kept (or NULL): {rho, sqrt(beta), exp(-S1^2), exp(-S2^2), erf(S1), erf(S2)} of
+// this end, taken instead of evaluating them.
 QLSKUM_HD void end64(double nx, double ny, double delx, double dely, const double q[4], const double dx[4],
                      const double dy[4], const double mx[4], const double mn[4], double e2, End64 &s,
                      const double *kept = nullptr)

@@ -1,6 +1,6 @@
-// Host entry points to the FP64 form's fast functions (qlskum_fast64.cuh), for
-// checking them against libm in long double on a machine without a GPU
-// (tests/test_fast64_math.py).  Same source as the device code, with the CUDA
+// Host entry points to the FP64 form's fast functions (qlskum_fast64.cuh) and to
+// the reverse of its flux (qlskum_reverse64.cuh), for checking them on a machine
+// without a GPU (tests/test_fast64_math.py, test_reverse64_math.py).  Same source as the device code, with the CUDA
 // intrinsics it uses defined here; those that approximate on the device
 // (__fdividef, rsqrtf: 2 ulp) are moved off the correctly rounded value by
 // `seed_shift` ulps.
@@ -45,6 +45,7 @@ template <typename T> inline T __ldg(const T *p) { return *p; }
 #define __noinline__
 #define QLSKUM_HOST_INTRINSICS
 #include "qlskum_fast64.cuh"
+#include "qlskum_reverse64.cuh"
 
 using namespace qlskum;
 
@@ -122,6 +123,70 @@ void qlskum_f64_limited(int n, const double *q, const double *dn, const double *
     for (int i = 0; i < n; i++) {
         out[i] = fast64::limited(q[i], dn[i], dp[i], eps2[i]);
         phi[i] = fast64::limited(0.0, dn[i], dp[i], eps2[i]) / dn[i];
+    }
+}
+
+// One end of an edge of a class-f point with half ranges `dir` and their
+// weights w = {x, y, second x, second y}, as the flux kernels evaluate it.
+// in: [q4 dx4 dy4 mx4 mn4] (20) -> v (4), kept (6).
+void qlskum_f64_end(int f, int dir, const double *in, double e2, double delx, double dely, double nx, double ny,
+                    const double *w, double *v, double *kept)
+{
+    DevCloud c;
+    c.gauss_tab = tables.gauss.data();
+    c.exp_tab = tables.exp.data();
+    const double hx = -0.5 * delx, hy = -0.5 * dely;
+    double t[4];
+    for (int r = 0; r < 4; r++) {
+        const double dn = std::fma(hx, in[4 + r], hy * in[8 + r]);
+        t[r] = fast64::limited(in[r], dn, (dn >= 0.0 ? in[12 + r] : in[16 + r]) - in[r], e2);
+    }
+    fast64::End s;
+    fast64::end(c, f, nx, ny, t, s);
+    fast64::keep_end(kept, 1, s);
+    const unsigned neg = 0x80000000u;
+    const unsigned sx = (dir & kXpos) ? 0u : neg, sy = (dir & kYpos) ? 0u : neg, s2 = f == kOuter ? 0u : neg;
+    const bool inner = f == kInterior;
+    for (int r = 0; r < 4; r++) v[r] = 0.0;
+    fast64::split_pair(s, sx, sy, inner ? 0.5 * w[0] : 0.0, 0.5 * w[1], v);
+    if (!inner) fast64::quad_x(s, sx, s2, 0.5 * w[0], v);
+    if ((dir & (kXpos | kXneg)) == (kXpos | kXneg)) {
+        if (inner) fast64::split_pair(s, neg, 0u, 0.5 * w[2], 0.0, v);
+        else fast64::quad_x(s, neg, s2, 0.5 * w[2], v);
+    }
+    if ((dir & (kYpos | kYneg)) == (kYpos | kYneg)) fast64::split_pair(s, 0u, neg, 0.0, 0.5 * w[3], v);
+    v[3] *= 0.5;
+}
+
+// Its reverse for the bar b of v.  out: bars of the 20 inputs, then bdelx,
+// bdely, bnx, bny, as adjk::k_flux distributes them.
+void qlskum_f64_end_vjp(int f, int dir, const double *in, double e2, double delx, double dely, double nx, double ny,
+                        const double *w, const double *kept, const double *b, double *out)
+{
+    const double hx = -0.5 * delx, hy = -0.5 * dely;
+    adjk::RevEnd s;
+    adjk::EndBar o;
+    double bt[4];
+    adjk::rev_end(f, nx, ny, hx, hy, in, in + 4, in + 8, in + 12, in + 16, e2, kept, 1, s);
+    adjk::flux_bars(f, dir, s.k, w[0], w[1], w[2], w[3], b, o);
+    adjk::end_vjp(s, o, bt);
+    for (int r = 0; r < 24; r++) out[r] = 0.0;
+    out[22] = s.t[1] * bt[2] - s.t[2] * bt[1];
+    out[23] = s.t[1] * bt[1] + s.t[2] * bt[2];
+    if (f != kInterior) {
+        const double bs = bt[1], bn = bt[2];
+        bt[1] = bs * ny + bn * nx;
+        bt[2] = bn * ny - bs * nx;
+    }
+    for (int r = 0; r < 4; r++) {
+        double bdn, bdp;
+        adjk::limited_vjp(s.l[r], bt[r], bdn, bdp);
+        out[r] = bt[r] - bdp;
+        out[4 + r] = hx * bdn;
+        out[8 + r] = hy * bdn;
+        out[(s.l[r].dn >= 0.0 ? 12 : 16) + r] = bdp;
+        out[20] -= 0.5 * bdn * in[4 + r];
+        out[21] -= 0.5 * bdn * in[8 + r];
     }
 }
 
