@@ -6,7 +6,9 @@
 // gradients, the least-squares gradient and neighbour min / max, the q
 // variables, and finally the local time step.  The forward stage states it
 // needs are recomputed by the FP64 forward kernels from the iteration's
-// checkpointed state.  One thread per point; a point's contributions to its
+// checkpointed state.  The flux reverse spreads a point's edges over several
+// threads, the gradient's, the inner step's and the time step's take four lanes
+// per point, the pointwise ones a thread; a point's contributions to its
 // neighbours' adjoints are scattered with FP64 atomics (the bar of a
 // neighbour's q, dq, qm, or wave speed).
 //
@@ -87,11 +89,11 @@ __global__ void k_update(AdjView a, CaseConst K, const double4_32a *__restrict__
 // point's edges spread over kRevThreads / P of them as in fp64::block_flux;
 // each thread adds its edges' owner bars to its own slots of shared memory,
 // which the block sums at the end.
-// Bound by the FP64 pipe: about 400 FP64 instructions per edge, 16 FP64
-// reductions to L2.  51,200 points (512,000 edges): 1707 us with one thread
+// Bound by the FP64 pipe (84% active; 466 lanes of FP64 instructions per edge,
+// those without an edge among them), 16 FP64 reductions to L2 per edge.  51,200 points (512,000 edges): 1707 us with one thread
 // per point and all four half ranges at every edge, 448 us in this form; the
 // geometry bars of a 20,480-point cloud (128 wall points) 922 and 37 us.  Four blocks
-// of 128 registers per SM: 3-8% over two at 178.
+// of 128 registers per SM, which spill 248 B: 3-8% over two at 178.
 constexpr int kRevThreads = 128;
 
 template <int P, bool GEO>

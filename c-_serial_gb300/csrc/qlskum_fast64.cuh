@@ -7,12 +7,17 @@
 // number of FP64 instructions alone.  What can be done beside the FP64 pipe
 // without touching the FP64 result is done there: comparisons on the bit
 // patterns, argument reductions and seeds in FP32, and the high-order terms
-// of an expansion, whose contribution is below 2^-28 of the result, so that
-// an FP32 evaluation (relative error 2^-24) stays below 2^-52 of it.
+// of an expansion, small enough that FP32's relative error of 2^-24 stays
+// below 2^-52 of the result (but for exp(-S^2) at |S| > 2, where the error of
+// S^2 itself is larger).
 //
-// Each function's error is at most about an ulp of its result (of 1 for erf),
-// as the CUDA functions it replaces; arguments outside the ranges below
-// (which a physical state does not reach, and every Inf / NaN) take those.
+// Errors against long double (tests/test_fast64_math.py): quotients and
+// reciprocal roots 0.503 ulp, exp32 1.02 (rms 0.34), erf 1.01 2^-53, and
+// exp(-S^2) 1.1 ulp below |S| = 1, then up to 1.6, 3.8, 8.8, 22 and 30 ulp (rms
+// 0.35, 0.47, 0.86, 1.8, 3.1) in each unit of |S| up to 6, where the expression
+// exp(-S * S) that it replaces has an rms error of 0.74, 2.1, 3.4, 6.8 and 9.6.
+// Arguments outside the ranges below (which a physical state does not reach, and
+// every Inf / NaN) take CUDA's functions.
 //
 // FP64 instructions per call: gauss_erf 10 (exp and erf: about 50), exp32 5
 // (about 16), rsqrt_rcp 7 for both, ratio64 3.
@@ -76,7 +81,7 @@ __device__ __forceinline__ double ratio64(double num, double den)
 
 // The same as a call, for places that are no inner loop: inlined three times
 // into an outer point's update it made the mixed flux kernel with 72 registers
-// spill (1.02 M points 1,357 -> 1,370 us per iteration).
+// spill (4 to 5 us of the 1,357 us per iteration at 1.02 M points).
 static __device__ __noinline__ double ratio64_call(double num, double den) { return ratio64(num, den); }
 
 // r = 1 / sqrt(x) and h = 1 / x from the FP32 seed y of r, whose square is

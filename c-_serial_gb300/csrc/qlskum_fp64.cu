@@ -345,6 +345,9 @@ __device__ __forceinline__ bool block_flux(const DevCloud &c, const double4_32a 
     return true;
 }
 
+// The same for the module path and for the adjoint, with the ends recorded (79%
+// of the FP64 pipe).  It keeps k_flux_update's cap of 128 registers and spills 148 B;
+// three blocks without the spills were not measured.
 template <int P>
 __global__ void __launch_bounds__(kFluxThreads, 4) k_flux_residual(DevCloud c, const double4_32a *__restrict__ q,
                                                      const double4_32a *__restrict__ dq, const double4_32a *__restrict__ qm,
@@ -403,8 +406,8 @@ __global__ void __launch_bounds__(kPointBlock) k_state_update(DevCloud c, CaseCo
 // edge and 32 directional sums (about 630 per edge), 1066 us in this form with
 // a thread per point, 951 us with the edges spread (flux_shape), 898 us with
 // the quotient, the reciprocals and the half weights in their present forms
-// (220 -> 200 per edge, FP64 pipe 86% active).  Four blocks of 128 registers a
-// thread per SM: 5% over three blocks at 146.
+// (220 -> 200 per edge, FP64 pipe 87% active).  Four blocks of 128 registers a
+// thread per SM, which spill 32 B: 5% over three blocks at 146.
 template <int P>
 __global__ void __launch_bounds__(kFluxThreads, 4) k_flux_update(DevCloud c, CaseConst K, const double4_32a *__restrict__ q,
                                                    const double4_32a *__restrict__ dq,

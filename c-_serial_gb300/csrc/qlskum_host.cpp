@@ -2591,7 +2591,7 @@ qlskum_status qlskum_partition_create(const qlskum_cloud *c, const qlskum_params
     for (int q = 0; q < n_parts; q++)
         for (int o = 0; o < n_parts; o++)
             if (peer[q][o] && o != q) P->parts[q]->peers.push_back(o);
-    // the shared residual arrays: a partial per 32 points of each partition is enough for any launch shape
+    // the shared residual arrays: a partial per 8 points of each partition is enough for any launch shape
     int maxp = 0;
     for (PartDev *d : P->parts) maxp += fp64::partials(d->G.n);
     P->R.max_blocks = maxp;

@@ -39,7 +39,7 @@ typedef enum {
     QLSKUM_ERR_INVALID = 1,      /* bad argument or malformed cloud */
     QLSKUM_ERR_DEGENERATE = 2,   /* a sub-stencil has a singular 2x2 least-squares matrix */
     QLSKUM_ERR_NONFINITE = 3,    /* the state or the residual became NaN / Inf */
-    QLSKUM_ERR_CUDA = 4,         /* a CUDA call failed */
+    QLSKUM_ERR_CUDA = 4,         /* a CUDA call failed, or a kernel gave up on a copy of its edge lists */
     QLSKUM_ERR_UNSUPPORTED = 5   /* option not available in this build / precision */
 } qlskum_status;
 
@@ -74,7 +74,8 @@ typedef struct {
     double power;                 /* least-squares weights dist^power */
     int inner_iterations;
     int precision;                /* qlskum_precision */
-    int block_size;               /* threads per block for the point kernels; 0 = default */
+    int block_size;               /* threads per block for the point kernels, a multiple of 32 up to 1024
+                                     (the mixed gradient takes at most 512); 0 = default */
     int reorder;                  /* 1 = Morton/class reorder of points on the device (default), 0 = file order */
     int verbose;                  /* 1 = print "iterations <it> residue : <r>" per iteration like fpi_solver_mod.h:150 */
 } qlskum_params;
@@ -174,11 +175,14 @@ long long qlskum_launch_count(const qlskum_handle *h);
 qlskum_status qlskum_get_launch_config(qlskum_handle *h, int *flux_block, int *flux_min_blocks, int *point_block,
                                        int *gather_depth);
 /* Pin the mixed form's launch shape instead of autotuning it: flux_variant in
- * 0 .. 9 (threads x min blocks 128x4, 128x5, 64x8, 256x2 with one gather per
- * edge in turn; 128x4, 128x5, 64x8, 256x2 with the next edge's neighbour data
- * in flight by cp.async; 128x4 with 2 lanes per point, 256x2 with 4 lanes per
- * point, a point's edges split over its lanes and their sums combined by
- * warp shuffles), point_block one of
+ * 0 .. 18 (threads x min blocks: 0 .. 3 128x4, 128x5, 64x8, 256x2 with one gather
+ * per edge in turn; 4 .. 7 the same shapes with the next edge's neighbour data in
+ * flight by cp.async; 8 and 9 128x4 with 2 lanes per point and 256x2 with 4, a
+ * point's edges split over its lanes and their sums combined by warp shuffles,
+ * the next edge's neighbour data in registers; 10 .. 13 128x4, 128x5, 64x6, 256x2
+ * with one lane per point and that prefetch; 14 and 15 128x5 and 128x6 with the
+ * point's own data in shared memory besides; 16 .. 18 128x6, 128x7, 128x8 of that
+ * form with only the next edge's index and edge data ahead), point_block one of
  * 64 / 128 / 256 / 512 for the per-edge gather form, staged 0 (that form) or
  * 1 .. 4 (staged gathers: 128 threads depth 2, 128 / 4, 256 / 3, 64 / 4).
  * The gradient / inner-loop kernels go back to one lane per point.
